@@ -11,6 +11,7 @@ import torch
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libnvfp4_b200.so")
+HOST_PATH = os.path.join(HERE, "_host.so")
 
 SCALES_SWIZZLED, SCALES_LINEAR = 0, 1
 DTYPE_BF16, DTYPE_FP32 = 0, 1
@@ -80,6 +81,25 @@ def load():
             lib.nvfp4_quant_tile_set_path(int(os.environ["NVFP4_TILE_PATH"]))
         _lib = lib
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host module (csrc/host.cpp), bound to the loaded library; raise if it has not been built.  Operators
+    call `_host or host()`: one global look-up once it is there."""
+    global _host
+    if _host is None:
+        lib = load()
+        if not os.path.exists(HOST_PATH):
+            raise Nvfp4Error(f"{HOST_PATH} not found: build it with `python -m nvfp4_training_b200.build` "
+                             "(there is no fallback path)")
+        from . import _host as h, linear, nvq
+        h.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in h.entry_points()}, Nvfp4Error,
+               linear.LinCtx, nvq, status_word)
+        _host = h
+    return _host
 
 
 def check(rc, what):

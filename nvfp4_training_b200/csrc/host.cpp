@@ -1,0 +1,587 @@
+// Native host path of the Python operators: argument checks, output allocation, stream look-up and the calls into the
+// C-ABI library, in one C++ call per operator and one per layer pass.
+//
+// What bounds the small and middle-sized layers is not the GPU but the interpreter: a forward and backward pass of one
+// linear is nine kernels and, written in Python over ctypes, 25 tensor allocations, 11 foreign calls of up to 20
+// converted arguments and 11 walks of torch's Python stream objects -- 340 us of host work around 55 us of kernels
+// at [128, 256] x [384, 256].  Here a pass is one call: scratch that dies with the call is one allocation addressed by
+// offsets, what the backward pass needs is one more, and the backward is an autograd node that runs without the
+// interpreter except for one look at the caller's switches (seed, gradient type, rounding mode, cached weight).  That
+// pass went from 340 to 95 us, [4096, 2048] x [3072, 2048] from 350 to 145, a forward without gradients from 80 to 29.
+//
+// The library itself is not linked: `bind` receives the addresses of its entry points from the ctypes binding, so both
+// always use the same build.  Exceptions: AssertionError for shapes and types (as the Python asserts it replaces),
+// the package's Nvfp4Error for CPU tensors and for calls the library rejects.
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAStream.h>
+#include <pybind11/pybind11.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <mutex>
+
+#include "../../include/nvfp4_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+// ------------------------------------------------------------------------------------------ library entry points
+#define NVFP4_API(X)                                                                                                        \
+  X(nvfp4_amax_bf16) X(nvfp4_amax_bf16_update) X(nvfp4_quant_rows) X(nvfp4_quant_cols_rht) X(nvfp4_quant_tile)             \
+  X(nvfp4_quant_w2d) X(nvfp4_gemm) X(nvfp4_error_string)
+struct Api {
+#define X(name) decltype(&::name) name = nullptr;
+  NVFP4_API(X)
+#undef X
+};
+Api lib;
+
+struct AssertionFailure : std::runtime_error { using std::runtime_error::runtime_error; };
+struct LibraryError : std::runtime_error { using std::runtime_error::runtime_error; };
+// Python objects the module keeps for the life of the process (never released: the interpreter may be gone by then)
+py::handle error_class, lin_ctx, nvq_module, status_word_fn;
+
+#define REQUIRE(cond, what) do { if (!(cond)) throw AssertionFailure(what); } while (0)
+
+void check(int rc, const char* what) {
+  if (rc != 0)
+    throw LibraryError(std::string(what) + ": " + lib.nvfp4_error_string(rc) + " (status " + std::to_string(rc) + ")");
+}
+void require_cuda(const Tensor& t) {
+  if (!t.is_cuda()) throw LibraryError("nvfp4_b200 kernels need CUDA tensors; there is no CPU path");
+}
+void require_cuda(const OptTensor& t) { if (t) require_cuda(*t); }
+
+std::string shape_of(int64_t a, int64_t b) { return "(" + std::to_string(a) + ", " + std::to_string(b) + ")"; }
+
+// ------------------------------------------------------------------------------------------ small pieces
+void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+Tensor empty(at::IntArrayRef size, at::ScalarType dtype, const Tensor& like) {
+  return at::detail::empty_cuda(size, dtype, like.device(), std::nullopt);
+}
+const void* cptr(const OptTensor& t) { return t ? t->const_data_ptr() : nullptr; }
+
+// Host seed or a device word: a CUDA int32 / uint32 tensor selects the device-side seed.
+struct Seed {
+  unsigned host = 0;
+  const unsigned* dev = nullptr;
+  Tensor keep;
+  Seed() = default;
+  explicit Seed(unsigned h) : host(h) {}
+  explicit Seed(py::handle o) {
+    if (THPVariable_Check(o.ptr())) {
+      keep = THPVariable_Unpack(o.ptr());
+      REQUIRE(keep.is_cuda() && keep.numel() >= 1 && keep.element_size() == 4, "seed: a CUDA tensor of 32-bit words");
+      dev = static_cast<const unsigned*>(keep.const_data_ptr());
+    } else {
+      host = (unsigned)PyLong_AsUnsignedLongLongMask(o.ptr());
+      if (PyErr_Occurred()) throw py::error_already_set();
+    }
+  }
+};
+
+// Per-device status word of the GEMM, created and owned by the Python binding.
+int* status_word(const Tensor& like) {
+  constexpr int kDevices = 64;
+  static int* words[kDevices] = {};
+  const int dev = like.get_device();
+  TORCH_CHECK(dev >= 0 && dev < kDevices);
+  if (!words[dev]) {
+    py::gil_scoped_acquire gil;
+    words[dev] = static_cast<int*>(py::cast<Tensor>(status_word_fn(like.device())).data_ptr());
+  }
+  return words[dev];
+}
+
+// Carves sub-buffers, each at a multiple of 256 bytes, out of one allocation; in a dry run it only adds up sizes.
+struct Carver {
+  char* base = nullptr;
+  size_t used = 0;
+  template <typename T = void>
+  T* take(size_t bytes) {
+    T* p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+    used += (bytes + 255) & ~size_t(255);
+    return p;
+  }
+};
+
+// A packed matrix [R, C]: codes, swizzled scales, tensor scale.
+struct Packed {
+  const void* d; const void* s; const float* gs;
+};
+struct PackedOut {
+  void* d; void* s; float* gs;
+  operator Packed() const { return {d, s, gs}; }
+};
+PackedOut carve_packed(Carver& c, int64_t R, int64_t C) {
+  void* d = c.take(R * C / 2);
+  void* s = c.take(R * C / 16);
+  return {d, s, c.take<float>(4)};
+}
+
+// Fresh output tensors of a packed matrix (the `d`, `s`, `gs` of a Q).
+struct PackedTensors {
+  Tensor d, s, gs;
+  PackedTensors(int64_t R, int64_t C, const Tensor& like)
+      : d(empty({R, C / 2}, at::kFloat4_e2m1fn_x2, like)), s(empty({R * C / 16}, at::kFloat8_e4m3fn, like)),
+        gs(empty({1}, at::kFloat, like)) {}
+  PackedOut out() const { return {d.data_ptr(), s.data_ptr(), gs.data_ptr<float>()}; }
+  py::tuple tuple() const { return py::make_tuple(d, s, gs); }
+};
+
+// ------------------------------------------------------------------------------------------ launches
+void run_amax(const Tensor& x, float* out, bool clear = true) {
+  check((clear ? lib.nvfp4_amax_bf16 : lib.nvfp4_amax_bf16_update)(x.const_data_ptr(), x.numel(), out, stream()), "amax");
+}
+
+void run_tile(const Tensor& x, const PackedOut* row, const PackedOut* col, const float* am, unsigned signs, int mode,
+              const Seed& seed, const Seed& seed_cols) {
+  check(lib.nvfp4_quant_tile(x.const_data_ptr(), x.stride(0), (int)x.size(0), (int)x.size(1), row ? row->d : nullptr,
+                             row ? row->s : nullptr, col ? col->d : nullptr, col ? col->s : nullptr, NVFP4_SCALES_SWIZZLED, am,
+                             row ? row->gs : nullptr, col ? col->gs : nullptr, signs & 0xFFFFu, mode, seed.host,
+                             seed_cols.host, seed.dev, seed_cols.dev, stream()), "quant_tile");
+}
+
+void run_w2d(const Tensor& w, const PackedOut* q, const PackedOut* qt, const float* am) {
+  check(lib.nvfp4_quant_w2d(w.const_data_ptr(), NVFP4_DTYPE_BF16, (int)w.size(0), (int)w.size(1), q ? q->d : nullptr,
+                            q ? q->s : nullptr, qt ? qt->d : nullptr, qt ? qt->s : nullptr, NVFP4_SCALES_SWIZZLED, am,
+                            (q ? q : qt)->gs, stream()), "quant_w2d");
+}
+
+// contiguous packed operands a [M, K], b [N, K] -> c [M, N]
+void run_mm(const Packed& a, const Packed& b, const Tensor& c, int64_t K, bool accumulate, int splitk) {
+  const bool fp32 = c.scalar_type() == at::kFloat;
+  check(lib.nvfp4_gemm(a.d, a.s, K / 2, b.d, b.s, K / 2, c.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16,
+                       c.stride(0), (int)c.size(0), (int)c.size(1), (int)K, NVFP4_ALPHA_GS, a.gs, b.gs, 1.f, 1.f, accumulate,
+                       fp32 ? splitk : 1, status_word(c), stream()), "mm");
+}
+
+// ------------------------------------------------------------------------------------------ nvq operators
+Tensor nvq_amax(const Tensor& x, const OptTensor& out_, bool clear) {
+  require_cuda(x); require_cuda(out_);
+  REQUIRE(out_ || clear, "amax: clear=False needs out");
+  REQUIRE(x.numel() % 8 == 0 && x.is_contiguous() && x.scalar_type() == at::kBFloat16, "amax: contiguous bf16, a multiple of 8 values");
+  Tensor out = out_ ? *out_ : empty({1}, at::kFloat, x);
+  run_amax(x, static_cast<float*>(out.data_ptr()), clear);
+  return out;
+}
+
+// amax word of `x`: the caller's, or computed now into a new one
+Tensor amax_or(const OptTensor& am, const Tensor& x) {
+  if (am) return *am;
+  at::NoGradGuard no_grad;
+  return nvq_amax(x.contiguous(), std::nullopt, true);
+}
+const float* word(const Tensor& am) { return static_cast<const float*>(am.const_data_ptr()); }
+
+py::tuple nvq_quant_rows(const Tensor& x, int mode, py::handle seed_, const OptTensor& am_) {
+  require_cuda(x);
+  REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16, "quant_rows: a bf16 matrix");
+  const int64_t R = x.size(0), C = x.size(1);
+  REQUIRE(x.stride(1) == 1 && C % 64 == 0 && R % 128 == 0, shape_of(R, C));
+  const Seed seed(seed_);
+  const Tensor am = amax_or(am_, x);
+  PackedTensors q(R, C, x);
+  const PackedOut o = q.out();
+  check(lib.nvfp4_quant_rows(x.const_data_ptr(), x.stride(0), (int)R, (int)C, o.d, o.s, NVFP4_SCALES_SWIZZLED, word(am), o.gs,
+                             mode, seed.host, seed.dev, stream()), "quant_rows");
+  return q.tuple();
+}
+
+py::tuple nvq_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, py::handle seed_, const OptTensor& am_) {
+  require_cuda(x_);
+  REQUIRE(x_.dim() == 2 && x_.scalar_type() == at::kBFloat16, "quant_cols_rht: a bf16 matrix");
+  at::NoGradGuard no_grad;
+  const Tensor x = x_.contiguous();
+  const int64_t M = x.size(0), C = x.size(1);
+  REQUIRE(M % 64 == 0 && C % 128 == 0, shape_of(M, C));
+  const Seed seed(seed_);
+  const Tensor am = amax_or(am_, x);
+  PackedTensors q(C, M, x);
+  const PackedOut o = q.out();
+  // the tile kernel takes whole 128-token tiles: same bits, faster than the register-tiled kernel
+  if (M % 128 == 0) run_tile(x, nullptr, &o, word(am), signs, mode, Seed(), seed);
+  else check(lib.nvfp4_quant_cols_rht(x.const_data_ptr(), (int)M, (int)C, o.d, o.s, NVFP4_SCALES_SWIZZLED, word(am), o.gs,
+                                      signs & 0xFFFFu, mode, seed.host, seed.dev, stream()), "quant_cols_rht");
+  return q.tuple();
+}
+
+py::tuple nvq_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py::handle seed_, py::handle seed_cols_,
+                                  const OptTensor& am_, bool want_rows, bool want_cols) {
+  require_cuda(x);
+  REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "quant_rows_cols_rht: a bf16 matrix with contiguous rows");
+  const int64_t M = x.size(0), C = x.size(1);
+  REQUIRE(M % 128 == 0 && C % 128 == 0, shape_of(M, C));
+  const Seed seed(seed_), seed_cols(seed_cols_);
+  const Tensor am = amax_or(am_, x);
+  std::optional<PackedTensors> qr, qc;
+  PackedOut r, c;
+  if (want_rows) { qr.emplace(M, C, x); r = qr->out(); }
+  if (want_cols) { qc.emplace(C, M, x); c = qc->out(); }
+  run_tile(x, want_rows ? &r : nullptr, want_cols ? &c : nullptr, word(am), signs, mode, seed, seed_cols);
+  return py::make_tuple(qr ? py::object(qr->tuple()) : py::none(), qc ? py::object(qc->tuple()) : py::none());
+}
+
+// Fresh outputs, the two operands sharing one tensor scale; a skipped operand is None.
+py::tuple nvq_quant_w2d(const Tensor& w_, const OptTensor& am_, bool want, bool want_t) {
+  require_cuda(w_);
+  REQUIRE(w_.dim() == 2 && w_.scalar_type() == at::kBFloat16, "quant_w2d: a bf16 matrix");
+  at::NoGradGuard no_grad;
+  const Tensor w = w_.contiguous();
+  const int64_t N = w.size(0), K = w.size(1);
+  REQUIRE(N % 128 == 0 && K % 128 == 0, shape_of(N, K));
+  const Tensor am = amax_or(am_, w);
+  const Tensor gs = empty({1}, at::kFloat, w);
+  auto alloc = [&](int64_t R, int64_t C, Tensor& d, Tensor& s) {
+    d = empty({R, C / 2}, at::kFloat4_e2m1fn_x2, w);
+    s = empty({R * C / 16}, at::kFloat8_e4m3fn, w);
+    return PackedOut{d.data_ptr(), s.data_ptr(), gs.data_ptr<float>()};
+  };
+  Tensor d, s, dt, st;
+  PackedOut q, qt;
+  if (want) q = alloc(N, K, d, s);
+  if (want_t) qt = alloc(K, N, dt, st);
+  run_w2d(w, want ? &q : nullptr, want_t ? &qt : nullptr, word(am));
+  return py::make_tuple(want ? py::object(py::make_tuple(d, s, gs)) : py::none(),
+                        want_t ? py::object(py::make_tuple(dt, st, gs)) : py::none());
+}
+
+// In place into an earlier call's buffers.
+void nvq_quant_w2d_into(const Tensor& w_, const OptTensor& am_, const OptTensor& d, const OptTensor& s, const OptTensor& dt,
+                        const OptTensor& st, const Tensor& gs) {
+  require_cuda(w_);
+  REQUIRE(w_.dim() == 2 && w_.scalar_type() == at::kBFloat16, "quant_w2d: a bf16 matrix");
+  at::NoGradGuard no_grad;
+  const Tensor w = w_.contiguous();
+  REQUIRE(w.size(0) % 128 == 0 && w.size(1) % 128 == 0, shape_of(w.size(0), w.size(1)));
+  const Tensor am = amax_or(am_, w);
+  float* g = static_cast<float*>(gs.data_ptr());
+  const PackedOut q{d ? d->data_ptr() : nullptr, s ? s->data_ptr() : nullptr, g};
+  const PackedOut qt{dt ? dt->data_ptr() : nullptr, st ? st->data_ptr() : nullptr, g};
+  run_w2d(w, d ? &q : nullptr, dt ? &qt : nullptr, word(am));
+}
+
+// A block-scaled GEMM into `out` (or a fresh tensor): alpha = product of the two words as `alpha_mode` says.
+Tensor gemm(const Tensor& ad, const Tensor& as, const Tensor& bd, const Tensor& bs, const OptTensor& out_, bool fp32, int alpha_mode,
+            const OptTensor& pa, const OptTensor& pb, float ka, float kb, bool accumulate, int splitk, const char* what) {
+  require_cuda(ad); require_cuda(bd);
+  const int64_t M = ad.size(0), N = bd.size(0), K = ad.size(1) * 2;
+  REQUIRE(bd.size(1) * 2 == K, shape_of(M, K / 2) + ", " + shape_of(N, bd.size(1)));
+  const at::ScalarType dtype = fp32 ? at::kFloat : at::kBFloat16;
+  if (out_) {
+    require_cuda(out_);
+    REQUIRE(out_->dim() == 2 && out_->size(0) == M && out_->size(1) == N && out_->scalar_type() == dtype && out_->stride(1) == 1,
+            "out: shape, type or row layout");
+  } else {
+    REQUIRE(!accumulate, "accumulate needs out");
+  }
+  Tensor out = out_ ? *out_ : empty({M, N}, dtype, ad);
+  check(lib.nvfp4_gemm(ad.const_data_ptr(), as.const_data_ptr(), ad.stride(0), bd.const_data_ptr(), bs.const_data_ptr(), bd.stride(0),
+                       out.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16, out.stride(0), (int)M, (int)N, (int)K, alpha_mode,
+                       static_cast<const float*>(cptr(pa)), static_cast<const float*>(cptr(pb)), ka, kb, accumulate,
+                       fp32 ? splitk : 1, status_word(ad), stream()), what);
+  return out;
+}
+
+Tensor nvq_mm(const Tensor& ad, const Tensor& as, const Tensor& ag, const Tensor& bd, const Tensor& bs, const Tensor& bg, bool fp32,
+              bool scale, const OptTensor& out, bool accumulate, int splitk) {
+  return gemm(ad, as, bd, bs, out, fp32, scale ? NVFP4_ALPHA_GS : NVFP4_ALPHA_ONE, scale ? OptTensor(ag) : OptTensor(),
+              scale ? OptTensor(bg) : OptTensor(), 1.f, 1.f, accumulate, splitk, "mm");
+}
+
+// ------------------------------------------------------------------------------------------ the linear layer
+// y = Q_rn(x) Q(W)^T with the row operand of x in scratch; `xt` (optional) receives the transposed operand.
+Tensor forward_core(const Tensor& x, const float* am, const Packed& w, int64_t N, const PackedOut* xt, unsigned signs) {
+  const int64_t T = x.size(0), K = x.size(1);
+  Carver size;
+  carve_packed(size, T, K);
+  const Tensor scratch = empty({(int64_t)size.used}, at::kByte, x);
+  Carver c{static_cast<char*>(scratch.data_ptr())};
+  const PackedOut qx = carve_packed(c, T, K);
+  run_tile(x, &qx, xt, am, signs, NVFP4_ROUND_NEAREST, Seed(), Seed());
+  Tensor y = empty({T, N}, at::kBFloat16, x);
+  run_mm(qx, w, y, K, false, 1);
+  return y;
+}
+
+struct BackwardArgs {
+  int64_t K;                       // in-features
+  unsigned signs;
+  int mode;
+  bool want_x = true, want_w = true;
+  OptTensor gw_out;                // FP32 [N, K] to add into (or overwrite); else a new tensor of `gw_dtype`
+  bool overwrite = false;
+  at::ScalarType gw_dtype = at::kFloat;
+  OptTensor am;                    // amax(gy) where the caller has it
+  OptTensor am_out;                // else a cleared word to compute it into
+};
+
+// gx = Q_sr(gy) Q(W^T)^T and gW = Q_sr(H gy)^T Q(H x): one amax, one pass over gy for both operands, two GEMMs
+std::pair<Tensor, Tensor> backward_core(const Tensor& gy, const Packed& wt, const Packed& xt, const Seed& seed,
+                                        const Seed& seed_cols, const BackwardArgs& a) {
+  const int64_t T = gy.size(0), N = gy.size(1);
+  Tensor gx, gw;
+  auto carve = [&](Carver& c, PackedOut& r, PackedOut& t, float*& am) {
+    am = c.take<float>(4);
+    if (a.want_x) r = carve_packed(c, T, N);
+    if (a.want_w) t = carve_packed(c, N, T);
+  };
+  PackedOut qg, qgt;
+  float* own_am;
+  Carver size;
+  carve(size, qg, qgt, own_am);
+  const Tensor scratch = empty({(int64_t)size.used}, at::kByte, gy);
+  Carver c{static_cast<char*>(scratch.data_ptr())};
+  carve(c, qg, qgt, own_am);
+  const float* am = a.am ? word(*a.am) : a.am_out ? word(*a.am_out) : own_am;
+  if (!a.am) run_amax(gy, const_cast<float*>(am), !a.am_out);
+  run_tile(gy, a.want_x ? &qg : nullptr, a.want_w ? &qgt : nullptr, am, a.signs, a.mode, seed, seed_cols);
+  if (a.want_x) {
+    gx = empty({T, a.K}, at::kBFloat16, gy);
+    run_mm(qg, wt, gx, N, false, 1);
+  }
+  if (a.want_w) {
+    gw = a.gw_out ? *a.gw_out : empty({N, a.K}, a.gw_dtype, gy);
+    run_mm(qgt, xt, gw, T, a.gw_out && !a.overwrite, a.gw_out ? 0 : 1);
+  }
+  return {gx, gw};
+}
+
+Packed packed_of(const Tensor& d, const Tensor& s, const Tensor& gs) {
+  return {d.const_data_ptr(), s.const_data_ptr(), word(gs)};
+}
+// whole [R, C/2] code matrices only: the layer addresses them by their sizes
+void require_packed(const Tensor& d, int64_t R, int64_t C, const char* what) {
+  require_cuda(d);
+  REQUIRE(d.dim() == 2 && d.size(0) == R && d.size(1) * 2 == C && d.is_contiguous(), what);
+}
+
+py::tuple linear_fwd(const Tensor& x, const Tensor& wd, const Tensor& ws, const Tensor& wg, unsigned signs, const OptTensor& am_out) {
+  require_cuda(x);
+  at::NoGradGuard no_grad;
+  const int64_t T = x.size(0), K = x.size(1), N = wd.size(0);
+  require_packed(wd, N, K, "linear_fwd: quantized weight");
+  const Tensor am = am_out ? nvq_amax(x.contiguous(), am_out, false) : nvq_amax(x.contiguous(), std::nullopt, true);
+  PackedTensors xt(K, T, x);
+  const PackedOut o = xt.out();
+  Tensor y = forward_core(x, word(am), packed_of(wd, ws, wg), N, &o, signs);
+  return py::make_tuple(y, am, xt.d, xt.s, xt.gs);
+}
+
+py::tuple linear_bwd(const Tensor& gy_, const Tensor& wd, const Tensor& ws, const Tensor& wg, const Tensor& xd, const Tensor& xs,
+                     const Tensor& xg, py::handle seed, py::handle seed_cols, unsigned signs, int mode, const OptTensor& gw_out,
+                     bool overwrite, bool gw_fp32, const OptTensor& am, const OptTensor& am_out) {
+  require_cuda(gy_); require_cuda(am_out);
+  at::NoGradGuard no_grad;
+  const Tensor gy = gy_.contiguous();
+  REQUIRE(gy.dim() == 2 && gy.scalar_type() == at::kBFloat16, "linear_bwd: bf16 output gradient");
+  BackwardArgs a;
+  a.K = wd.size(0);
+  require_packed(wd, a.K, gy.size(1), "linear_bwd: quantized transposed weight");
+  require_packed(xd, a.K, gy.size(0), "linear_bwd: transposed operand of x");
+  a.signs = signs; a.mode = mode; a.gw_out = gw_out; a.overwrite = overwrite; a.am = am; a.am_out = am_out;
+  a.gw_dtype = gw_fp32 ? at::kFloat : at::kBFloat16;
+  if (gw_out) {
+    require_cuda(gw_out);
+    REQUIRE(gw_out->dim() == 2 && gw_out->size(0) == gy.size(1) && gw_out->size(1) == a.K && gw_out->scalar_type() == at::kFloat &&
+                gw_out->stride(1) == 1, "linear_bwd: gw_out is fp32 [N, K]");
+  }
+  auto [gx, gw] = backward_core(gy, packed_of(wd, ws, wg), packed_of(xd, xs, xg), Seed(seed), Seed(seed_cols), a);
+  return py::make_tuple(gx, gw);
+}
+
+// Offsets inside the one buffer a forward pass keeps for its backward pass.
+struct Kept {
+  PackedOut xt, wt;
+  Kept(Carver& c, int64_t T, int64_t K, int64_t N, bool keep_x, bool keep_w) {
+    if (keep_x) xt = carve_packed(c, K, T);
+    if (keep_w) wt = carve_packed(c, K, N);
+  }
+};
+
+struct Q3 { Tensor d, s, gs; };
+Q3 q_of(py::handle q) {
+  return {py::cast<Tensor>(q.attr("d")), py::cast<Tensor>(q.attr("s")), py::cast<Tensor>(q.attr("gs"))};
+}
+
+struct LinearNode : torch::autograd::Node {
+  torch::autograd::SavedVariable w, kept;       // the weight: only so that an in-place change of it is noticed
+  int64_t T, K, N;
+  unsigned lid, signs;
+  bool keep_x, keep_w;
+  PyObject* cache = nullptr;                    // the layer's WeightCache, or null
+
+  ~LinearNode() override {
+    if (cache && Py_IsInitialized()) {
+      py::gil_scoped_acquire gil;
+      Py_DECREF(cache);
+    }
+  }
+  std::string name() const override { return "FP4LinearBackward"; }
+  void release_variables() override { w.reset_data(); kept.reset_data(); }
+
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    torch::autograd::variable_list out(2);
+    if (!grads[0].defined()) return out;
+    at::NoGradGuard no_grad;
+    w.unpack(getptr());                         // raises when the graph was freed or the weight changed in place
+    const Tensor buf = kept.unpack(getptr());
+    BackwardArgs a;
+    a.K = K; a.signs = signs;
+    a.want_x = task_should_compute_output(0);
+    a.want_w = task_should_compute_output(1);
+    if (!a.want_x && !a.want_w) return out;
+    unsigned seed;
+    Q3 cached;
+    {
+      // the switches as they stand when the backward pass runs
+      py::gil_scoped_acquire gil;
+      const py::object s = lin_ctx.attr("seed");
+      seed = (unsigned)PyLong_AsUnsignedLongLongMask(s.ptr()) * 1000003u + lid * 7919u;
+      if (PyErr_Occurred()) throw py::error_already_set();
+      const py::object dtype = lin_ctx.attr("wgrad_dtype");
+      a.gw_dtype = reinterpret_cast<THPDtype*>(dtype.ptr())->scalar_type;
+      a.mode = py::cast<int>(nvq_module.attr("SR_MODE"));
+      if (cache && a.want_x) cached = q_of(py::handle(cache).attr("qt"));
+    }
+    REQUIRE(a.gw_dtype == at::kFloat || a.gw_dtype == at::kBFloat16, "LinCtx.wgrad_dtype: float32 or bfloat16");
+    Carver c{static_cast<char*>(buf.data_ptr())};
+    const Kept k(c, T, K, N, keep_x, keep_w);
+    Packed wt = k.wt;
+    if (cached.d.defined()) {
+      require_packed(cached.d, K, N, "cached transposed weight");
+      wt = packed_of(cached.d, cached.s, cached.gs);
+    }
+    const Tensor gy = grads[0].contiguous();
+    std::tie(out[0], out[1]) = backward_core(gy, wt, k.xt, Seed(seed), Seed(seed ^ 0x5bd1e995u), a);
+    return out;
+  }
+};
+
+// The layer on x [T, K], w [N, K] -> y [T, N].  With `cache` the quantized weight is taken from it, else W is quantized
+// here: both orientations in one pass when the backward pass will want W^T (one amax and one read of W instead of two
+// of each).  Without gradients only the row operand of x is produced.
+Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py::handle cache, unsigned signs) {
+  require_cuda(x_);
+  const Tensor w_ = w_opt.value_or(Tensor());
+  const bool cached = !cache.is_none();
+  const bool grad = at::GradMode::is_enabled();
+  const bool need_x = grad && x_.requires_grad(), need_w = grad && w_.defined() && w_.requires_grad();
+  REQUIRE(x_.dim() == 2 && x_.scalar_type() == at::kBFloat16 && x_.stride(1) == 1, "linear: x is bf16 [T, K] with contiguous rows");
+  const int64_t T = x_.size(0), K = x_.size(1);
+  REQUIRE(T % 128 == 0 && K % 128 == 0, shape_of(T, K));
+  Tensor y;
+  std::shared_ptr<LinearNode> node;
+  Tensor kept_buf;
+  int64_t N;
+  {
+    at::NoGradGuard no_grad;
+    const Tensor x = x_.detach();
+    Packed qw;
+    Q3 cq;
+    Tensor w;
+    if (cached) {
+      cq = q_of(cache.attr("q"));
+      N = cq.d.size(0);
+      require_packed(cq.d, N, K, "cached weight");
+      qw = packed_of(cq.d, cq.s, cq.gs);
+    } else {
+      REQUIRE(w_.defined(), "linear: no weight");
+      require_cuda(w_);
+      REQUIRE(w_.dim() == 2 && w_.scalar_type() == at::kBFloat16, "quant_w2d: a bf16 matrix");
+      w = w_.contiguous();
+      N = w.size(0);
+      REQUIRE(N % 128 == 0 && w.size(1) == K, shape_of(N, w.size(1)));
+    }
+    const bool keep_w = !cached && need_x;
+    Carver ksize;
+    Kept(ksize, T, K, N, need_w, keep_w);
+    if (need_x || need_w) kept_buf = empty({(int64_t)ksize.used}, at::kByte, x);
+    Carver kc{kept_buf.defined() ? static_cast<char*>(kept_buf.data_ptr()) : nullptr};
+    const Kept kept(kc, T, K, N, need_w, keep_w);
+
+    PackedOut wq;
+    auto carve = [&](Carver& c, float*& am_x, float*& am_w) {
+      am_x = c.take<float>(4);
+      if (!cached) { am_w = c.take<float>(4); wq = carve_packed(c, N, K); }
+    };
+    float *am_x = nullptr, *am_w = nullptr;
+    Carver size;
+    carve(size, am_x, am_w);
+    const Tensor scratch = empty({(int64_t)size.used}, at::kByte, x);
+    Carver c{static_cast<char*>(scratch.data_ptr())};
+    carve(c, am_x, am_w);
+    run_amax(x.contiguous(), am_x);
+    if (!cached) {
+      run_amax(w, am_w);
+      if (keep_w) wq.gs = kept.wt.gs;         // both orientations share one tensor scale, which the backward pass reads
+      run_w2d(w, &wq, keep_w ? &kept.wt : nullptr, am_w);
+      qw = wq;
+    }
+    y = forward_core(x, am_x, qw, N, need_w ? &kept.xt : nullptr, signs);
+  }
+  if (need_x || need_w) {
+    node = std::shared_ptr<LinearNode>(new LinearNode(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x_, w_));
+    node->T = T; node->K = K; node->N = N;
+    node->lid = (unsigned)PyLong_AsUnsignedLongLongMask(lid.ptr());
+    if (PyErr_Occurred()) throw py::error_already_set();
+    node->signs = signs; node->keep_x = need_w; node->keep_w = !cached && need_x;
+    if (cached) { node->cache = cache.ptr(); Py_INCREF(node->cache); }
+    node->w = torch::autograd::SavedVariable(w_, false);
+    node->kept = torch::autograd::SavedVariable(kept_buf, false);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+void bind(const py::dict& addresses, py::object error, py::object lin, py::object nvq, py::object status) {
+#define X(name) lib.name = reinterpret_cast<decltype(lib.name)>(py::cast<uintptr_t>(addresses[#name]));
+  NVFP4_API(X)
+#undef X
+  error_class = error.release();
+  lin_ctx = lin.release();
+  nvq_module = nvq.release();
+  status_word_fn = status.release();
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+  py::register_exception_translator([](std::exception_ptr p) {
+    try {
+      if (p) std::rethrow_exception(p);
+    } catch (const AssertionFailure& e) {
+      PyErr_SetString(PyExc_AssertionError, e.what());
+    } catch (const LibraryError& e) {
+      PyErr_SetString(error_class.ptr(), e.what());
+    }
+  });
+  m.def("bind", &bind);
+  m.def("entry_points", [] {
+    py::list names;
+#define X(name) names.append(#name);
+    NVFP4_API(X)
+#undef X
+    return names;
+  });
+  m.def("amax", &nvq_amax);
+  m.def("quant_rows", &nvq_quant_rows);
+  m.def("quant_cols_rht", &nvq_quant_cols_rht);
+  m.def("quant_rows_cols_rht", &nvq_quant_rows_cols_rht);
+  m.def("quant_w2d", &nvq_quant_w2d);
+  m.def("quant_w2d_into", &nvq_quant_w2d_into);
+  m.def("mm", &nvq_mm);
+  m.def("linear_fwd", &linear_fwd);
+  m.def("linear_bwd", &linear_bwd);
+  m.def("linear_apply", &linear_apply);
+}

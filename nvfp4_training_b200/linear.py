@@ -13,6 +13,7 @@ quantizes a weight once per optimizer step instead of twice per microbatch -- th
 import torch
 import torch.nn as nn
 
+from . import _lib as L
 from . import nvq
 
 
@@ -56,10 +57,10 @@ def linear_fwd(x, qw, keep_xt=False, signs=_RHT_SIGNS, am_out=None):
     the same pass over x and returned as a third value, so the backward pass neither re-reads nor
     has to keep x.  `am_out`: a zeroed device word that receives amax(x) (callers that clear many such words with
     one fill save a fill per call)."""
-    am = nvq.amax(x.contiguous()) if am_out is None else nvq.amax(x.contiguous(), out=am_out, clear=False)
     if keep_xt and _tileable(x):
-        qx, qxt = nvq.quant_rows_cols_rht(x, signs, am=am)
-        return nvq.mm(qx, qw), am, qxt
+        y, am, *qxt = (L._host or L.host()).linear_fwd(x, qw.d, qw.s, qw.gs, signs & 0xFFFF, am_out)
+        return y, am, nvq.Q(*qxt)
+    am = nvq.amax(x.contiguous()) if am_out is None else nvq.amax(x.contiguous(), out=am_out, clear=False)
     y = nvq.mm(nvq.quant_rows(x, am=am), qw)
     return (y, am, nvq.quant_cols_rht(x, signs, am=am)) if keep_xt else (y, am)
 
@@ -81,6 +82,9 @@ def linear_bwd(x, am_x, gy, qwt, seed, seed_cols, gw_out=None, wgrad_dtype=torch
     `gw_owners`: data-parallel reduce-scatter in the weight-gradient GEMM's epilogue: the addresses of `gw_out` on every
     rank; the product is added into the row slab each rank owns (`nvq.mm(owners=)`; `overwrite` is then ignored: the
     caller clears the slabs once per step)."""
+    if qxt is not None and gw_owners is None and (gw_out is None or wgrad_stream is None) and _tileable(gy):
+        return (L._host or L.host()).linear_bwd(gy, qwt.d, qwt.s, qwt.gs, qxt.d, qxt.s, qxt.gs, seed, seed_cols, signs & 0xFFFF,
+                                                sr_mode or nvq.SR_MODE, gw_out, overwrite, wgrad_dtype == torch.float32, am_gy, am_out)
     gy = gy.contiguous()
     ag = am_gy if am_gy is not None else (nvq.amax(gy) if am_out is None else nvq.amax(gy, out=am_out, clear=False))
     if _tileable(gy):
@@ -111,27 +115,16 @@ def linear_bwd(x, am_x, gy, qwt, seed, seed_cols, gw_out=None, wgrad_dtype=torch
     return gx, gw
 
 
-class FP4LinearFn(torch.autograd.Function):
-    """x [T, K] bf16, w [N, K] bf16 -> y [T, N] bf16 (llm-1b/model.py:45-69)."""
+class FP4LinearFn:
+    """x [T, K] bf16, w [N, K] bf16 -> y [T, N] bf16 (llm-1b/model.py:45-69), an autograd function in native code
+    (`linear_apply` of csrc/host.cpp).  `cache`: a `WeightCache`, else w is quantized here.  The forward pass keeps x only
+    as the transposed RHT operand that wgrad needs (0.56 byte per element), and W^T's operand when W was quantized here;
+    the backward pass reads `LinCtx`, `nvq.SR_MODE` and `cache.qt` as they stand when it runs.  Gradients nobody asked
+    for, and operands only they would need, are not computed."""
 
     @staticmethod
-    def forward(ctx, x, w, lid, cache=None):
-        qw = cache.q if cache is not None else nvq.quant_w2d(w, want=(True, False))[0]
-        # the backward pass needs x only as the transposed RHT operand: keep that (0.56 byte per
-        # element) instead of x
-        y, am, qxt = linear_fwd(x, qw, keep_xt=True)
-        ctx.save_for_backward(w, am, qxt.d, qxt.s, qxt.gs)
-        ctx.lid, ctx.cache = lid, cache
-        return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        w, am, xd, xs, xg = ctx.saved_tensors
-        seed = sr_seed(ctx.lid)
-        qwt = ctx.cache.qt if ctx.cache is not None else nvq.quant_w2d(w, want=(False, True))[1]
-        gx, gw = linear_bwd(None, am, gy, qwt, seed, seed ^ 0x5bd1e995, wgrad_dtype=LinCtx.wgrad_dtype,
-                            qxt=nvq.Q(xd, xs, xg))
-        return gx, gw, None, None
+    def apply(x, w, lid, cache=None):
+        return (L._host or L.host()).linear_apply(x, w, lid, cache, _RHT_SIGNS)
 
 
 class Linear(nn.Module):
@@ -151,12 +144,12 @@ class Linear(nn.Module):
             self.cache.refresh()
 
     def forward(self, x):
-        shp = x.shape
-        x2 = x.reshape(-1, shp[-1])
+        flat = x.dim() == 2
+        x2 = x if flat else x.reshape(-1, x.shape[-1])
         if LinCtx.fp4:
             if self.cache is not None and self.cache.q is None:
                 self.cache.refresh()
             y = FP4LinearFn.apply(x2, self.weight, self.lid, self.cache)
         else:
             y = x2 @ self.weight.t()
-        return y.view(*shp[:-1], -1)
+        return y if flat else y.view(*x.shape[:-1], -1)

@@ -1,0 +1,63 @@
+"""The native host path (csrc/host.cpp): the autograd linear gives the same bits whichever gradients are asked for, with
+and without a weight cache, and keeps autograd's rules (versions, freed graphs, error types)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(T, K, N, cache):
+    from nvfp4_training_b200.linear import Linear
+    torch.manual_seed(T + K + N)
+    with torch.device("cuda"):
+        lin = Linear(K, N, std=0.02, cache_weights=cache)
+    lin = lin.bfloat16()
+    lin.lid = 3
+    lin.refresh()
+    x = torch.randn(T, K, device="cuda").bfloat16()
+    gy = (torch.randn(T, N, device="cuda") * 1e-3).bfloat16()
+    return lin, x, gy
+
+
+@pytest.mark.parametrize("cache", [False, True])
+@pytest.mark.parametrize("T,K,N", [(128, 128, 128), (384, 256, 640)])
+def test_linear_gradients_are_the_same_whichever_are_wanted(T, K, N, cache):
+    lin, x, gy = _layer(T, K, N, cache)
+    xg = x.clone().requires_grad_(True)
+    y = lin(xg)
+    gx, gw = torch.autograd.grad(y, (xg, lin.weight), gy, retain_graph=True)
+    again = torch.autograd.grad(y, (xg, lin.weight), gy)
+    assert torch.equal(gx, again[0]) and torch.equal(gw, again[1])
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(y, (xg, lin.weight), gy)              # the graph has been freed
+    with torch.no_grad():
+        assert torch.equal(lin(xg), y)
+    assert torch.equal(torch.autograd.grad(lin(x), lin.weight, gy)[0], gw)           # x needs no gradient
+    assert torch.equal(torch.autograd.grad(lin(xg), xg, gy)[0], gx)                  # only x's asked for
+    lin.weight.requires_grad_(False)                                                 # frozen weight
+    y2 = lin(xg)
+    assert torch.equal(y2, y) and torch.equal(torch.autograd.grad(y2, xg, gy)[0], gx)
+    y3 = lin(xg.view(2, T // 2, K))                                                  # leading dimensions are flattened
+    assert y3.shape == (2, T // 2, N) and torch.equal(y3.view(T, N), y)
+
+
+def test_linear_notices_an_in_place_weight_change():
+    lin, x, gy = _layer(128, 128, 256, False)
+    y = lin(x)
+    with torch.no_grad():
+        lin.weight.mul_(2)
+    with pytest.raises(RuntimeError):
+        torch.autograd.grad(y, lin.weight, gy)
+
+
+def test_host_errors_keep_their_types():
+    from nvfp4_training_b200 import _lib, nvq
+    with pytest.raises(_lib.Nvfp4Error):
+        nvq.amax(torch.zeros(8, dtype=torch.bfloat16))
+    with pytest.raises(AssertionError):
+        nvq.quant_rows(torch.zeros(100, 64, dtype=torch.bfloat16, device="cuda"))
+    with pytest.raises(AssertionError):
+        nvq.quant_rows(torch.zeros(128, 64, device="cuda"))
+    q = nvq.quant_rows(torch.ones(128, 64, dtype=torch.bfloat16, device="cuda"))
+    with pytest.raises(AssertionError):
+        nvq.mm(q, nvq.quant_rows(torch.ones(128, 128, dtype=torch.bfloat16, device="cuda")))
