@@ -42,6 +42,7 @@ extern "C" {
 
 #define NVFP4_SCALES_SWIZZLED  0
 #define NVFP4_SCALES_LINEAR    1
+#define NVFP4_SCALES_BOTH      2   /* the row-major bytes, then as many swizzled ones (a buffer of twice the size) */
 
 #define NVFP4_DTYPE_BF16       0
 #define NVFP4_DTYPE_FP32       1
@@ -79,6 +80,12 @@ int nvfp4_amax_bf16(const void* x, long long n, float* out, void* stream);
  * the fill the amax kernel follows the previous kernel of the stream directly (one graph node less per call).
  */
 int nvfp4_amax_bf16_update(const void* x, long long n, float* out, void* stream);
+
+/*
+ * max|x| of a contiguous FP32 tensor into *out, for FP32 master weights (`x.abs().amax()` of llm-1b/fp4ops.py:25-26).  A
+ * NaN anywhere gives NaN.  Requires n % 4 == 0, x 16-byte aligned.  n == 0 gives 0.
+ */
+int nvfp4_amax_f32(const float* x, long long n, float* out, void* stream);
 
 /*
  * Programmatic dependent launch of this library's amax, one-read quantizer and GEMM kernels: when on, such a kernel
@@ -132,7 +139,7 @@ int nvfp4_quant_cols_rht(const void* x, int M, int C, void* codes, void* scales,
  *     tensor memory, the quantizing warps read it with tcgen05.ld.  One documented difference: an input
  *     that is exactly -0 gives code 0x0 (the scalar kernels and the reference's convert give 0x8);
  *   - scalar (any other accepted shape): TMA tiles of 128 x 64 in a shared-memory ring, read by the
- *     quantizing warps.
+ *     quantizing warps.  NVFP4_SCALES_BOTH is written by the first kernel only.
  * Requires M % 128 == 0, C % 64 == 0 (C % 128 == 0 with SWIZZLED scales and codes_c), ldx % 8 == 0,
  * x and codes_c 16-byte aligned, codes_r and scales_c 8-byte aligned.  A wait that expires inside the kernel (1 s) is reported by nvfp4_quant_tile_status.
  */

@@ -13,7 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libnvfp4_b200.so")
 HOST_PATH = os.path.join(HERE, "_host.so")
 
-SCALES_SWIZZLED, SCALES_LINEAR = 0, 1
+SCALES_SWIZZLED, SCALES_LINEAR, SCALES_BOTH = 0, 1, 2
 DTYPE_BF16, DTYPE_FP32 = 0, 1
 ROUND_NEAREST, ROUND_SR_DITHER, ROUND_SR_DITHER_K, ROUND_SR_HW = 0, 1, 2, 3
 ALPHA_ONE, ALPHA_GS, ALPHA_AMAX, ALPHA_ROW = 0, 1, 2, 3
@@ -27,6 +27,7 @@ SIGNATURES = {
     "nvfp4_error_string": (_c.c_char_p, [_i]),
     "nvfp4_amax_bf16": (_i, [_vp, _ll, _vp, _vp]),
     "nvfp4_amax_bf16_update": (_i, [_vp, _ll, _vp, _vp]),
+    "nvfp4_amax_f32": (_i, [_vp, _ll, _vp, _vp]),
     "nvfp4_set_pdl": (_i, [_i]),
     "nvfp4_gemm_reset_scheduler": (_i, []),
     "nvfp4_gemm_set_scheduler": (_i, [_i]),

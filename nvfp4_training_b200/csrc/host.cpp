@@ -36,7 +36,8 @@ namespace {
 // ------------------------------------------------------------------------------------------ library entry points
 #define NVFP4_API(X)                                                                                                        \
   X(nvfp4_amax_bf16) X(nvfp4_amax_bf16_update) X(nvfp4_quant_rows) X(nvfp4_quant_cols_rht) X(nvfp4_quant_tile)             \
-  X(nvfp4_quant_w2d) X(nvfp4_gemm) X(nvfp4_error_string)
+  X(nvfp4_quant_w2d) X(nvfp4_gemm) X(nvfp4_error_string) X(nvfp4_amax_f32) X(nvfp4_swizzle_scales) X(nvfp4_emit_rows)        \
+  X(nvfp4_emit_cols) X(nvfp4_rms_emit) X(nvfp4_swiglu_emit) X(nvfp4_mom_acc)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
   NVFP4_API(X)
@@ -544,6 +545,221 @@ Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py
   return y;
 }
 
+
+// ------------------------------------------------------------------------------------------ fp4ops operators
+// max|x| as FP32 [1]: one kernel for contiguous bf16 and FP32, torch's reduction for everything else
+Tensor k_amax(const Tensor& x) {
+  at::NoGradGuard no_grad;
+  const bool bf16 = x.scalar_type() == at::kBFloat16, f32 = x.scalar_type() == at::kFloat;
+  if (x.is_cuda() && (bf16 || f32) && x.is_contiguous() && x.numel() > 0 && x.numel() % (bf16 ? 8 : 4) == 0 &&
+      (bf16 || (reinterpret_cast<uintptr_t>(x.const_data_ptr()) & 15u) == 0)) {
+    Tensor out = empty({1}, at::kFloat, x);
+    if (bf16) run_amax(x, out.data_ptr<float>());
+    else check(lib.nvfp4_amax_f32(static_cast<const float*>(x.const_data_ptr()), x.numel(), out.data_ptr<float>(), stream()), "amax");
+    return out;
+  }
+  return x.abs().amax().to(at::kFloat).reshape({1});
+}
+Tensor k_amax_or(const OptTensor& am, const Tensor& x) { return am ? *am : k_amax(x); }
+
+// Row-major scales [R, C16]; where whole swizzled tiles exist the same buffer also holds the swizzled bytes, which the
+// quantizers then write in the same pass (`sw`: what the tensor core reads, so that a GEMM on the result has nothing
+// left to convert).
+struct LinearScales {
+  Tensor s;
+  OptTensor sw;
+  int layout;
+  LinearScales(int64_t R, int64_t C, bool both, const Tensor& like) : layout(both ? NVFP4_SCALES_BOTH : NVFP4_SCALES_LINEAR) {
+    const int64_t n = R * (C / 16);
+    if (both) {
+      const Tensor buf = empty({2 * n}, at::kByte, like);
+      s = buf.as_strided({R, C / 16}, {C / 16, 1}, 0);
+      sw = buf.as_strided({n}, {1}, n);
+    } else {
+      s = empty({R, C / 16}, at::kByte, like);
+    }
+  }
+};
+bool whole_tiles(int64_t R, int64_t C) { return R % 128 == 0 && C % 128 == 0 && R > 0 && C > 0; }
+
+py::tuple k_quant_rows(const Tensor& x_, int mode, py::handle seed_, const OptTensor& am_) {
+  require_cuda(x_);
+  at::NoGradGuard no_grad;
+  REQUIRE(x_.dim() == 2 && x_.scalar_type() == at::kBFloat16 && x_.size(1) % 16 == 0, "quant_rows: a bf16 matrix, columns a multiple of 16");
+  const Tensor x = x_.contiguous();
+  const int64_t R = x.size(0), C = x.size(1);
+  const Seed seed(seed_);
+  const Tensor am = k_amax_or(am_, x);
+  Tensor d = empty({R, C / 2}, at::kByte, x);
+  LinearScales s(R, C, whole_tiles(R, C), x);
+  check(lib.nvfp4_quant_rows(x.const_data_ptr(), C, (int)R, (int)C, d.data_ptr(), s.s.data_ptr(), s.layout, word(am), nullptr, mode,
+                             seed.host, seed.dev, stream()), "quant_rows");
+  return py::make_tuple(d, s.s, am, s.sw);
+}
+
+py::tuple k_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, py::handle seed_, const OptTensor& am_) {
+  require_cuda(x_);
+  at::NoGradGuard no_grad;
+  const Tensor x = x_.contiguous();
+  REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.size(0) % 16 == 0 && x.size(1) % 8 == 0,
+          "quant_cols_rht: a bf16 matrix, rows a multiple of 16, columns of 8");
+  const int64_t M = x.size(0), C = x.size(1);
+  const Seed seed(seed_);
+  const Tensor am = k_amax_or(am_, x);
+  Tensor d = empty({C, M / 2}, at::kByte, x);
+  LinearScales s(C, M, whole_tiles(C, M), x);
+  check(lib.nvfp4_quant_cols_rht(x.const_data_ptr(), (int)M, (int)C, d.data_ptr(), s.s.data_ptr(), s.layout, word(am), nullptr, signs,
+                                 mode, seed.host, seed.dev, stream()), "quant_cols_rht");
+  return py::make_tuple(d, s.s, am, s.sw);
+}
+
+py::tuple k_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py::handle seed_, py::handle seed_cols_, const OptTensor& am_) {
+  require_cuda(x);
+  at::NoGradGuard no_grad;
+  REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "quant_rows_cols_rht: a bf16 matrix with contiguous rows");
+  const int64_t M = x.size(0), C = x.size(1);
+  REQUIRE(M % 128 == 0 && C % 64 == 0, shape_of(M, C));
+  const Seed seed(seed_), seed_cols(seed_cols_);
+  const Tensor am = k_amax_or(am_, x);
+  const bool both = whole_tiles(M, C);
+  Tensor dr = empty({M, C / 2}, at::kByte, x), dc = empty({C, M / 2}, at::kByte, x);
+  LinearScales sr(M, C, both, x), sc(C, M, both, x);
+  check(lib.nvfp4_quant_tile(x.const_data_ptr(), x.stride(0), (int)M, (int)C, dr.data_ptr(), sr.s.data_ptr(), dc.data_ptr(),
+                             sc.s.data_ptr(), sr.layout, word(am), nullptr, nullptr, signs, mode, seed.host, seed_cols.host,
+                             seed.dev, seed_cols.dev, stream()), "quant_tile");
+  return py::make_tuple(py::make_tuple(dr, sr.s, am, sr.sw), py::make_tuple(dc, sc.s, am, sc.sw));
+}
+
+Tensor k_swizzle(const Tensor& s, const OptTensor& out_) {
+  const int64_t R = s.size(0), C16 = s.size(1);
+  REQUIRE(R % 128 == 0 && C16 % 4 == 0, shape_of(R, C16));
+  Tensor out = out_ ? *out_ : empty({R * C16}, at::kByte, s);
+  check(lib.nvfp4_swizzle_scales(s.const_data_ptr(), s.stride(0), (int)R, (int)C16, out.data_ptr(), stream()), "swizzle_scales");
+  return out;
+}
+
+// Buffers of one weight: (d, s, sw) of W and of W^T and the shared amax.
+py::tuple k_w2d_buffers(const Tensor& w) {
+  require_cuda(w);
+  REQUIRE(w.dim() == 2 && w.scalar_type() == at::kFloat && w.size(0) % 16 == 0 && w.size(1) % 16 == 0, "quant_w2d: an FP32 matrix, sides multiples of 16");
+  const int64_t N = w.size(0), K = w.size(1);
+  const bool both = whole_tiles(N, K);
+  LinearScales s(N, K, both, w), st(K, N, both, w);
+  return py::make_tuple(empty({N, K / 2}, at::kByte, w), s.s, s.sw, empty({K, N / 2}, at::kByte, w), st.s, st.sw, empty({1}, at::kFloat, w));
+}
+
+void k_quant_w2d(const Tensor& w_, const Tensor& d, const Tensor& s, const OptTensor& sw, const Tensor& dt, const Tensor& st,
+                 const OptTensor& stw, const Tensor& am) {
+  require_cuda(w_);
+  at::NoGradGuard no_grad;
+  REQUIRE(w_.dim() == 2 && w_.scalar_type() == at::kFloat && w_.size(0) % 16 == 0 && w_.size(1) % 16 == 0, "quant_w2d: an FP32 matrix, sides multiples of 16");
+  const Tensor w = w_.contiguous();
+  const int64_t N = w.size(0), K = w.size(1);
+  if (w.numel() > 0 && w.numel() % 4 == 0 && (reinterpret_cast<uintptr_t>(w.const_data_ptr()) & 15u) == 0)
+    check(lib.nvfp4_amax_f32(static_cast<const float*>(w.const_data_ptr()), w.numel(), static_cast<float*>(am.data_ptr()), stream()), "amax");
+  else
+    am.copy_(k_amax(w));
+  // the kernel writes both layouts where the swizzled bytes follow the row-major ones
+  auto follows = [](const Tensor& a, const OptTensor& b) {
+    return b && static_cast<const char*>(a.const_data_ptr()) + a.numel() == static_cast<const char*>(b->const_data_ptr());
+  };
+  const bool both = whole_tiles(N, K) && follows(s, sw) && follows(st, stw);
+  check(lib.nvfp4_quant_w2d(w.const_data_ptr(), NVFP4_DTYPE_FP32, (int)N, (int)K, d.data_ptr(), s.data_ptr(), dt.data_ptr(),
+                            st.data_ptr(), both ? NVFP4_SCALES_BOTH : NVFP4_SCALES_LINEAR, word(am), nullptr, stream()), "quant_w2d");
+  if (!both) {
+    if (sw) k_swizzle(s, sw);
+    if (stw) k_swizzle(st, stw);
+  }
+}
+
+// a [M, K], b [N, K] with row-major scales and, where they are known, swizzled ones
+Tensor k_gemm(const Tensor& ad, const Tensor& as, const OptTensor& asw, const Tensor& aam, float ak, const Tensor& bd, const Tensor& bs,
+              const OptTensor& bsw, const Tensor& bam, float bk, const OptTensor& out_, int splitk) {
+  require_cuda(ad); require_cuda(bd);
+  at::NoGradGuard no_grad;
+  const int64_t M = ad.size(0), N = bd.size(0), K = as.size(1) * 16;
+  REQUIRE(M % 128 == 0 && N % 128 == 0 && K % 128 == 0, shape_of(M, N) + ", " + std::to_string(K));
+  const bool fp32 = splitk != 1 || out_;
+  Tensor out;
+  if (!fp32) {
+    out = empty({M, N}, at::kBFloat16, ad);
+  } else {
+    out = out_ ? *out_ : at::zeros({M, N}, ad.options().dtype(at::kFloat));
+    REQUIRE(out.scalar_type() == at::kFloat && out.stride(1) == 1, "gemm: out is FP32 with contiguous rows");
+  }
+  const Tensor sa = asw ? *asw : k_swizzle(as, std::nullopt), sb = bsw ? *bsw : k_swizzle(bs, std::nullopt);
+  check(lib.nvfp4_gemm(ad.const_data_ptr(), sa.const_data_ptr(), ad.stride(0), bd.const_data_ptr(), sb.const_data_ptr(), bd.stride(0),
+                       out.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16, out.stride(0), (int)M, (int)N, (int)K,
+                       NVFP4_ALPHA_AMAX, word(aam), word(bam), ak, bk, fp32, splitk, status_word(ad), stream()), "gemm");
+  return out;
+}
+
+// ------------------------------------------------------------------------------------------ operand emitters
+const unsigned* words(const OptTensor& t) { return static_cast<const unsigned*>(cptr(t)); }
+
+void e_rows(const Tensor& x, const Tensor& d, const Tensor& s, const Tensor& rs, const OptTensor& rng, int sr, unsigned salt) {
+  require_cuda(x); require_cuda(d); require_cuda(s); require_cuda(rs);
+  const int64_t T = x.size(0), C = x.size(1);
+  REQUIRE(x.scalar_type() == at::kBFloat16 && x.stride(1) == 1 && C % 256 == 0, "row_emit: bf16, contiguous rows, columns a multiple of 256");
+  REQUIRE(T % 128 == 0, std::to_string(T));
+  if (sr) REQUIRE(rng && rng->is_cuda() && rng->element_size() == 4, "row_emit: stochastic rounding needs rng");
+  check(lib.nvfp4_emit_rows(x.const_data_ptr(), x.stride(0), (int)T, (int)C, d.data_ptr(), s.data_ptr(), static_cast<float*>(rs.data_ptr()),
+                            sr, words(rng), salt, stream()), "emit_rows");
+}
+
+void e_cols(const Tensor& x, const Tensor& d, const Tensor& s, const Tensor& use, const Tensor& cur, const Tensor& rng, int sr, unsigned salt) {
+  require_cuda(x); require_cuda(d); require_cuda(s); require_cuda(use); require_cuda(cur); require_cuda(rng);
+  const int64_t M = x.size(0), C = x.size(1);
+  REQUIRE(x.scalar_type() == at::kBFloat16 && x.stride(1) == 1 && M % 256 == 0 && C % 64 == 0, "col_emit: bf16, contiguous rows, tokens a multiple of 256");
+  REQUIRE(C % 128 == 0, std::to_string(C));          // swizzled scale tiles of 128 columns are written whole
+  REQUIRE(rng.element_size() == 4 && rng.numel() >= 2 && cur.element_size() == 4, "col_emit: rng holds two 32-bit words, amax_cur one");
+  check(lib.nvfp4_emit_cols(x.const_data_ptr(), x.stride(0), (int)M, (int)C, d.data_ptr(), s.data_ptr(), word(use),
+                            static_cast<unsigned*>(cur.data_ptr()), sr, words(rng), salt, stream()), "emit_cols");
+}
+
+void e_rms(const Tensor& x, const Tensor& w, const OptTensor& d, const OptTensor& s, const OptTensor& rs, const OptTensor& h,
+           const OptTensor& rstd, const OptTensor& y, const OptTensor& ys, const OptTensor& ygw, const OptTensor& xout, float eps) {
+  const int64_t T = x.size(0), D = x.size(1);
+  REQUIRE(x.scalar_type() == at::kBFloat16 && x.is_contiguous() && w.scalar_type() == at::kBFloat16 && w.numel() == D, "rms_emit: x, w");
+  require_cuda(x); require_cuda(w);
+  if (y) {
+    REQUIRE(y->sizes() == x.sizes() && y->is_contiguous() && ys && ygw && xout, "rms_emit: y comes with ys, ygw and xout");
+    REQUIRE(xout->sizes() == x.sizes() && xout->is_contiguous() && ys->scalar_type() == at::kFloat && ygw->scalar_type() == at::kFloat, "rms_emit: xout, ys, ygw");
+  }
+  if (d) REQUIRE(T % 128 == 0 && d->size(0) == T && d->size(1) == D / 2, "rms_emit: q");
+  if (h) REQUIRE(h->sizes() == x.sizes() && h->is_contiguous() && h->scalar_type() == at::kBFloat16, "rms_emit: h");
+  auto p = [](const OptTensor& t) { return t ? t->data_ptr() : nullptr; };
+  check(lib.nvfp4_rms_emit(x.const_data_ptr(), cptr(y), static_cast<const float*>(cptr(ys)), static_cast<const float*>(cptr(ygw)), p(xout),
+                           w.const_data_ptr(), p(h), p(d), p(s), static_cast<float*>(p(rs)), static_cast<float*>(p(rstd)), (int)T, (int)D,
+                           eps, stream()), "rms_emit");
+}
+
+void e_swiglu(const Tensor& gu, const Tensor& rs_in, const Tensor& gw, const OptTensor& d, const OptTensor& s, const OptTensor& rs,
+              const OptTensor& a, const OptTensor& a_f32) {
+  const int64_t T = gu.size(0), F2 = gu.size(1), F = F2 / 2;
+  REQUIRE(gu.scalar_type() == at::kBFloat16 && gu.is_contiguous() && F2 % 512 == 0, "swiglu_emit: gu");
+  REQUIRE(rs_in.scalar_type() == at::kFloat && rs_in.numel() == T && gw.scalar_type() == at::kFloat, "swiglu_emit: rs_in, gw");
+  require_cuda(gu); require_cuda(rs_in); require_cuda(gw);
+  if (d) REQUIRE(T % 128 == 0 && d->size(0) == T && d->size(1) == F / 2, "swiglu_emit: q");
+  auto p = [](const OptTensor& t) { return t ? t->data_ptr() : nullptr; };
+  check(lib.nvfp4_swiglu_emit(gu.const_data_ptr(), word(rs_in), word(gw), (int)F, p(a), static_cast<float*>(p(a_f32)), p(d), p(s),
+                              static_cast<float*>(p(rs)), (int)T, stream()), "swiglu_emit");
+}
+
+void e_mom(const Tensor& m, const Tensor& g, const Tensor& alpha, float scale, const Tensor& rng, unsigned salt) {
+  const int64_t n = m.numel();
+  REQUIRE(n % 8 == 0 && g.numel() == n && m.scalar_type() == at::kBFloat16 && g.scalar_type() == at::kBFloat16, "mom_acc: bf16 m and g of one size");
+  REQUIRE(m.is_contiguous() && g.is_contiguous() && alpha.scalar_type() == at::kFloat, "mom_acc: contiguous m and g, FP32 alpha");
+  require_cuda(m); require_cuda(g); require_cuda(alpha); require_cuda(rng);
+  check(lib.nvfp4_mom_acc(m.data_ptr(), g.const_data_ptr(), word(alpha), scale, n, words(rng), salt, stream()), "mom_acc");
+}
+
+// raw = A B^T with block scales only (alpha_mode ONE), or times the words of `pa`, `pb`
+Tensor e_mm(const Tensor& ad, const Tensor& as, const Tensor& bd, const Tensor& bs, bool fp32, int alpha_mode, const OptTensor& pa,
+            const OptTensor& pb, const OptTensor& out, bool accumulate, int splitk) {
+  return gemm(ad, as, bd, bs, out, fp32, alpha_mode, pa, pb, 1.f, 1.f, accumulate, splitk, "gemm");
+}
+
 void bind(const py::dict& addresses, py::object error, py::object lin, py::object nvq, py::object status) {
 #define X(name) lib.name = reinterpret_cast<decltype(lib.name)>(py::cast<uintptr_t>(addresses[#name]));
   NVFP4_API(X)
@@ -584,4 +800,18 @@ PYBIND11_MODULE(_host, m) {
   m.def("linear_fwd", &linear_fwd);
   m.def("linear_bwd", &linear_bwd);
   m.def("linear_apply", &linear_apply);
+  m.def("k_amax", &k_amax);
+  m.def("k_quant_rows", &k_quant_rows);
+  m.def("k_quant_cols_rht", &k_quant_cols_rht);
+  m.def("k_quant_rows_cols_rht", &k_quant_rows_cols_rht);
+  m.def("k_swizzle", &k_swizzle);
+  m.def("k_w2d_buffers", &k_w2d_buffers);
+  m.def("k_quant_w2d", &k_quant_w2d);
+  m.def("k_gemm", &k_gemm);
+  m.def("e_rows", &e_rows);
+  m.def("e_cols", &e_cols);
+  m.def("e_rms", &e_rms);
+  m.def("e_swiglu", &e_swiglu);
+  m.def("e_mom", &e_mom);
+  m.def("e_mm", &e_mm);
 }

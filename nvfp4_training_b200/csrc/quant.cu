@@ -3,18 +3,12 @@
 // 128-bit coalesced loads, register-resident blocks, warp shuffles for exchanges/reductions.
 #include <stdlib.h>
 
+#include <mutex>
+#include <unordered_map>
+
 #include "common.cuh"
 
 namespace nvfp4 {
-
-__device__ __forceinline__ void unpack8(const uint4& q, float* f) {
-  const u32 w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    f[2 * i] = __uint_as_float(w[i] << 16);
-    f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
-}
 
 __device__ __forceinline__ uint4 ldg128(const void* p) {
   uint4 v;
@@ -24,56 +18,78 @@ __device__ __forceinline__ uint4 ldg128(const void* p) {
 }
 
 // ------------------------------------------------------------------------------------------ amax
-// max|x| via atomicMax on the float bit pattern (non-negative floats order like unsigned ints).
 __device__ __forceinline__ uint4 ld_cg_128(const uint4* p) {
   uint4 v;
   asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 
-__global__ void __launch_bounds__(256) amax_bf16_kernel(const uint4* __restrict__ x, long long n8, float* out) {
+// Meeting point of the blocks of one launch: running maximum and number of blocks done, both zero between launches.
+struct AmaxSlot { u32 bits, done; };
+constexpr int kAmaxSlots = 1024;
+__device__ AmaxSlot g_amax_slots[kAmaxSlots];
+
+// Running maximum of |x| as integer bit patterns (non-negative floats order like unsigned ints): bf16 values in both
+// halves of a word, FP32 values whole.
+template <bool F32>
+__device__ __forceinline__ u32 amax_take(u32 m, const uint4& v) {
+  if (F32) return max(max(m, v.x & 0x7FFFFFFFu), max(max(v.y & 0x7FFFFFFFu, v.z & 0x7FFFFFFFu), v.w & 0x7FFFFFFFu));
+  m = __vmaxu2(m, v.x & 0x7FFF7FFFu); m = __vmaxu2(m, v.y & 0x7FFF7FFFu);
+  m = __vmaxu2(m, v.z & 0x7FFF7FFFu);
+  return __vmaxu2(m, v.w & 0x7FFF7FFFu);
+}
+
+// HBM-bound: 6.8 TB/s on tensors of 300 MB and more.  With a slot the launch needs no cleared output: every block
+// raises the slot and the last one to arrive moves the result to `out` and leaves the slot zero.  (A memset in front of
+// the kernel cost 1.4 us of its own and a launch gap, against 2-6 us of kernel on tensors of up to 16 MB.)
+template <bool F32>
+__global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, long long nv, float* out, AmaxSlot* slot) {
   pdl_trigger();
   pdl_wait();
-  u32 m = 0u;  // running max of |x| as bf16 bit patterns in both halves of a word
+  u32 m = 0u;
   const long long stride = (long long)gridDim.x * blockDim.x;
   // batches of four loads in flight per thread.  The last, partial batch clamps the indices past the end to the last
   // element (a maximum does not mind reading it again) rather than walking one load at a time: on a 33 MB tensor a
   // thread has seven loads, and three of them in sequence cost more than the first four together.
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + 3 * stride < n8; i += 4 * stride) {
+  for (; i + 3 * stride < nv; i += 4 * stride) {
     uint4 v[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) v[j] = ld_cg_128(x + i + j * stride);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      m = __vmaxu2(m, v[j].x & 0x7FFF7FFFu); m = __vmaxu2(m, v[j].y & 0x7FFF7FFFu);
-      m = __vmaxu2(m, v[j].z & 0x7FFF7FFFu); m = __vmaxu2(m, v[j].w & 0x7FFF7FFFu);
-    }
+    for (int j = 0; j < 4; j++) m = amax_take<F32>(m, v[j]);
   }
-  if (i < n8) {
-    const long long last = n8 - 1;
+  if (i < nv) {
+    const long long last = nv - 1;
     uint4 v[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) v[j] = ld_cg_128(x + min(i + j * stride, last));
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      m = __vmaxu2(m, v[j].x & 0x7FFF7FFFu); m = __vmaxu2(m, v[j].y & 0x7FFF7FFFu);
-      m = __vmaxu2(m, v[j].z & 0x7FFF7FFFu); m = __vmaxu2(m, v[j].w & 0x7FFF7FFFu);
-    }
+    for (int j = 0; j < 4; j++) m = amax_take<F32>(m, v[j]);
   }
-  u32 mm = max(m & 0xFFFFu, m >> 16);
-  // NaN patterns (> 0x7F80) count as +inf
-  mm = min(mm, 0x7F80u);
-#pragma unroll
-  for (int o = 16; o; o >>= 1) mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+  // bf16: NaN patterns (> 0x7F80) count as +inf;  FP32: a NaN is larger than every number and stays
+  u32 mm = F32 ? m : min(max(m & 0xFFFFu, m >> 16), 0x7F80u) << 16;
+  mm = __reduce_max_sync(0xffffffffu, mm);
   __shared__ u32 sm[8];
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mm;
   __syncthreads();
   if (threadIdx.x < 32) {
-    mm = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0u;
-#pragma unroll
-    for (int o = 4; o; o >>= 1) mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-    if (threadIdx.x == 0 && mm) atomicMax(reinterpret_cast<unsigned*>(out), mm << 16);
+    mm = __reduce_max_sync(0xffffffffu, sm[threadIdx.x & 7]);
+    if (threadIdx.x == 0) {
+      if (!slot) {
+        if (mm) atomicMax(reinterpret_cast<unsigned*>(out), mm);
+      } else if (gridDim.x == 1) {
+        *out = __uint_as_float(mm);
+      } else {
+        if (mm) atomicMax(&slot->bits, mm);
+        __threadfence();
+        if (atomicAdd(&slot->done, 1u) == gridDim.x - 1) {
+          __threadfence();
+          *out = __uint_as_float(atomicExch(&slot->bits, 0u));
+          atomicExch(&slot->done, 0u);
+        }
+      }
+    }
   }
 }
 
@@ -98,12 +114,13 @@ __device__ __forceinline__ Block32 load_block(const __nv_bfloat16* p) {
 template <int ROUNDING, bool WIDE>
 __global__ void __launch_bounds__(256, 4) quant_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
                                                           uint2* __restrict__ codes, unsigned char* __restrict__ scales,
-                                                          const float* __restrict__ amax, int R, int C, int linear,
+                                                          const float* __restrict__ amax, int R, int C, int layout,
                                                           u32 seed, const u32* __restrict__ seed_dev,
                                                           float* __restrict__ gs_out) {
   if (ROUNDING != NVFP4_ROUND_NEAREST && seed_dev) seed = __ldg(seed_dev);
   const int lane = threadIdx.x & 31;
   const int nblk = C >> 4;
+  unsigned char* scales_sw = layout == NVFP4_SCALES_BOTH ? scales + (long long)R * nblk : scales;
   const int nseg = (nblk + 31) >> 5;
   __shared__ __align__(8) float lut[kLutFloats];
   const TensorScale ts = make_tensor_scale<ROUNDING>(__ldg(amax), 1.f, lut,
@@ -128,7 +145,8 @@ __global__ void __launch_bounds__(256, 4) quant_rows_kernel(const __nv_bfloat16*
       const u32 sb = block_scale_byte(absmax16(P), ts);
       const long long b = (long long)r * nblk + blk;
       codes[b] = quant_block16<ROUNDING>(P, sb, ts, seed, (u32)b, (u32)(b * 16));
-      scales[linear ? b : sw_off(r, blk, nblk >> 2)] = (unsigned char)sb;
+      if (layout != NVFP4_SCALES_SWIZZLED) scales[b] = (unsigned char)sb;
+      if (layout != NVFP4_SCALES_LINEAR) scales_sw[sw_off(r, blk, nblk >> 2)] = (unsigned char)sb;
     }
     r = rn; seg = sn; cur = nxt;
   }
@@ -143,7 +161,7 @@ template <int ROUNDING>
 __global__ void __launch_bounds__(256, 2) quant_cols_rht_kernel(const __nv_bfloat16* __restrict__ x,
                                                               unsigned char* __restrict__ codes,
                                                               unsigned char* __restrict__ scales,
-                                                              const float* __restrict__ amax, int M, int C, int linear,
+                                                              const float* __restrict__ amax, int M, int C, int layout,
                                                               u32 signs, u32 seed, const u32* __restrict__ seed_dev,
                                                               float* __restrict__ gs_out) {
   if (ROUNDING != NVFP4_ROUND_NEAREST && seed_dev) seed = __ldg(seed_dev);
@@ -151,6 +169,7 @@ __global__ void __launch_bounds__(256, 2) quant_cols_rht_kernel(const __nv_bfloa
   const int cchunk = blockIdx.x * 16 + (lane & 15);            // 8-column chunk index
   const int mb = blockIdx.y * 16 + warp * 2 + (lane >> 4);     // 16-token block index
   const int nmb = M >> 4;
+  unsigned char* scales_sw = layout == NVFP4_SCALES_BOTH ? scales + (long long)C * nmb : scales;
   __shared__ __align__(8) float lut[kLutFloats];
   // the x0.25 that follows the butterflies is folded into the tensor scale (a power of two)
   const TensorScale ts = make_tensor_scale<ROUNDING>(__ldg(amax), 4.f, lut,
@@ -186,118 +205,172 @@ __global__ void __launch_bounds__(256, 2) quant_cols_rht_kernel(const __nv_bfloa
                               o0, o1, sb0, sb1);
     *reinterpret_cast<uint2*>(codes + b0 * 8) = o0;
     *reinterpret_cast<uint2*>(codes + b1 * 8) = o1;
-    scales[linear ? b0 : sw_off(c, mb, nmb >> 2)] = (unsigned char)sb0;
-    scales[linear ? b1 : sw_off(c + 1, mb, nmb >> 2)] = (unsigned char)sb1;
+    if (layout != NVFP4_SCALES_SWIZZLED) { scales[b0] = (unsigned char)sb0; scales[b1] = (unsigned char)sb1; }
+    if (layout != NVFP4_SCALES_LINEAR) {
+      scales_sw[sw_off(c, mb, nmb >> 2)] = (unsigned char)sb0;
+      scales_sw[sw_off(c + 1, mb, nmb >> 2)] = (unsigned char)sb1;
+    }
 #pragma unroll
     for (int i = 0; i < 16; i++) { raw[i].x = raw[i].y; raw[i].y = raw[i].z; raw[i].z = raw[i].w; }
   }
 }
 
 // ------------------------------------------------------------------------------------------ 16x16 weights
-// Persistent CTAs; one warp per group of four 16x16 blocks that are neighbours along N (same K
-// block): lane = (row, 8-column half) of each block, four independent 16-byte loads in flight per
-// lane.  Block max by warp shuffles, codes for W written as one word per lane and block, codes for
-// W^T gathered with shuffles (lane = (k row, 8-row half)) and, after one exchange inside each lane
-// pair, stored as 16 contiguous bytes per lane: a k row's 32 bytes for the four blocks leave together.
-template <typename T>
-__global__ void __launch_bounds__(256) quant_w2d_kernel(const T* __restrict__ w, u32* __restrict__ q,
-                                                         unsigned char* __restrict__ s, u32* __restrict__ qt,
-                                                         unsigned char* __restrict__ st, const float* __restrict__ amax,
-                                                         int N, int K, int linear, float* __restrict__ gs_out) {
-  const int lane = threadIdx.x & 31;
+// Sixteen values of one row of W, as they travel: bf16 pairs, or FP32.
+template <typename T> struct RawRow;
+template <> struct RawRow<__nv_bfloat16> {
+  uint4 v[2];
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) {
+    v[0] = ld_cg_128(reinterpret_cast<const uint4*>(p)); v[1] = ld_cg_128(reinterpret_cast<const uint4*>(p) + 1);
+  }
+  __device__ __forceinline__ void clear() { v[0] = v[1] = make_uint4(0u, 0u, 0u, 0u); }
+  __device__ __forceinline__ void pairs(u64 (&P)[8]) const {
+    const u32 w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
+#pragma unroll
+    for (int i = 0; i < 8; i++) P[i] = f2_from_bf16x2(w[i]);
+  }
+};
+template <> struct RawRow<float> {
+  uint4 v[4];
+  __device__ __forceinline__ void load(const float* p) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = ld_cg_128(reinterpret_cast<const uint4*>(p) + i);
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  __device__ __forceinline__ void pairs(u64 (&P)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      P[2 * i] = (u64)v[i].x | ((u64)v[i].y << 32);
+      P[2 * i + 1] = (u64)v[i].z | ((u64)v[i].w << 32);
+    }
+  }
+};
+
+// Transposition of the 16 x 16 nibbles that the 16 lanes of a half-warp hold (lane i: nibble j of {lo, hi} = element
+// (i, j)): four butterfly steps, each swapping half of every lane's 64 bits with the lane at distance 8, 4, 2, 1.
+struct NibbleTranspose {
+  bool b8, b1;
+  u32 send4, lo4, hi4, send2, lo2, hi2;      // byte selectors of the two middle steps
+  __device__ __forceinline__ explicit NibbleTranspose(int lane) {
+    b8 = lane & 8; b1 = lane & 1;
+    send4 = (lane & 4) ? 0x5410u : 0x7632u; lo4 = (lane & 4) ? 0x3254u : 0x5410u; hi4 = (lane & 4) ? 0x3276u : 0x7610u;
+    send2 = (lane & 2) ? 0x6420u : 0x7531u; lo2 = (lane & 2) ? 0x3514u : 0x5240u; hi2 = (lane & 2) ? 0x3716u : 0x7260u;
+  }
+  __device__ __forceinline__ uint2 operator()(uint2 v) const {
+    u32 lo = v.x, hi = v.y;
+    u32 r = __shfl_xor_sync(0xffffffffu, b8 ? lo : hi, 8);
+    if (b8) lo = r; else hi = r;
+    r = __shfl_xor_sync(0xffffffffu, __byte_perm(lo, hi, send4), 4);
+    lo = __byte_perm(lo, r, lo4); hi = __byte_perm(hi, r, hi4);
+    r = __shfl_xor_sync(0xffffffffu, __byte_perm(lo, hi, send2), 2);
+    lo = __byte_perm(lo, r, lo2); hi = __byte_perm(hi, r, hi2);
+    constexpr u32 L = 0x0F0F0F0Fu, H = 0xF0F0F0F0u;
+    r = __shfl_xor_sync(0xffffffffu, b1 ? (lo & L) | ((hi << 4) & H) : ((lo >> 4) & L) | (hi & H), 1);
+    lo = b1 ? (lo & H) | (r & L) : (lo & L) | ((r << 4) & H);
+    hi = b1 ? (hi & H) | ((r >> 4) & L) : (hi & L) | (r & H);
+    return make_uint2(lo, hi);
+  }
+};
+
+// A half-warp owns a patch of 64 rows (N) x 32 columns (K) of W, a lane one row of each 16 x 16 block: block maximum by
+// four shuffles, eight bytes of codes per block and lane, the transposed block's row of codes by NibbleTranspose.  The
+// patch gives every lane 16 contiguous bytes of codes of W per row and 32 of W^T, and the two halves of a warp
+// neighbour along K, so that a warp reads 128 and writes 32 contiguous bytes per row.  All loads of the patch (for
+// FP32: of one row of it) are issued before the first block is quantized: that, not occupancy, is what keeps HBM busy.
+// HBM / issue bound: 7 instructions per value instead of 12 for a block spread over 32 lanes with 8 single-nibble
+// shuffles.  FULL: whole patches and 16-byte aligned outputs; otherwise 4-byte stores with bounds checks.
+template <typename T, bool FULL>
+__global__ void __launch_bounds__(256, 2) quant_w2d_kernel(const T* __restrict__ w, unsigned char* __restrict__ q,
+                                                           unsigned char* __restrict__ s, unsigned char* __restrict__ qt,
+                                                           unsigned char* __restrict__ st, const float* __restrict__ amax,
+                                                           int N, int K, int layout, float* __restrict__ gs_out) {
+  constexpr int NB = 4, KB = 2;                      // blocks of the patch along N and K
+  constexpr int AHEAD = sizeof(T) == 2 ? NB : 1;     // rows in flight per lane: 128 to 256 bytes, what the registers allow
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, i = lane & 15;
   const int nb = N >> 4, kb = K >> 4;
-  const int ngrp = (nb + 3) >> 2;
+  const int kgroups = (kb + 2 * KB - 1) / (2 * KB);
+  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int gn = (int)(item / kgroups) * NB;         // first block row, block column of this half-warp's patch
+  const int gk = (int)(item % kgroups) * (2 * KB) + (lane >> 4) * KB;
+  const bool any = gn < nb;
   __shared__ __align__(8) float lut[kLutFloats];
-  const TensorScale ts = make_tensor_scale<NVFP4_ROUND_NEAREST>(__ldg(amax), 1.f, lut,
+  pdl_wait();
+  RawRow<T> raw[AHEAD][KB];
+  auto fetch = [&](int b) {
+#pragma unroll
+    for (int c = 0; c < KB; c++) {
+      if (FULL ? any : (gn + b < nb && gk + c < kb)) raw[b % AHEAD][c].load(w + (long long)((gn + b) * 16 + i) * K + (gk + c) * 16);
+      else raw[b % AHEAD][c].clear();
+    }
+  };
+#pragma unroll
+  for (int b = 0; b < AHEAD; b++) fetch(b);
+  const TensorScale ts = make_tensor_scale<NVFP4_ROUND_NEAREST>(ld_cg_f32(amax), 1.f, lut,
                                                                (blockIdx.x == 0 && threadIdx.x == 0) ? gs_out : nullptr);
-  const u64 G = f2_pack(ts.gs, ts.gs), NRG = f2_pack(ts.nrgs, ts.nrgs);
-  const int r = lane >> 1, c0 = (lane & 1) * 8;
-  const bool wide_t = !(N & 31) && !(reinterpret_cast<uintptr_t>(qt) & 15u);   // 16-byte stores of W^T codes possible
-  const long long nitems = (long long)ngrp * kb;
-  const long long wstride = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < nitems; item += wstride) {
-    // consecutive warps walk K: the loads of a CTA are contiguous along each row
-    const int grp = (int)(item / kb), bk = (int)(item - (long long)grp * kb);
-    float v[4][8];
+  if (FULL && !any) return;
+  const NibbleTranspose transpose(lane);
+  unsigned char* s_sw = layout == NVFP4_SCALES_BOTH ? s + (long long)N * kb : s;
+  unsigned char* st_sw = layout == NVFP4_SCALES_BOTH ? st + (long long)K * nb : st;
+  uint2 wt[KB][NB];
+  u32 sb_t[KB] = {};                                 // scale bytes of the patch, four block rows packed
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int bn = grp * 4 + j;
-      if (bn < nb) {
-        const T* src = w + (long long)(bn * 16 + r) * K + bk * 16 + c0;
-        if constexpr (sizeof(T) == 2) {
-          unpack8(ldg128(src), v[j]);
-        } else {
-          const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
-          v[j][0] = a.x; v[j][1] = a.y; v[j][2] = a.z; v[j][3] = a.w; v[j][4] = b.x; v[j][5] = b.y; v[j][6] = b.z; v[j][7] = b.w;
-        }
+  for (int b = 0; b < NB; b++) {
+    uint2 wq[KB];
+    u32 sb_w = 0u;
+#pragma unroll
+    for (int c = 0; c < KB; c++) {
+      u64 P[8];
+      raw[b % AHEAD][c].pairs(P);
+      float m = absmax16(P);
+#pragma unroll
+      for (int o = 8; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      const u32 sb = block_scale_byte(m, ts);
+      wq[c] = quant_block16<NVFP4_ROUND_NEAREST>(P, sb, ts, 0u, 0u, 0u);
+      if (qt) wt[c][b] = transpose(wq[c]);
+      sb_w |= sb << (8 * c);
+      sb_t[c] |= sb << (8 * b);
+    }
+    if (b + AHEAD < NB) fetch(b + AHEAD);
+    const int row = (gn + b) * 16 + i;
+    if (q) {
+      unsigned char* dst = q + (long long)row * (K >> 1) + gk * 8;
+      if (FULL) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(wq[0].x, wq[0].y, wq[1].x, wq[1].y);
+        if (layout != NVFP4_SCALES_SWIZZLED) *reinterpret_cast<unsigned short*>(s + (long long)row * kb + gk) = (unsigned short)sb_w;
+        if (layout != NVFP4_SCALES_LINEAR) *reinterpret_cast<unsigned short*>(s_sw + sw_off(row, gk, kb >> 2)) = (unsigned short)sb_w;
       } else {
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[j][i] = 0.f;
-      }
-    }
-    u32 wt[4], sbs[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int bn = grp * 4 + j;
-      float bmax = absmax3(v[j][0], v[j][1], v[j][2]);
-      bmax = absmax3(bmax, v[j][3], v[j][4]);
-      bmax = absmax3(bmax, v[j][5], v[j][6]);
-      bmax = absmax3(bmax, v[j][7], bmax);
-#pragma unroll
-      for (int o = 16; o; o >>= 1) bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
-      const u32 sb = block_scale_byte(bmax, ts);
-      sbs[j] = sb;
-      const float2 kf = lut_entry(ts, sb);
-      const u64 NRH = f2_pack(kf.x, kf.x), NRL = f2_pack(kf.y, kf.y);
-      float y[8];
-#pragma unroll
-      for (int i = 0; i < 8; i += 2) {
-        const u64 t = f2_div_bs(f2_ndiv(f2_pack(v[j][i], v[j][i + 1]), G, NRG), NRH, NRL);
-        y[i] = f2_lo(t); y[i + 1] = f2_hi(t);
-      }
-      const u32 word = e2m1x8_rn(y);
-      if (q && bn < nb) {
-        q[((long long)(bn * 16 + r) * K + bk * 16 + c0) >> 3] = word;
-        if (!(lane & 1)) s[linear ? (long long)(bn * 16 + r) * kb + bk : sw_off(bn * 16 + r, bk, kb >> 2)] = (unsigned char)sb;
-      }
-      // transposed block: this lane builds k-row kk = lane>>1, n values (lane&1)*8 .. +7
-      const int kk = lane >> 1;
-      u32 t = 0u;
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const u32 ww = __shfl_sync(0xffffffffu, word, 2 * (c0 + i) + (kk >> 3));
-        t |= ((ww >> (4 * (kk & 7))) & 15u) << (4 * i);
-      }
-      wt[j] = t;
-    }
-    if (qt) {
-      const int kk = lane >> 1;
-      const long long krow = (long long)bk * 16 + kk;
-      if (grp * 4 + 3 < nb && wide_t) {
-        // even lane keeps blocks 0,1 (both 8-row halves), odd lane blocks 2,3: 16 contiguous bytes each
-        const bool odd = lane & 1;
-        const u32 give0 = odd ? wt[0] : wt[2], give1 = odd ? wt[1] : wt[3];
-        const u32 got0 = __shfl_xor_sync(0xffffffffu, give0, 1), got1 = __shfl_xor_sync(0xffffffffu, give1, 1);
-        const uint4 o = odd ? make_uint4(got0, wt[2], got1, wt[3]) : make_uint4(wt[0], got0, wt[1], got1);
-        *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(qt) + krow * (N >> 1) + grp * 32 + (odd ? 16 : 0)) = o;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-          if (grp * 4 + j < nb) qt[(krow * N + (grp * 4 + j) * 16 + c0) >> 3] = wt[j];
-      }
-      if (!(lane & 1)) {
-        if (grp * 4 + 3 < nb && (!linear || !(nb & 3))) {
-          // the four blocks' scale bytes are neighbours in both layouts
-          const long long o = linear ? krow * nb + grp * 4 : sw_off(krow, grp * 4, nb >> 2);
-          *reinterpret_cast<u32*>(st + o) = sbs[0] | (sbs[1] << 8) | (sbs[2] << 16) | (sbs[3] << 24);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const int bn = grp * 4 + j;
-            if (bn < nb) st[linear ? krow * nb + bn : sw_off(krow, bn, nb >> 2)] = (unsigned char)sbs[j];
+        for (int c = 0; c < KB; c++)
+          if (gn + b < nb && gk + c < kb) {
+            reinterpret_cast<u32*>(dst + 8 * c)[0] = wq[c].x; reinterpret_cast<u32*>(dst + 8 * c)[1] = wq[c].y;
+            if (layout != NVFP4_SCALES_SWIZZLED) s[(long long)row * kb + gk + c] = (unsigned char)(sb_w >> (8 * c));
+            if (layout != NVFP4_SCALES_LINEAR) s_sw[sw_off(row, gk + c, kb >> 2)] = (unsigned char)(sb_w >> (8 * c));
           }
-        }
       }
+    }
+  }
+  if (!qt) return;
+#pragma unroll
+  for (int c = 0; c < KB; c++) {
+    const int row = (gk + c) * 16 + i;               // row of W^T
+    unsigned char* dst = qt + (long long)row * (N >> 1) + gn * 8;
+    if (FULL) {
+      reinterpret_cast<uint4*>(dst)[0] = make_uint4(wt[c][0].x, wt[c][0].y, wt[c][1].x, wt[c][1].y);
+      reinterpret_cast<uint4*>(dst)[1] = make_uint4(wt[c][2].x, wt[c][2].y, wt[c][3].x, wt[c][3].y);
+      if (layout != NVFP4_SCALES_SWIZZLED) *reinterpret_cast<u32*>(st + (long long)row * nb + gn) = sb_t[c];
+      if (layout != NVFP4_SCALES_LINEAR) *reinterpret_cast<u32*>(st_sw + sw_off(row, gn, nb >> 2)) = sb_t[c];
+    } else {
+#pragma unroll
+      for (int b = 0; b < NB; b++)
+        if (gn + b < nb && gk + c < kb) {
+          reinterpret_cast<u32*>(dst + 8 * b)[0] = wt[c][b].x; reinterpret_cast<u32*>(dst + 8 * b)[1] = wt[c][b].y;
+          if (layout != NVFP4_SCALES_SWIZZLED) st[(long long)row * nb + gn + b] = (unsigned char)(sb_t[c] >> (8 * b));
+          if (layout != NVFP4_SCALES_LINEAR) st_sw[sw_off(row, gn + b, nb >> 2)] = (unsigned char)(sb_t[c] >> (8 * b));
+        }
     }
   }
 }
@@ -360,18 +433,52 @@ extern "C" int nvfp4_set_pdl(int on) {
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// The slot of `st` on the current device, or null where none can be had.  Launches of one stream never overlap (a
+// programmatically dependent one waits before it touches memory), so a stream needs one slot; it is found by the
+// stream's id, which is never given out twice.  Not inside a capture: a graph may be replayed on another stream beside
+// later work of this one.  The table is fixed memory of the library; streams beyond it take the memset.
+static AmaxSlot* amax_slot(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  int dev = 0;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cudaStreamGetId(st, &id) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  if (cap != cudaStreamCaptureStatusNone || dev < 0 || dev >= 64) return nullptr;
+  static std::mutex lock;
+  static AmaxSlot* base[64];
+  static std::unordered_map<unsigned long long, int> index[64];
+  std::lock_guard<std::mutex> hold(lock);
+  if (!base[dev]) {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_amax_slots) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
+    base[dev] = static_cast<AmaxSlot*>(p);
+  }
+  const auto it = index[dev].find(id);
+  if (it != index[dev].end()) return base[dev] + it->second;
+  const int n = (int)index[dev].size();
+  if (n >= kAmaxSlots) return nullptr;
+  index[dev].emplace(id, n);
+  return base[dev] + n;
+}
+
+// `n` values, 16 / sizeof of them per load
+template <bool F32>
 static int amax_launch(const void* x, long long n, float* out, bool clear, void* stream) {
+  constexpr int kPer = F32 ? 4 : 8;
   if (!out || (!x && n > 0)) return NVFP4_ERR_NULL;
-  if (n < 0 || (n & 7)) return NVFP4_ERR_SHAPE;
+  if (n < 0 || n % kPer) return NVFP4_ERR_SHAPE;
   if (!aligned16(x)) return NVFP4_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (clear && cudaMemsetAsync(out, 0, sizeof(float), st) != cudaSuccess) return NVFP4_ERR_CUDA;
+  AmaxSlot* slot = clear && n > 0 ? amax_slot(st) : nullptr;
+  if (clear && !slot && cudaMemsetAsync(out, 0, sizeof(float), st) != cudaSuccess) return NVFP4_ERR_CUDA;
   if (n == 0) return NVFP4_OK;
-  const long long n8 = n >> 3;
-  long long blocks = (n8 + 256 * 4 - 1) / (256 * 4);
+  const long long nv = n / kPer;
+  long long blocks = (nv + 256 * 4 - 1) / (256 * 4);
   const long long cap = (long long)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  if (nvfp4_launch_kernel(amax_bf16_kernel, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const uint4*>(x), n8, out) != cudaSuccess) {
+  if (nvfp4_launch_kernel(amax_kernel<F32>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const uint4*>(x), nv, out, slot) != cudaSuccess) {
     (void)cudaGetLastError();
     return NVFP4_ERR_CUDA;
   }
@@ -379,21 +486,25 @@ static int amax_launch(const void* x, long long n, float* out, bool clear, void*
 }
 
 extern "C" int nvfp4_amax_bf16(const void* x, long long n, float* out, void* stream) {
-  return amax_launch(x, n, out, true, stream);
+  return amax_launch<false>(x, n, out, true, stream);
 }
 
 extern "C" int nvfp4_amax_bf16_update(const void* x, long long n, float* out, void* stream) {
-  return amax_launch(x, n, out, false, stream);
+  return amax_launch<false>(x, n, out, false, stream);
+}
+
+extern "C" int nvfp4_amax_f32(const float* x, long long n, float* out, void* stream) {
+  return amax_launch<true>(x, n, out, true, stream);
 }
 
 extern "C" int nvfp4_quant_rows(const void* x, long long ldx, int R, int C, void* codes, void* scales,
                                 int scale_layout, const float* amax, float* gs_out, int rounding, unsigned seed,
                                 const unsigned* seed_dev, void* stream) {
   if (!x || !codes || !scales || !amax) return NVFP4_ERR_NULL;
-  if (scale_layout != NVFP4_SCALES_SWIZZLED && scale_layout != NVFP4_SCALES_LINEAR) return NVFP4_ERR_ENUM;
+  if (scale_layout < NVFP4_SCALES_SWIZZLED || scale_layout > NVFP4_SCALES_BOTH) return NVFP4_ERR_ENUM;
   if (rounding < NVFP4_ROUND_NEAREST || rounding > NVFP4_ROUND_SR_HW) return NVFP4_ERR_ENUM;
   if (R < 0 || C < 0 || (C & 15) || ldx < C) return NVFP4_ERR_SHAPE;
-  if (scale_layout == NVFP4_SCALES_SWIZZLED && ((R & 127) || (C & 63))) return NVFP4_ERR_SHAPE;
+  if (scale_layout != NVFP4_SCALES_LINEAR && ((R & 127) || (C & 63))) return NVFP4_ERR_SHAPE;
   if (!aligned16(x) || (ldx & 7) || (reinterpret_cast<uintptr_t>(codes) & 7u)) return NVFP4_ERR_ALIGN;
   if (R == 0 || C == 0) return NVFP4_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -401,7 +512,6 @@ extern "C" int nvfp4_quant_rows(const void* x, long long ldx, int R, int C, void
   long long blocks = (nitems + 7) / 8;
   const long long cap = (long long)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  const int linear = scale_layout == NVFP4_SCALES_LINEAR;
   const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
   uint2* cp = static_cast<uint2*>(codes);
   unsigned char* sp = static_cast<unsigned char*>(scales);
@@ -409,8 +519,8 @@ extern "C" int nvfp4_quant_rows(const void* x, long long ldx, int R, int C, void
   const bool wide = (reinterpret_cast<uintptr_t>(x) & 31u) == 0 && (ldx & 15) == 0;
 #define NVFP4_ROWS(RND)                                                                                              \
   do {                                                                                                               \
-    if (wide) quant_rows_kernel<RND, true><<<(unsigned)blocks, 256, 0, st>>>(xp, ldx, cp, sp, amax, R, C, linear, seed, seed_dev, gs_out); \
-    else quant_rows_kernel<RND, false><<<(unsigned)blocks, 256, 0, st>>>(xp, ldx, cp, sp, amax, R, C, linear, seed, seed_dev, gs_out);     \
+    if (wide) quant_rows_kernel<RND, true><<<(unsigned)blocks, 256, 0, st>>>(xp, ldx, cp, sp, amax, R, C, scale_layout, seed, seed_dev, gs_out); \
+    else quant_rows_kernel<RND, false><<<(unsigned)blocks, 256, 0, st>>>(xp, ldx, cp, sp, amax, R, C, scale_layout, seed, seed_dev, gs_out);     \
   } while (0)
   switch (rounding) {
     case NVFP4_ROUND_NEAREST: NVFP4_ROWS(NVFP4_ROUND_NEAREST); break;
@@ -427,29 +537,28 @@ extern "C" int nvfp4_quant_cols_rht(const void* x, int M, int C, void* codes, vo
                                     const float* amax, float* gs_out, unsigned signs, int rounding, unsigned seed,
                                     const unsigned* seed_dev, void* stream) {
   if (!x || !codes || !scales || !amax) return NVFP4_ERR_NULL;
-  if (scale_layout != NVFP4_SCALES_SWIZZLED && scale_layout != NVFP4_SCALES_LINEAR) return NVFP4_ERR_ENUM;
+  if (scale_layout < NVFP4_SCALES_SWIZZLED || scale_layout > NVFP4_SCALES_BOTH) return NVFP4_ERR_ENUM;
   if (rounding < NVFP4_ROUND_NEAREST || rounding > NVFP4_ROUND_SR_HW) return NVFP4_ERR_ENUM;
   if (M < 0 || C < 0 || (M & 15) || (C & 7)) return NVFP4_ERR_SHAPE;
-  if (scale_layout == NVFP4_SCALES_SWIZZLED && ((C & 127) || (M & 63))) return NVFP4_ERR_SHAPE;
+  if (scale_layout != NVFP4_SCALES_LINEAR && ((C & 127) || (M & 63))) return NVFP4_ERR_SHAPE;
   if (!aligned16(x) || (reinterpret_cast<uintptr_t>(codes) & 7u)) return NVFP4_ERR_ALIGN;
   if (M == 0 || C == 0) return NVFP4_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   dim3 grid((unsigned)((C + 127) / 128), (unsigned)((M + 255) / 256));
   if (grid.y > 65535u) return NVFP4_ERR_TOO_LARGE;
-  const int linear = scale_layout == NVFP4_SCALES_LINEAR;
   const __nv_bfloat16* xp = static_cast<const __nv_bfloat16*>(x);
   unsigned char* cp = static_cast<unsigned char*>(codes);
   unsigned char* sp = static_cast<unsigned char*>(scales);
   signs &= 0xFFFFu;
   switch (rounding) {
     case NVFP4_ROUND_NEAREST:
-      quant_cols_rht_kernel<NVFP4_ROUND_NEAREST><<<grid, 256, 0, st>>>(xp, cp, sp, amax, M, C, linear, signs, seed, seed_dev, gs_out); break;
+      quant_cols_rht_kernel<NVFP4_ROUND_NEAREST><<<grid, 256, 0, st>>>(xp, cp, sp, amax, M, C, scale_layout, signs, seed, seed_dev, gs_out); break;
     case NVFP4_ROUND_SR_DITHER:
-      quant_cols_rht_kernel<NVFP4_ROUND_SR_DITHER><<<grid, 256, 0, st>>>(xp, cp, sp, amax, M, C, linear, signs, seed, seed_dev, gs_out); break;
+      quant_cols_rht_kernel<NVFP4_ROUND_SR_DITHER><<<grid, 256, 0, st>>>(xp, cp, sp, amax, M, C, scale_layout, signs, seed, seed_dev, gs_out); break;
     case NVFP4_ROUND_SR_DITHER_K:
-      quant_cols_rht_kernel<NVFP4_ROUND_SR_DITHER_K><<<grid, 256, 0, st>>>(xp, cp, sp, amax, M, C, linear, signs, seed, seed_dev, gs_out); break;
+      quant_cols_rht_kernel<NVFP4_ROUND_SR_DITHER_K><<<grid, 256, 0, st>>>(xp, cp, sp, amax, M, C, scale_layout, signs, seed, seed_dev, gs_out); break;
     default:
-      quant_cols_rht_kernel<NVFP4_ROUND_SR_HW><<<grid, 256, 0, st>>>(xp, cp, sp, amax, M, C, linear, signs, seed, seed_dev, gs_out); break;
+      quant_cols_rht_kernel<NVFP4_ROUND_SR_HW><<<grid, 256, 0, st>>>(xp, cp, sp, amax, M, C, scale_layout, signs, seed, seed_dev, gs_out); break;
   }
   NVFP4_LAUNCH_CHECK();
   return NVFP4_OK;
@@ -458,26 +567,28 @@ extern "C" int nvfp4_quant_cols_rht(const void* x, int M, int C, void* codes, vo
 extern "C" int nvfp4_quant_w2d(const void* w, int w_dtype, int N, int K, void* q, void* s, void* qt, void* st_,
                                int scale_layout, const float* amax, float* gs_out, void* stream) {
   if (!w || !amax || (!q && !qt) || (q && !s) || (qt && !st_)) return NVFP4_ERR_NULL;
-  if (scale_layout != NVFP4_SCALES_SWIZZLED && scale_layout != NVFP4_SCALES_LINEAR) return NVFP4_ERR_ENUM;
+  if (scale_layout < NVFP4_SCALES_SWIZZLED || scale_layout > NVFP4_SCALES_BOTH) return NVFP4_ERR_ENUM;
   if (w_dtype != NVFP4_DTYPE_BF16 && w_dtype != NVFP4_DTYPE_FP32) return NVFP4_ERR_ENUM;
   if (N < 0 || K < 0 || (N & 15) || (K & 15)) return NVFP4_ERR_SHAPE;
-  if (scale_layout == NVFP4_SCALES_SWIZZLED && ((N & 127) || (K & 127))) return NVFP4_ERR_SHAPE;
+  if (scale_layout != NVFP4_SCALES_LINEAR && ((N & 127) || (K & 127))) return NVFP4_ERR_SHAPE;
   if (!aligned16(w) || (q && (reinterpret_cast<uintptr_t>(q) & 3u)) || (qt && ((reinterpret_cast<uintptr_t>(qt) | reinterpret_cast<uintptr_t>(st_)) & 3u)))
     return NVFP4_ERR_ALIGN;
   if (N == 0 || K == 0) return NVFP4_OK;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long long nwarps = (long long)(((N >> 4) + 3) >> 2) * (K >> 4);
-  long long blocks = (nwarps + 7) / 8;
-  const long long cap = (long long)sm_count() * 8;
-  if (blocks > cap) blocks = cap;
-  const int linear = scale_layout == NVFP4_SCALES_LINEAR;
-  if (w_dtype == NVFP4_DTYPE_BF16)
-    quant_w2d_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(w), static_cast<u32*>(q),
-        static_cast<unsigned char*>(s), static_cast<u32*>(qt), static_cast<unsigned char*>(st_), amax, N, K, linear, gs_out);
-  else
-    quant_w2d_kernel<float><<<(unsigned)blocks, 256, 0, st>>>(static_cast<const float*>(w), static_cast<u32*>(q),
-        static_cast<unsigned char*>(s), static_cast<u32*>(qt), static_cast<unsigned char*>(st_), amax, N, K, linear, gs_out);
-  NVFP4_LAUNCH_CHECK();
+  cudaStream_t stm = static_cast<cudaStream_t>(stream);
+  const bool full = !(N & 63) && !(K & 63) && aligned16(q) && aligned16(qt) && !(reinterpret_cast<uintptr_t>(s) & 1u);
+  const long long warps = (long long)(((N >> 4) + 3) / 4) * (((K >> 4) + 3) / 4);
+  const dim3 grid((unsigned)((warps + 7) / 8));
+  unsigned char *qp = static_cast<unsigned char*>(q), *sp = static_cast<unsigned char*>(s);
+  unsigned char *qtp = static_cast<unsigned char*>(qt), *stp = static_cast<unsigned char*>(st_);
+  cudaError_t rc;
+#define NVFP4_W2D(T, FULL) nvfp4_launch_kernel(quant_w2d_kernel<T, FULL>, grid, dim3(256), 0, stm, static_cast<const T*>(w), qp, sp, qtp, stp, amax, N, K, scale_layout, gs_out)
+  if (w_dtype == NVFP4_DTYPE_BF16) rc = full ? NVFP4_W2D(__nv_bfloat16, true) : NVFP4_W2D(__nv_bfloat16, false);
+  else rc = full ? NVFP4_W2D(float, true) : NVFP4_W2D(float, false);
+#undef NVFP4_W2D
+  if (rc != cudaSuccess) {
+    (void)cudaGetLastError();
+    return NVFP4_ERR_CUDA;
+  }
   return NVFP4_OK;
 }
 

@@ -56,7 +56,7 @@ struct TcParams {
   unsigned char* codes_c; unsigned char* scales_c;    // transposed operand [C, M/2], scales [C, M/16]
   const float* amax;
   float* gs_r_out; float* gs_c_out;
-  int M, C, linear;
+  int M, C, layout;                                   // NVFP4_SCALES_*; BOTH: the swizzled bytes follow the row-major ones
   u32 signs;
   u32 seed_r, seed_c;
   const u32* seed_r_dev; const u32* seed_c_dev;
@@ -333,8 +333,9 @@ __global__ void __launch_bounds__(kQThreads, 2) quant_tc_kernel(const __grid_con
     // per-thread output positions of tile (0, 0); a tile adds a multiple of its coordinates
     const long long tok0 = quad * 32 + lane, col0 = quad * 32 + lane;
     const long long row_code_stride = (long long)kQTok * (p.C >> 1), col_code_stride = (long long)kQCol * nmb * 8;
-    const long long row_sc0 = p.linear ? tok0 * nblk + half * 4 : (long long)half * 512 + lane * 16 + quad * 4;
-    const long long col_sc0 = p.linear ? col0 * nmb + half * 4 : (long long)half * 512 + lane * 16 + quad * 4;
+    const bool linear = p.layout != NVFP4_SCALES_SWIZZLED, swizzled = p.layout != NVFP4_SCALES_LINEAR;
+    const long long row_sc0 = tok0 * nblk + half * 4, col_sc0 = col0 * nmb + half * 4;
+    const long long sw_sc0 = (p.layout == NVFP4_SCALES_BOTH ? (long long)p.M * nblk : 0) + (long long)half * 512 + lane * 16 + quad * 4;
 
     bool alive = true;
     // wait for buffer `buf` to be full; false (for the whole warp) when the CTA is aborting
@@ -405,17 +406,15 @@ __global__ void __launch_bounds__(kQThreads, 2) quant_tc_kernel(const __grid_con
         *reinterpret_cast<uint4*>(dst) = make_uint4(orow[0].x, orow[0].y, orow[1].x, orow[1].y);
         *reinterpret_cast<uint4*>(dst + 16) = make_uint4(orow[2].x, orow[2].y, orow[3].x, orow[3].y);
         // the four scale bytes are neighbours in both layouts
-        const long long so = p.linear ? (long long)mt * kQTok * nblk + ct * (kQCol / 16) + row_sc0
-                                      : ((long long)mt * (nblk >> 2) + ct * 2) * 512 + row_sc0;
-        *reinterpret_cast<u32*>(p.scales_r + so) = sb_row;
+        if (linear) *reinterpret_cast<u32*>(p.scales_r + (long long)mt * kQTok * nblk + ct * (kQCol / 16) + row_sc0) = sb_row;
+        if (swizzled) *reinterpret_cast<u32*>(p.scales_r + ((long long)mt * (nblk >> 2) + ct * 2) * 512 + sw_sc0) = sb_row;
       };
       auto store_cols = [&]() {
         unsigned char* dst = p.codes_c + (long long)ct * col_code_stride + (col0 * nmb + mb0) * 8;
         *reinterpret_cast<uint4*>(dst) = make_uint4(ocol[0].x, ocol[0].y, ocol[1].x, ocol[1].y);
         *reinterpret_cast<uint4*>(dst + 16) = make_uint4(ocol[2].x, ocol[2].y, ocol[3].x, ocol[3].y);
-        const long long so = p.linear ? (long long)ct * kQCol * nmb + mt * (kQTok / 16) + col_sc0
-                                      : ((long long)ct * (nmb >> 2) + mt * 2) * 512 + col_sc0;
-        *reinterpret_cast<u32*>(p.scales_c + so) = sb_col;
+        if (linear) *reinterpret_cast<u32*>(p.scales_c + (long long)ct * kQCol * nmb + mt * (kQTok / 16) + col_sc0) = sb_col;
+        if (swizzled) *reinterpret_cast<u32*>(p.scales_c + ((long long)ct * (nmb >> 2) + mt * 2) * 512 + sw_sc0) = sb_col;
       };
 
       if (ROWS) {
@@ -539,7 +538,7 @@ int nvfp4_quant_tc_launch(const void* x, long long ldx, int M, int C, void* code
   p.codes_r = static_cast<unsigned char*>(codes_r); p.scales_r = static_cast<unsigned char*>(scales_r);
   p.codes_c = static_cast<unsigned char*>(codes_c); p.scales_c = static_cast<unsigned char*>(scales_c);
   p.amax = amax; p.gs_r_out = gs_r_out; p.gs_c_out = gs_c_out;
-  p.M = M; p.C = C; p.linear = scale_layout == NVFP4_SCALES_LINEAR;
+  p.M = M; p.C = C; p.layout = scale_layout;
   p.signs = signs & 0xFFFFu;
   p.seed_r = seed_r; p.seed_c = seed_c; p.seed_r_dev = seed_r_dev; p.seed_c_dev = seed_c_dev;
   p.tc_rht = g_tc_rht;

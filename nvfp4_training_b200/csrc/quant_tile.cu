@@ -336,7 +336,7 @@ extern "C" int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void
                                 unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
                                 const unsigned* seed_r_dev, const unsigned* seed_c_dev, void* stream) {
   if (!x || !amax || (!codes_r && !codes_c) || (codes_r && !scales_r) || (codes_c && !scales_c)) return NVFP4_ERR_NULL;
-  if (scale_layout != NVFP4_SCALES_SWIZZLED && scale_layout != NVFP4_SCALES_LINEAR) return NVFP4_ERR_ENUM;
+  if (scale_layout < NVFP4_SCALES_SWIZZLED || scale_layout > NVFP4_SCALES_BOTH) return NVFP4_ERR_ENUM;
   if (rounding < NVFP4_ROUND_NEAREST || rounding > NVFP4_ROUND_SR_HW) return NVFP4_ERR_ENUM;
   if (M < 0 || C < 0 || (M % kTileTok) || (C % kTileCol) || ldx < C) return NVFP4_ERR_SHAPE;
   if (codes_c && scale_layout == NVFP4_SCALES_SWIZZLED && (C & 127)) return NVFP4_ERR_SHAPE;
@@ -347,6 +347,7 @@ extern "C" int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void
   if (g_tile_path != 1 && nvfp4_quant_tc_accepts(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c))
     return nvfp4_quant_tc_launch(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c, scale_layout, amax, gs_r_out, gs_c_out,
                                  signs, rounding, seed_r, seed_c, seed_r_dev, seed_c_dev, stream);
+  if (scale_layout == NVFP4_SCALES_BOTH) return NVFP4_ERR_SHAPE;       // the scalar kernel writes one layout
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap map;
   if (!make_tile_map(&map, x, M, C, ldx)) return NVFP4_ERR_CUDA;
