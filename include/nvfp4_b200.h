@@ -82,6 +82,15 @@ int nvfp4_amax_bf16(const void* x, long long n, float* out, void* stream);
 int nvfp4_amax_bf16_update(const void* x, long long n, float* out, void* stream);
 
 /*
+ * nvfp4_amax_bf16 for a caller that launches the consumers of the result next: *word (a host variable) receives the
+ * device address of a word of this library that holds max|x| for kernels launched by this host thread on this stream
+ * before its seventh later call.  Nothing has to be cleared, so the call is one kernel.  Where the library has no such
+ * word (inside a stream capture, or beyond 1024 pairs of thread and stream) *word is `fallback`, a device word of the
+ * caller, and the call is nvfp4_amax_bf16 (null: nothing is launched).  n > 0.  No reference counterpart.
+ */
+int nvfp4_amax_bf16_word(const void* x, long long n, float* fallback, const float** word, void* stream);
+
+/*
  * max|x| of a contiguous FP32 tensor into *out, for FP32 master weights (`x.abs().amax()` of llm-1b/fp4ops.py:25-26).  A
  * NaN anywhere gives NaN.  Requires n % 4 == 0, x 16-byte aligned.  n == 0 gives 0.
  */
@@ -160,7 +169,7 @@ int nvfp4_quant_tile_set_path(int path);
 /* Reads (synchronously) the status word of nvfp4_quant_tile launches on the current device:
  * 0, or the role whose wait expired first (scalar kernel: 1 producer, 2 consumer; tensor-core-fed kernel:
  * 17 / 19 the loading and MMA-issuing warp waiting for a tile / for a free stage, 18 a consumer; row emitter's ring
- * kernel: 33 producer, 34 consumer); `reset` != 0 clears it. */
+ * kernel: 33 producer, 34 consumer; weight quantizer: 48); `reset` != 0 clears it. */
 int nvfp4_quant_tile_status(int* out, int reset);
 
 /*

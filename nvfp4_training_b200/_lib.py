@@ -27,6 +27,7 @@ SIGNATURES = {
     "nvfp4_error_string": (_c.c_char_p, [_i]),
     "nvfp4_amax_bf16": (_i, [_vp, _ll, _vp, _vp]),
     "nvfp4_amax_bf16_update": (_i, [_vp, _ll, _vp, _vp]),
+    "nvfp4_amax_bf16_word": (_i, [_vp, _ll, _vp, _vp, _vp]),
     "nvfp4_amax_f32": (_i, [_vp, _ll, _vp, _vp]),
     "nvfp4_set_pdl": (_i, [_i]),
     "nvfp4_gemm_reset_scheduler": (_i, []),

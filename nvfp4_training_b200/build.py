@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libnvfp4_b200.so")
 HOST = os.path.join(HERE, "_host.so")
-SOURCES = ["quant.cu", "quant_tile.cu", "quant_mma.cu", "emit_ops.cu", "emit_rows_ring.cu", "emit_fused.cu", "gemm.cu", "noalloc.cu", "selftest.cu"]
+SOURCES = ["quant.cu", "quant_tile.cu", "quant_mma.cu", "quant_w2d.cu", "emit_ops.cu", "emit_rows_ring.cu", "emit_fused.cu", "gemm.cu", "noalloc.cu", "selftest.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

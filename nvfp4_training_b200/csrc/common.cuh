@@ -383,4 +383,30 @@ __device__ __forceinline__ void quant_block16x2(const u64 (&P)[16], const Tensor
   o1 = make_uint2(w1[0], w1[1]);
 }
 
+// Transposition of the 16 x 16 nibbles that the 16 lanes of a half-warp hold (lane i: nibble j of {lo, hi} = element
+// (i, j)): four butterfly steps, each swapping half of every lane's 64 bits with the lane at distance 8, 4, 2, 1.
+struct NibbleTranspose {
+  bool b8, b1;
+  u32 send4, lo4, hi4, send2, lo2, hi2;      // byte selectors of the two middle steps
+  __device__ __forceinline__ explicit NibbleTranspose(int lane) {
+    b8 = lane & 8; b1 = lane & 1;
+    send4 = (lane & 4) ? 0x5410u : 0x7632u; lo4 = (lane & 4) ? 0x3254u : 0x5410u; hi4 = (lane & 4) ? 0x3276u : 0x7610u;
+    send2 = (lane & 2) ? 0x6420u : 0x7531u; lo2 = (lane & 2) ? 0x3514u : 0x5240u; hi2 = (lane & 2) ? 0x3716u : 0x7260u;
+  }
+  __device__ __forceinline__ uint2 operator()(uint2 v) const {
+    u32 lo = v.x, hi = v.y;
+    u32 r = __shfl_xor_sync(0xffffffffu, b8 ? lo : hi, 8);
+    if (b8) lo = r; else hi = r;
+    r = __shfl_xor_sync(0xffffffffu, __byte_perm(lo, hi, send4), 4);
+    lo = __byte_perm(lo, r, lo4); hi = __byte_perm(hi, r, hi4);
+    r = __shfl_xor_sync(0xffffffffu, __byte_perm(lo, hi, send2), 2);
+    lo = __byte_perm(lo, r, lo2); hi = __byte_perm(hi, r, hi2);
+    constexpr u32 L = 0x0F0F0F0Fu, H = 0xF0F0F0F0u;
+    r = __shfl_xor_sync(0xffffffffu, b1 ? (lo & L) | ((hi << 4) & H) : ((lo >> 4) & L) | (hi & H), 1);
+    lo = b1 ? (lo & H) | (r & L) : (lo & L) | ((r << 4) & H);
+    hi = b1 ? (hi & H) | ((r >> 4) & L) : (hi & L) | (r & H);
+    return make_uint2(lo, hi);
+  }
+};
+
 }  // namespace nvfp4

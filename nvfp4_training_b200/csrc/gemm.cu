@@ -663,7 +663,7 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const u32 rank = cluster_ctarank();                 // 0 = leader (issues the MMAs), 1 = peer
-  const int tiles_m = p.M / 256, tiles_n = (p.N + BN - 1) / BN;
+  const int tiles_m = (p.M + 255) / 256, tiles_n = (p.N + BN - 1) / BN;     // edge tiles read zeros beyond M and N and store what is inside
   const int ktiles = (p.K + kBK - 1) / kBK;
   const int num_work = tiles_m * tiles_n * p.splitk;
   const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
@@ -916,6 +916,7 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 #undef NVFP4_RELEASE_ACC
 
       const long long row0 = (long long)mt * 256 + rank * 128 + quad * 32;      // first row of this warp
+      if (row0 >= p.M) continue;          // the peer's half of an edge tile (M is a multiple of 128)
       float alpha = 1.f;
       if (p.alpha_mode == NVFP4_ALPHA_GS) alpha = ld_cg_f32(p.pa) * ld_cg_f32(p.pb);
       else if (p.alpha_mode == NVFP4_ALPHA_AMAX) alpha = ld_cg_f32(p.pa) * ld_cg_f32(p.pb) * p.kscale;
@@ -1052,7 +1053,7 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   if (g_sm_budget > 0 && g_sm_budget < sms) sms = g_sm_budget >= 2 ? (g_sm_budget & ~1) : 2;
 
   const int ktiles = (K + kBK - 1) / kBK;
-  if (auto_split && c_dtype == NVFP4_DTYPE_FP32 && (M % 256 == 0) && g_force_bn == 0 && ktiles >= 16) {
+  if (auto_split && c_dtype == NVFP4_DTYPE_FP32 && g_force_bn == 0 && ktiles >= 16) {
     // Weight-gradient shapes have few output tiles and a long contraction: 96 or 176 tiles over 74 SM pairs leave
     // a third of the machine idle in the last round.  Slicing K evens that out; the price is the per-tile fixed
     // cost once more per slice, FP32 atomic adds instead of stores, and a zero fill when the call overwrites C.
@@ -1062,8 +1063,8 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
     for (int s = 1; s <= 8 && s <= ktiles; s++) {
       const int per_s = (ktiles + s - 1) / s;
       if ((ktiles + per_s - 1) / per_s != s) continue;
-      const long long t256 = (N % 256 == 0) ? (long long)(M / 256) * (N / 256) * s : 0;
-      const long long t192 = (long long)(M / 256) * ((N + 191) / 192) * s;
+      const long long t256 = (N % 256 == 0) ? (long long)((M + 255) / 256) * (N / 256) * s : 0;
+      const long long t192 = (long long)((M + 255) / 256) * ((N + 191) / 192) * s;
       double cost = (double)((t192 + ncl - 1) / ncl) * (1.88 + 0.3255 * per_s);
       if (t256) cost = fmin(cost, (double)((t256 + ncl - 1) / ncl) * (2.98 + 0.346 * per_s));
       if (s > 1) {
@@ -1089,8 +1090,8 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   const int bn = wide ? 256 : 128;
 
   // CTA-pair kernels (an SM pair per 256-row tile): the fast path whenever M allows it
-  bool use_pair = (M % 256 == 0) && g_force_bn != 128 && g_force_bn != 256;
-  if (g_force_bn == 0 && (long long)(M / 256) * ((N + 255) / 256) * splitk < sms / 4) use_pair = false;   // too few tiles: finer tiles fill more SMs
+  bool use_pair = g_force_bn != 128 && g_force_bn != 256;
+  if (g_force_bn == 0 && (long long)((M + 255) / 256) * ((N + 255) / 256) * splitk < sms / 4) use_pair = false;   // too few tiles: finer tiles fill more SMs
   if (owners) use_pair = true;                    // the scatter lives in the pair kernel's epilogue only
   if (use_pair) {
     // tile width: 256 moves the fewest operand bytes per FLOP but consecutive tiles wait for each other's
@@ -1101,8 +1102,8 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
       // 1.88 + 0.3255 (0.78 of the 256-wide tile at K = 2048, 0.89 at K = 11264); what decides is mostly how
       // evenly the tile count divides over the SM pairs
       const long long ncl = sms / 2;
-      const long long r256 = ((long long)(M / 256) * (N / 256) * splitk + ncl - 1) / ncl;
-      const long long r192 = ((long long)(M / 256) * ((N + 191) / 192) * splitk + ncl - 1) / ncl;
+      const long long r256 = ((long long)((M + 255) / 256) * (N / 256) * splitk + ncl - 1) / ncl;
+      const long long r192 = ((long long)((M + 255) / 256) * ((N + 191) / 192) * splitk + ncl - 1) / ncl;
       if (r256 * (2.98 + 0.346 * per) <= r192 * (1.88 + 0.3255 * per)) pbn = 256;
     }
     if (g_pair_bn == 128 || g_pair_bn == 192 || (g_pair_bn == 256 && N % 256 == 0)) pbn = g_pair_bn;   // forced (tuning and tests)
@@ -1126,8 +1127,8 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
     static std::atomic<unsigned> launch_seq{0};
     pp.counter = di->counters + (launch_seq.fetch_add(1u, std::memory_order_relaxed) & 4095u);
     // (items shorter than four K tiles stay dealt out in advance: one draw takes about as long as such an item)
-    pp.dynamic = (g_dynamic_sched && per >= 4 && splitk <= 255 && (M / 256) < (int)kSchedEnd && (N + pbn - 1) / pbn <= (int)kSchedEnd) ? g_dynamic_sched : 0;
-    const long long work = (long long)(M / 256) * ((N + pbn - 1) / pbn) * splitk;
+    pp.dynamic = (g_dynamic_sched && per >= 4 && splitk <= 255 && ((M + 255) / 256) < (int)kSchedEnd && (N + pbn - 1) / pbn <= (int)kSchedEnd) ? g_dynamic_sched : 0;
+    const long long work = (long long)((M + 255) / 256) * ((N + pbn - 1) / pbn) * splitk;
     const long long clusters = work < sms / 2 ? work : sms / 2;
     const unsigned grid = (unsigned)(2 * clusters);
 #define NVFP4_LAUNCH_PAIR(BN_, FLAG)                                                                                      \

@@ -36,7 +36,7 @@ namespace {
 // ------------------------------------------------------------------------------------------ library entry points
 #define NVFP4_API(X)                                                                                                        \
   X(nvfp4_amax_bf16) X(nvfp4_amax_bf16_update) X(nvfp4_quant_rows) X(nvfp4_quant_cols_rht) X(nvfp4_quant_tile)             \
-  X(nvfp4_quant_w2d) X(nvfp4_gemm) X(nvfp4_error_string) X(nvfp4_amax_f32) X(nvfp4_swizzle_scales) X(nvfp4_emit_rows)        \
+  X(nvfp4_quant_w2d) X(nvfp4_gemm) X(nvfp4_error_string) X(nvfp4_amax_f32) X(nvfp4_amax_bf16_word) X(nvfp4_swizzle_scales) X(nvfp4_emit_rows)        \
   X(nvfp4_emit_cols) X(nvfp4_rms_emit) X(nvfp4_swiglu_emit) X(nvfp4_mom_acc)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
@@ -144,6 +144,14 @@ void run_amax(const Tensor& x, float* out, bool clear = true) {
   check((clear ? lib.nvfp4_amax_bf16 : lib.nvfp4_amax_bf16_update)(x.const_data_ptr(), x.numel(), out, stream()), "amax");
 }
 
+// amax for consumers that this thread launches next: a word of the library, or `fallback` (null: nothing is launched)
+// where it has none
+const float* passing_amax(const Tensor& x, float* fallback) {
+  const float* word = nullptr;
+  check(lib.nvfp4_amax_bf16_word(x.const_data_ptr(), x.numel(), fallback, &word, stream()), "amax");
+  return word;
+}
+
 void run_tile(const Tensor& x, const PackedOut* row, const PackedOut* col, const float* am, unsigned signs, int mode,
               const Seed& seed, const Seed& seed_cols) {
   check(lib.nvfp4_quant_tile(x.const_data_ptr(), x.stride(0), (int)x.size(0), (int)x.size(1), row ? row->d : nullptr,
@@ -176,13 +184,20 @@ Tensor nvq_amax(const Tensor& x, const OptTensor& out_, bool clear) {
   return out;
 }
 
-// amax word of `x`: the caller's, or computed now into a new one
-Tensor amax_or(const OptTensor& am, const Tensor& x) {
-  if (am) return *am;
-  at::NoGradGuard no_grad;
-  return nvq_amax(x.contiguous(), std::nullopt, true);
-}
 const float* word(const Tensor& am) { return static_cast<const float*>(am.const_data_ptr()); }
+// amax word of `x` for the launches that follow: the caller's, or computed now.  `keep` holds the word where the
+// library has none to offer.
+const float* amax_or(const OptTensor& am, const Tensor& x, Tensor& keep) {
+  if (am) return word(*am);
+  REQUIRE(x.numel() % 8 == 0, "amax: a multiple of 8 values");
+  at::NoGradGuard no_grad;
+  const Tensor xc = x.contiguous();
+  const float* w = xc.numel() ? passing_amax(xc, nullptr) : nullptr;
+  if (w) return w;
+  keep = empty({1}, at::kFloat, x);
+  run_amax(xc, keep.data_ptr<float>());
+  return word(keep);
+}
 
 py::tuple nvq_quant_rows(const Tensor& x, int mode, py::handle seed_, const OptTensor& am_) {
   require_cuda(x);
@@ -190,10 +205,11 @@ py::tuple nvq_quant_rows(const Tensor& x, int mode, py::handle seed_, const OptT
   const int64_t R = x.size(0), C = x.size(1);
   REQUIRE(x.stride(1) == 1 && C % 64 == 0 && R % 128 == 0, shape_of(R, C));
   const Seed seed(seed_);
-  const Tensor am = amax_or(am_, x);
   PackedTensors q(R, C, x);
   const PackedOut o = q.out();
-  check(lib.nvfp4_quant_rows(x.const_data_ptr(), x.stride(0), (int)R, (int)C, o.d, o.s, NVFP4_SCALES_SWIZZLED, word(am), o.gs,
+  Tensor keep;
+  const float* am = amax_or(am_, x, keep);
+  check(lib.nvfp4_quant_rows(x.const_data_ptr(), x.stride(0), (int)R, (int)C, o.d, o.s, NVFP4_SCALES_SWIZZLED, am, o.gs,
                              mode, seed.host, seed.dev, stream()), "quant_rows");
   return q.tuple();
 }
@@ -206,12 +222,13 @@ py::tuple nvq_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, py::han
   const int64_t M = x.size(0), C = x.size(1);
   REQUIRE(M % 64 == 0 && C % 128 == 0, shape_of(M, C));
   const Seed seed(seed_);
-  const Tensor am = amax_or(am_, x);
   PackedTensors q(C, M, x);
   const PackedOut o = q.out();
+  Tensor keep;
+  const float* am = amax_or(am_, x, keep);
   // the tile kernel takes whole 128-token tiles: same bits, faster than the register-tiled kernel
-  if (M % 128 == 0) run_tile(x, nullptr, &o, word(am), signs, mode, Seed(), seed);
-  else check(lib.nvfp4_quant_cols_rht(x.const_data_ptr(), (int)M, (int)C, o.d, o.s, NVFP4_SCALES_SWIZZLED, word(am), o.gs,
+  if (M % 128 == 0) run_tile(x, nullptr, &o, am, signs, mode, Seed(), seed);
+  else check(lib.nvfp4_quant_cols_rht(x.const_data_ptr(), (int)M, (int)C, o.d, o.s, NVFP4_SCALES_SWIZZLED, am, o.gs,
                                       signs & 0xFFFFu, mode, seed.host, seed.dev, stream()), "quant_cols_rht");
   return q.tuple();
 }
@@ -223,12 +240,13 @@ py::tuple nvq_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py:
   const int64_t M = x.size(0), C = x.size(1);
   REQUIRE(M % 128 == 0 && C % 128 == 0, shape_of(M, C));
   const Seed seed(seed_), seed_cols(seed_cols_);
-  const Tensor am = amax_or(am_, x);
   std::optional<PackedTensors> qr, qc;
   PackedOut r, c;
   if (want_rows) { qr.emplace(M, C, x); r = qr->out(); }
   if (want_cols) { qc.emplace(C, M, x); c = qc->out(); }
-  run_tile(x, want_rows ? &r : nullptr, want_cols ? &c : nullptr, word(am), signs, mode, seed, seed_cols);
+  Tensor keep;
+  const float* am = amax_or(am_, x, keep);
+  run_tile(x, want_rows ? &r : nullptr, want_cols ? &c : nullptr, am, signs, mode, seed, seed_cols);
   return py::make_tuple(qr ? py::object(qr->tuple()) : py::none(), qc ? py::object(qc->tuple()) : py::none());
 }
 
@@ -240,7 +258,6 @@ py::tuple nvq_quant_w2d(const Tensor& w_, const OptTensor& am_, bool want, bool 
   const Tensor w = w_.contiguous();
   const int64_t N = w.size(0), K = w.size(1);
   REQUIRE(N % 128 == 0 && K % 128 == 0, shape_of(N, K));
-  const Tensor am = amax_or(am_, w);
   const Tensor gs = empty({1}, at::kFloat, w);
   auto alloc = [&](int64_t R, int64_t C, Tensor& d, Tensor& s) {
     d = empty({R, C / 2}, at::kFloat4_e2m1fn_x2, w);
@@ -251,7 +268,8 @@ py::tuple nvq_quant_w2d(const Tensor& w_, const OptTensor& am_, bool want, bool 
   PackedOut q, qt;
   if (want) q = alloc(N, K, d, s);
   if (want_t) qt = alloc(K, N, dt, st);
-  run_w2d(w, want ? &q : nullptr, want_t ? &qt : nullptr, word(am));
+  Tensor keep;
+  run_w2d(w, want ? &q : nullptr, want_t ? &qt : nullptr, amax_or(am_, w, keep));
   return py::make_tuple(want ? py::object(py::make_tuple(d, s, gs)) : py::none(),
                         want_t ? py::object(py::make_tuple(dt, st, gs)) : py::none());
 }
@@ -264,11 +282,11 @@ void nvq_quant_w2d_into(const Tensor& w_, const OptTensor& am_, const OptTensor&
   at::NoGradGuard no_grad;
   const Tensor w = w_.contiguous();
   REQUIRE(w.size(0) % 128 == 0 && w.size(1) % 128 == 0, shape_of(w.size(0), w.size(1)));
-  const Tensor am = amax_or(am_, w);
   float* g = static_cast<float*>(gs.data_ptr());
   const PackedOut q{d ? d->data_ptr() : nullptr, s ? s->data_ptr() : nullptr, g};
   const PackedOut qt{dt ? dt->data_ptr() : nullptr, st ? st->data_ptr() : nullptr, g};
-  run_w2d(w, d ? &q : nullptr, dt ? &qt : nullptr, word(am));
+  Tensor keep;
+  run_w2d(w, d ? &q : nullptr, dt ? &qt : nullptr, amax_or(am_, w, keep));
 }
 
 // A block-scaled GEMM into `out` (or a fresh tensor): alpha = product of the two words as `alpha_mode` says.
@@ -344,7 +362,10 @@ std::pair<Tensor, Tensor> backward_core(const Tensor& gy, const Packed& wt, cons
   Carver c{static_cast<char*>(scratch.data_ptr())};
   carve(c, qg, qgt, own_am);
   const float* am = a.am ? word(*a.am) : a.am_out ? word(*a.am_out) : own_am;
-  if (!a.am) run_amax(gy, const_cast<float*>(am), !a.am_out);
+  if (!a.am) {
+    if (a.am_out) run_amax(gy, const_cast<float*>(am), false);
+    else am = passing_amax(gy, own_am);
+  }
   run_tile(gy, a.want_x ? &qg : nullptr, a.want_w ? &qgt : nullptr, am, a.signs, a.mode, seed, seed_cols);
   if (a.want_x) {
     gx = empty({T, a.K}, at::kBFloat16, gy);
@@ -521,14 +542,14 @@ Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py
     const Tensor scratch = empty({(int64_t)size.used}, at::kByte, x);
     Carver c{static_cast<char*>(scratch.data_ptr())};
     carve(c, am_x, am_w);
-    run_amax(x.contiguous(), am_x);
+    const float* amx = passing_amax(x.contiguous(), am_x);
     if (!cached) {
-      run_amax(w, am_w);
+      const float* amw = passing_amax(w, am_w);
       if (keep_w) wq.gs = kept.wt.gs;         // both orientations share one tensor scale, which the backward pass reads
-      run_w2d(w, &wq, keep_w ? &kept.wt : nullptr, am_w);
+      run_w2d(w, &wq, keep_w ? &kept.wt : nullptr, amw);
       qw = wq;
     }
-    y = forward_core(x, am_x, qw, N, need_w ? &kept.xt : nullptr, signs);
+    y = forward_core(x, amx, qw, N, need_w ? &kept.xt : nullptr, signs);
   }
   if (need_x || need_w) {
     node = std::shared_ptr<LinearNode>(new LinearNode(), torch::autograd::deleteNode);

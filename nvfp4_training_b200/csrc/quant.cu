@@ -5,6 +5,7 @@
 
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 #include "common.cuh"
 
@@ -28,6 +29,8 @@ __device__ __forceinline__ uint4 ld_cg_128(const uint4* p) {
 struct AmaxSlot { u32 bits, done; };
 constexpr int kAmaxSlots = 1024;
 __device__ AmaxSlot g_amax_slots[kAmaxSlots];
+struct AmaxWords { float v[8]; };
+__device__ AmaxWords g_amax_words[kAmaxSlots];      // see nvfp4_amax_bf16_word
 
 // Running maximum of |x| as integer bit patterns (non-negative floats order like unsigned ints): bf16 values in both
 // halves of a word, FP32 values whole.
@@ -39,33 +42,32 @@ __device__ __forceinline__ u32 amax_take(u32 m, const uint4& v) {
   return __vmaxu2(m, v.w & 0x7FFF7FFFu);
 }
 
-// HBM-bound: 6.8 TB/s on tensors of 300 MB and more.  With a slot the launch needs no cleared output: every block
-// raises the slot and the last one to arrive moves the result to `out` and leaves the slot zero.  (A memset in front of
-// the kernel cost 1.4 us of its own and a launch gap, against 2-6 us of kernel on tensors of up to 16 MB.)
+// HBM-bound: 6.9 TB/s on tensors of 300 MB and more.  A thread keeps four loads in flight all the time (the oldest is
+// consumed and replaced): batches of four with a wait in between left the memory idle once per batch, which on a tensor
+// of two or three batches is a fifth of the time (46 MB: 11.0 -> 8.7 us; 33 MB from L2: 4.6 -> 3.8 us).
+// Where the result goes:
+//   slot null    raise *out, which is zero or a running maximum; `next`, if any, is a word to clear for a later launch
+//   slot given   *out needs no clearing: every block raises the slot, the last one to arrive moves the result to *out and
+//                leaves the slot zero (1.8 us for the two dependent atomics and fences; a memset in front is 1.4 us, a
+//                launch, and no programmatic launch across it)
 template <bool F32>
-__global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, long long nv, float* out, AmaxSlot* slot) {
+__global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, long long nv, float* out, float* next, AmaxSlot* slot) {
   pdl_trigger();
   pdl_wait();
   u32 m = 0u;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  // batches of four loads in flight per thread.  The last, partial batch clamps the indices past the end to the last
-  // element (a maximum does not mind reading it again) rather than walking one load at a time: on a 33 MB tensor a
-  // thread has seven loads, and three of them in sequence cost more than the first four together.
+  const long long stride = (long long)gridDim.x * blockDim.x, last = nv - 1;
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + 3 * stride < nv; i += 4 * stride) {
-    uint4 v[4];
+  if (next && i == 0) *next = 0.f;
+  uint4 v[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) v[j] = ld_cg_128(x + i + j * stride);
+  for (int j = 0; j < 4; j++) v[j] = ld_cg_128(x + min(i + j * stride, last));      // a maximum does not mind reading the last one again
+  for (i += 4 * stride; i - 4 * stride < nv;) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) m = amax_take<F32>(m, v[j]);
-  }
-  if (i < nv) {
-    const long long last = nv - 1;
-    uint4 v[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) v[j] = ld_cg_128(x + min(i + j * stride, last));
-#pragma unroll
-    for (int j = 0; j < 4; j++) m = amax_take<F32>(m, v[j]);
+    for (int j = 0; j < 4; j++) {
+      m = amax_take<F32>(m, v[j]);
+      if (i < nv) v[j] = ld_cg_128(x + i);
+      i += stride;
+    }
   }
   // bf16: NaN patterns (> 0x7F80) count as +inf;  FP32: a NaN is larger than every number and stays
   u32 mm = F32 ? m : min(max(m & 0xFFFFu, m >> 16), 0x7F80u) << 16;
@@ -249,46 +251,16 @@ template <> struct RawRow<float> {
   }
 };
 
-// Transposition of the 16 x 16 nibbles that the 16 lanes of a half-warp hold (lane i: nibble j of {lo, hi} = element
-// (i, j)): four butterfly steps, each swapping half of every lane's 64 bits with the lane at distance 8, 4, 2, 1.
-struct NibbleTranspose {
-  bool b8, b1;
-  u32 send4, lo4, hi4, send2, lo2, hi2;      // byte selectors of the two middle steps
-  __device__ __forceinline__ explicit NibbleTranspose(int lane) {
-    b8 = lane & 8; b1 = lane & 1;
-    send4 = (lane & 4) ? 0x5410u : 0x7632u; lo4 = (lane & 4) ? 0x3254u : 0x5410u; hi4 = (lane & 4) ? 0x3276u : 0x7610u;
-    send2 = (lane & 2) ? 0x6420u : 0x7531u; lo2 = (lane & 2) ? 0x3514u : 0x5240u; hi2 = (lane & 2) ? 0x3716u : 0x7260u;
-  }
-  __device__ __forceinline__ uint2 operator()(uint2 v) const {
-    u32 lo = v.x, hi = v.y;
-    u32 r = __shfl_xor_sync(0xffffffffu, b8 ? lo : hi, 8);
-    if (b8) lo = r; else hi = r;
-    r = __shfl_xor_sync(0xffffffffu, __byte_perm(lo, hi, send4), 4);
-    lo = __byte_perm(lo, r, lo4); hi = __byte_perm(hi, r, hi4);
-    r = __shfl_xor_sync(0xffffffffu, __byte_perm(lo, hi, send2), 2);
-    lo = __byte_perm(lo, r, lo2); hi = __byte_perm(hi, r, hi2);
-    constexpr u32 L = 0x0F0F0F0Fu, H = 0xF0F0F0F0u;
-    r = __shfl_xor_sync(0xffffffffu, b1 ? (lo & L) | ((hi << 4) & H) : ((lo >> 4) & L) | (hi & H), 1);
-    lo = b1 ? (lo & H) | (r & L) : (lo & L) | ((r << 4) & H);
-    hi = b1 ? (hi & H) | ((r >> 4) & L) : (hi & L) | (r & H);
-    return make_uint2(lo, hi);
-  }
-};
-
-// A half-warp owns a patch of 64 rows (N) x 32 columns (K) of W, a lane one row of each 16 x 16 block: block maximum by
-// four shuffles, eight bytes of codes per block and lane, the transposed block's row of codes by NibbleTranspose.  The
-// patch gives every lane 16 contiguous bytes of codes of W per row and 32 of W^T, and the two halves of a warp
-// neighbour along K, so that a warp reads 128 and writes 32 contiguous bytes per row.  All loads of the patch (for
-// FP32: of one row of it) are issued before the first block is quantized: that, not occupancy, is what keeps HBM busy.
-// HBM / issue bound: 7 instructions per value instead of 12 for a block spread over 32 lanes with 8 single-nibble
-// shuffles.  FULL: whole patches and 16-byte aligned outputs; otherwise 4-byte stores with bounds checks.
-template <typename T, bool FULL>
+// Any N and K that are multiples of 16 (weights in whole 128 x 128 tiles take the TMA-fed kernel of quant_w2d.cu): a
+// half-warp owns 64 rows (N) x 32 columns (K) of W, a lane one row of each 16 x 16 block; block maximum by four
+// shuffles, the transposed block's row of codes by NibbleTranspose, bounds-checked 4-byte stores.  L1-bound: the 32
+// lanes of a load or store are on 32 rows.
+template <typename T>
 __global__ void __launch_bounds__(256, 2) quant_w2d_kernel(const T* __restrict__ w, unsigned char* __restrict__ q,
                                                            unsigned char* __restrict__ s, unsigned char* __restrict__ qt,
                                                            unsigned char* __restrict__ st, const float* __restrict__ amax,
                                                            int N, int K, int layout, float* __restrict__ gs_out) {
   constexpr int NB = 4, KB = 2;                      // blocks of the patch along N and K
-  constexpr int AHEAD = sizeof(T) == 2 ? NB : 1;     // rows in flight per lane: 128 to 256 bytes, what the registers allow
   pdl_trigger();
   const int lane = threadIdx.x & 31, i = lane & 15;
   const int nb = N >> 4, kb = K >> 4;
@@ -296,81 +268,42 @@ __global__ void __launch_bounds__(256, 2) quant_w2d_kernel(const T* __restrict__
   const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int gn = (int)(item / kgroups) * NB;         // first block row, block column of this half-warp's patch
   const int gk = (int)(item % kgroups) * (2 * KB) + (lane >> 4) * KB;
-  const bool any = gn < nb;
   __shared__ __align__(8) float lut[kLutFloats];
   pdl_wait();
-  RawRow<T> raw[AHEAD][KB];
-  auto fetch = [&](int b) {
-#pragma unroll
-    for (int c = 0; c < KB; c++) {
-      if (FULL ? any : (gn + b < nb && gk + c < kb)) raw[b % AHEAD][c].load(w + (long long)((gn + b) * 16 + i) * K + (gk + c) * 16);
-      else raw[b % AHEAD][c].clear();
-    }
-  };
-#pragma unroll
-  for (int b = 0; b < AHEAD; b++) fetch(b);
   const TensorScale ts = make_tensor_scale<NVFP4_ROUND_NEAREST>(ld_cg_f32(amax), 1.f, lut,
                                                                (blockIdx.x == 0 && threadIdx.x == 0) ? gs_out : nullptr);
-  if (FULL && !any) return;
   const NibbleTranspose transpose(lane);
   unsigned char* s_sw = layout == NVFP4_SCALES_BOTH ? s + (long long)N * kb : s;
   unsigned char* st_sw = layout == NVFP4_SCALES_BOTH ? st + (long long)K * nb : st;
-  uint2 wt[KB][NB];
-  u32 sb_t[KB] = {};                                 // scale bytes of the patch, four block rows packed
+  const bool linear = layout != NVFP4_SCALES_SWIZZLED, swizzled = layout != NVFP4_SCALES_LINEAR;
 #pragma unroll
-  for (int b = 0; b < NB; b++) {
-    uint2 wq[KB];
-    u32 sb_w = 0u;
+  for (int c = 0; c < KB; c++) {
 #pragma unroll
-    for (int c = 0; c < KB; c++) {
+    for (int b = 0; b < NB; b++) {
+      const bool in = gn + b < nb && gk + c < kb;
+      const int rn = (gn + b) * 16 + i, rk = (gk + c) * 16 + i;        // this lane's row of W and of W^T
+      RawRow<T> raw;
+      if (in) raw.load(w + (long long)rn * K + (gk + c) * 16); else raw.clear();
       u64 P[8];
-      raw[b % AHEAD][c].pairs(P);
+      raw.pairs(P);
       float m = absmax16(P);
 #pragma unroll
       for (int o = 8; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
       const u32 sb = block_scale_byte(m, ts);
-      wq[c] = quant_block16<NVFP4_ROUND_NEAREST>(P, sb, ts, 0u, 0u, 0u);
-      if (qt) wt[c][b] = transpose(wq[c]);
-      sb_w |= sb << (8 * c);
-      sb_t[c] |= sb << (8 * b);
-    }
-    if (b + AHEAD < NB) fetch(b + AHEAD);
-    const int row = (gn + b) * 16 + i;
-    if (q) {
-      unsigned char* dst = q + (long long)row * (K >> 1) + gk * 8;
-      if (FULL) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(wq[0].x, wq[0].y, wq[1].x, wq[1].y);
-        if (layout != NVFP4_SCALES_SWIZZLED) *reinterpret_cast<unsigned short*>(s + (long long)row * kb + gk) = (unsigned short)sb_w;
-        if (layout != NVFP4_SCALES_LINEAR) *reinterpret_cast<unsigned short*>(s_sw + sw_off(row, gk, kb >> 2)) = (unsigned short)sb_w;
-      } else {
-#pragma unroll
-        for (int c = 0; c < KB; c++)
-          if (gn + b < nb && gk + c < kb) {
-            reinterpret_cast<u32*>(dst + 8 * c)[0] = wq[c].x; reinterpret_cast<u32*>(dst + 8 * c)[1] = wq[c].y;
-            if (layout != NVFP4_SCALES_SWIZZLED) s[(long long)row * kb + gk + c] = (unsigned char)(sb_w >> (8 * c));
-            if (layout != NVFP4_SCALES_LINEAR) s_sw[sw_off(row, gk + c, kb >> 2)] = (unsigned char)(sb_w >> (8 * c));
-          }
+      const uint2 wq = quant_block16<NVFP4_ROUND_NEAREST>(P, sb, ts, 0u, 0u, 0u);
+      const uint2 wt = transpose(wq);
+      if (in && q) {
+        u32* dst = reinterpret_cast<u32*>(q + (long long)rn * (K >> 1) + (gk + c) * 8);
+        dst[0] = wq.x; dst[1] = wq.y;
+        if (linear) s[(long long)rn * kb + gk + c] = (unsigned char)sb;
+        if (swizzled) s_sw[sw_off(rn, gk + c, kb >> 2)] = (unsigned char)sb;
       }
-    }
-  }
-  if (!qt) return;
-#pragma unroll
-  for (int c = 0; c < KB; c++) {
-    const int row = (gk + c) * 16 + i;               // row of W^T
-    unsigned char* dst = qt + (long long)row * (N >> 1) + gn * 8;
-    if (FULL) {
-      reinterpret_cast<uint4*>(dst)[0] = make_uint4(wt[c][0].x, wt[c][0].y, wt[c][1].x, wt[c][1].y);
-      reinterpret_cast<uint4*>(dst)[1] = make_uint4(wt[c][2].x, wt[c][2].y, wt[c][3].x, wt[c][3].y);
-      if (layout != NVFP4_SCALES_SWIZZLED) *reinterpret_cast<u32*>(st + (long long)row * nb + gn) = sb_t[c];
-      if (layout != NVFP4_SCALES_LINEAR) *reinterpret_cast<u32*>(st_sw + sw_off(row, gn, nb >> 2)) = sb_t[c];
-    } else {
-#pragma unroll
-      for (int b = 0; b < NB; b++)
-        if (gn + b < nb && gk + c < kb) {
-          reinterpret_cast<u32*>(dst + 8 * b)[0] = wt[c][b].x; reinterpret_cast<u32*>(dst + 8 * b)[1] = wt[c][b].y;
-          if (layout != NVFP4_SCALES_SWIZZLED) st[(long long)row * nb + gn + b] = (unsigned char)(sb_t[c] >> (8 * b));
-          if (layout != NVFP4_SCALES_LINEAR) st_sw[sw_off(row, gn + b, nb >> 2)] = (unsigned char)(sb_t[c] >> (8 * b));
-        }
+      if (in && qt) {
+        u32* dst = reinterpret_cast<u32*>(qt + (long long)rk * (N >> 1) + (gn + b) * 8);
+        dst[0] = wt.x; dst[1] = wt.y;
+        if (linear) st[(long long)rk * nb + gn + b] = (unsigned char)sb;
+        if (swizzled) st_sw[sw_off(rk, gn + b, nb >> 2)] = (unsigned char)sb;
+      }
     }
   }
 }
@@ -433,34 +366,88 @@ extern "C" int nvfp4_set_pdl(int on) {
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// The slot of `st` on the current device, or null where none can be had.  Launches of one stream never overlap (a
-// programmatically dependent one waits before it touches memory), so a stream needs one slot; it is found by the
-// stream's id, which is never given out twice.  Not inside a capture: a graph may be replayed on another stream beside
-// later work of this one.  The table is fixed memory of the library; streams beyond it take the memset.
-static AmaxSlot* amax_slot(cudaStream_t st) {
+// (device, unique id) of a stream outside a capture; false where there is none to be had.  Launches of one stream never
+// overlap (a programmatically dependent one waits before it touches memory), so memory that belongs to a stream is
+// free for its next launch.  Not inside a capture: a graph may be replayed on another stream beside later work of
+// this one.  Ids are never given out twice.
+static bool stream_id(cudaStream_t st, int& dev, unsigned long long& id) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  unsigned long long id = 0;
-  int dev = 0;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cudaStreamGetId(st, &id) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
     (void)cudaGetLastError();
-    return nullptr;
+    return false;
   }
-  if (cap != cudaStreamCaptureStatusNone || dev < 0 || dev >= 64) return nullptr;
-  static std::mutex lock;
-  static AmaxSlot* base[64];
-  static std::unordered_map<unsigned long long, int> index[64];
-  std::lock_guard<std::mutex> hold(lock);
+  return cap == cudaStreamCaptureStatusNone && dev >= 0 && dev < 64;
+}
+
+template <typename T>
+static T* symbol_base(const T (&sym)[kAmaxSlots], int dev) {
+  static T* base[64];
   if (!base[dev]) {
     void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_amax_slots) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
-    base[dev] = static_cast<AmaxSlot*>(p);
+    if (cudaGetSymbolAddress(&p, sym) != cudaSuccess) { (void)cudaGetLastError(); return nullptr; }
+    base[dev] = static_cast<T*>(p);
   }
+  return base[dev];
+}
+
+// The slot of a stream; null (the caller then clears with a memset) inside captures and for streams beyond the table.
+static AmaxSlot* amax_slot(cudaStream_t st) {
+  int dev;
+  unsigned long long id;
+  if (!stream_id(st, dev, id)) return nullptr;
+  static std::mutex lock;
+  static std::unordered_map<unsigned long long, int>* index = new std::unordered_map<unsigned long long, int>[64];
+  std::lock_guard<std::mutex> hold(lock);
+  AmaxSlot* base = symbol_base(g_amax_slots, dev);
+  if (!base) return nullptr;
   const auto it = index[dev].find(id);
-  if (it != index[dev].end()) return base[dev] + it->second;
+  if (it != index[dev].end()) return base + it->second;
   const int n = (int)index[dev].size();
   if (n >= kAmaxSlots) return nullptr;
   index[dev].emplace(id, n);
-  return base[dev] + n;
+  return base + n;
+}
+
+// Result words for an amax whose consumers this thread launches next on the same stream: a ring of eight per (thread,
+// stream).  The launch that fills one word clears the next, so none needs a memset or a meeting point of blocks, and a
+// word is not touched again before the thread's seventh later call on that stream.  A ring per thread, because two
+// threads that share a stream could slip any number of calls between one's amax and its consumer.  The rings are fixed
+// memory of the library; a thread's are handed on, per stream, when it ends; calls beyond the table get null.
+struct WordRing { unsigned long long id; int dev, slot; unsigned at; };
+struct WordRings {
+  static std::mutex& lock() { static std::mutex* m = new std::mutex; return *m; }
+  static std::vector<WordRing>& spare() { static auto* v = new std::vector<WordRing>; return *v; }
+  static int* taken() { static int n[64]; return n; }
+  std::vector<WordRing> mine;
+  ~WordRings() {
+    std::lock_guard<std::mutex> hold(lock());
+    spare().insert(spare().end(), mine.begin(), mine.end());
+  }
+  WordRing* find(int dev, unsigned long long id) {
+    for (WordRing& r : mine)
+      if (r.id == id && r.dev == dev) return &r;
+    std::lock_guard<std::mutex> hold(lock());
+    for (size_t k = 0; k < spare().size(); k++)
+      if (spare()[k].id == id && spare()[k].dev == dev) {
+        mine.push_back(spare()[k]);
+        spare().erase(spare().begin() + k);
+        return &mine.back();
+      }
+    if (taken()[dev] >= kAmaxSlots) return nullptr;
+    mine.push_back(WordRing{id, dev, taken()[dev]++, 0u});
+    return &mine.back();
+  }
+};
+
+template <bool F32>
+static cudaError_t amax_start(const void* x, long long nv, float* out, float* next, AmaxSlot* slot, cudaStream_t st) {
+  // four loads per thread and four CTAs per SM (or as many as there is work for)
+  long long blocks = (nv + 256 * 4 - 1) / (256 * 4);
+  const long long cap = (long long)sm_count() * 4;
+  if (blocks > cap) blocks = cap;
+  const cudaError_t rc = nvfp4_launch_kernel(amax_kernel<F32>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const uint4*>(x), nv, out, next, slot);
+  if (rc != cudaSuccess) (void)cudaGetLastError();
+  return rc;
 }
 
 // `n` values, 16 / sizeof of them per load
@@ -474,14 +461,28 @@ static int amax_launch(const void* x, long long n, float* out, bool clear, void*
   AmaxSlot* slot = clear && n > 0 ? amax_slot(st) : nullptr;
   if (clear && !slot && cudaMemsetAsync(out, 0, sizeof(float), st) != cudaSuccess) return NVFP4_ERR_CUDA;
   if (n == 0) return NVFP4_OK;
-  const long long nv = n / kPer;
-  long long blocks = (nv + 256 * 4 - 1) / (256 * 4);
-  const long long cap = (long long)sm_count() * 8;
-  if (blocks > cap) blocks = cap;
-  if (nvfp4_launch_kernel(amax_kernel<F32>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const uint4*>(x), nv, out, slot) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return NVFP4_ERR_CUDA;
+  return amax_start<F32>(x, n / kPer, out, nullptr, slot, st) == cudaSuccess ? NVFP4_OK : NVFP4_ERR_CUDA;
+}
+
+extern "C" int nvfp4_amax_bf16_word(const void* x, long long n, float* fallback, const float** word, void* stream) {
+  if (!word || !x) return NVFP4_ERR_NULL;
+  if (n <= 0 || (n & 7)) return NVFP4_ERR_SHAPE;
+  if (!aligned16(x)) return NVFP4_ERR_ALIGN;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  static thread_local WordRings rings;
+  int dev;
+  unsigned long long id;
+  WordRing* ring = stream_id(st, dev, id) ? rings.find(dev, id) : nullptr;
+  AmaxWords* base = ring ? symbol_base(g_amax_words, dev) : nullptr;
+  if (!base) {
+    *word = fallback;
+    return fallback ? nvfp4_amax_bf16(x, n, fallback, stream) : NVFP4_OK;
   }
+  AmaxWords& w = base[ring->slot];
+  float* out = &w.v[ring->at & 7u];
+  if (amax_start<false>(x, n >> 3, out, &w.v[(ring->at + 1u) & 7u], nullptr, st) != cudaSuccess) return NVFP4_ERR_CUDA;
+  ring->at++;
+  *word = out;
   return NVFP4_OK;
 }
 
@@ -564,6 +565,11 @@ extern "C" int nvfp4_quant_cols_rht(const void* x, int M, int C, void* codes, vo
   return NVFP4_OK;
 }
 
+// the TMA-fed kernel (quant_w2d.cu)
+bool nvfp4_quant_w2d_tile_accepts(const void* w, int N, int K, const void* q, const void* s, const void* qt, const void* st);
+int nvfp4_quant_w2d_tile_launch(const void* w, int w_dtype, int N, int K, void* q, void* s, void* qt, void* st, int scale_layout,
+                                const float* amax, float* gs_out, void* stream);
+
 extern "C" int nvfp4_quant_w2d(const void* w, int w_dtype, int N, int K, void* q, void* s, void* qt, void* st_,
                                int scale_layout, const float* amax, float* gs_out, void* stream) {
   if (!w || !amax || (!q && !qt) || (q && !s) || (qt && !st_)) return NVFP4_ERR_NULL;
@@ -575,15 +581,16 @@ extern "C" int nvfp4_quant_w2d(const void* w, int w_dtype, int N, int K, void* q
     return NVFP4_ERR_ALIGN;
   if (N == 0 || K == 0) return NVFP4_OK;
   cudaStream_t stm = static_cast<cudaStream_t>(stream);
-  const bool full = !(N & 63) && !(K & 63) && aligned16(q) && aligned16(qt) && !(reinterpret_cast<uintptr_t>(s) & 1u);
+  if (nvfp4_quant_w2d_tile_accepts(w, N, K, q, s, qt, st_))
+    return nvfp4_quant_w2d_tile_launch(w, w_dtype, N, K, q, s, qt, st_, scale_layout, amax, gs_out, stream);
   const long long warps = (long long)(((N >> 4) + 3) / 4) * (((K >> 4) + 3) / 4);
   const dim3 grid((unsigned)((warps + 7) / 8));
   unsigned char *qp = static_cast<unsigned char*>(q), *sp = static_cast<unsigned char*>(s);
   unsigned char *qtp = static_cast<unsigned char*>(qt), *stp = static_cast<unsigned char*>(st_);
   cudaError_t rc;
-#define NVFP4_W2D(T, FULL) nvfp4_launch_kernel(quant_w2d_kernel<T, FULL>, grid, dim3(256), 0, stm, static_cast<const T*>(w), qp, sp, qtp, stp, amax, N, K, scale_layout, gs_out)
-  if (w_dtype == NVFP4_DTYPE_BF16) rc = full ? NVFP4_W2D(__nv_bfloat16, true) : NVFP4_W2D(__nv_bfloat16, false);
-  else rc = full ? NVFP4_W2D(float, true) : NVFP4_W2D(float, false);
+#define NVFP4_W2D(T) nvfp4_launch_kernel(quant_w2d_kernel<T>, grid, dim3(256), 0, stm, static_cast<const T*>(w), qp, sp, qtp, stp, amax, N, K, scale_layout, gs_out)
+  if (w_dtype == NVFP4_DTYPE_BF16) rc = NVFP4_W2D(__nv_bfloat16);
+  else rc = NVFP4_W2D(float);
 #undef NVFP4_W2D
   if (rc != cudaSuccess) {
     (void)cudaGetLastError();

@@ -319,6 +319,7 @@ int nvfp4_quant_tc_launch(const void* x, long long ldx, int M, int C, void* code
 int nvfp4_quant_tc_status(int* out, int reset);
 void nvfp4_quant_tc_set_rht(int on);
 int nvfp4_emit_rows_ring_status(int* out, int reset);
+int nvfp4_quant_w2d_status(int* out, int reset);
 
 // 0 = tensor-core-fed kernel where it applies, 1 = always the scalar tile kernel, 2 = tensor-core-fed kernel with the
 // Hadamard transform inside the MMA
@@ -419,6 +420,10 @@ extern "C" int nvfp4_quant_tile_status(int* out, int reset) {
   int ring = 0;
   const int rc2 = nvfp4_emit_rows_ring_status(&ring, reset);
   if (rc2 != NVFP4_OK) return rc2;
+  int w2d = 0;
+  const int rc3 = nvfp4_quant_w2d_status(&w2d, reset);
+  if (rc3 != NVFP4_OK) return rc3;
+  if (*out == 0 && w2d) *out = 48;          // weight quantizer waiting for a tile
   if (*out == 0 && ring) *out = 32 + ring;  // TMA-fed row emitter: 33 producer, 34 consumer
   if (*out == 0 && tc) *out = 16 + tc;    // tensor-core-fed kernel: 17 / 19 its loading and MMA-issuing warp (waiting for a tile / a free stage), 18 a consumer
   return NVFP4_OK;
