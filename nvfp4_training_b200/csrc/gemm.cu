@@ -23,14 +23,14 @@
 
 #include "tma.cuh"
 
+// 16-byte store of finished bf16 output with the streaming hint: the output is not read again by this
+// kernel and should not push operand tiles out of L2 (measured +3 % on 16384x11264x2048, neutral elsewhere)
+#define NVFP4_STORE_C16(ptr, v) __stcs(reinterpret_cast<uint4*>(ptr), v)
+
 // Waits of warps that have nothing else to do (producer waiting for a free stage, epilogue waiting
 // for an accumulator) carry a suspend-time hint: the warp sleeps in hardware instead of polling,
 // which measured 1-2 % faster on the large shapes (fewer issue slots and less power spent spinning).
 #define NVFP4_IDLE_WAIT mbar_wait_parked
-
-// 16-byte store of finished bf16 output with the streaming hint: the output is not read again by this
-// kernel and should not push operand tiles out of L2 (measured +3 % on 16384x11264x2048, neutral elsewhere)
-#define NVFP4_STORE_C16(ptr, v) __stcs(reinterpret_cast<uint4*>(ptr), v)
 
 namespace nvfp4 {
 
@@ -387,8 +387,8 @@ gemm_nvf4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 //   leader      warp 1 copies scales to tensor memory (both CTAs at once), issues the MMAs and commits
 //               to the `empty` / `acc_full` barriers of both CTAs (one commit per CTA)
 //   both CTAs   warps 2..9 drain their accumulator, arrive on the leader's `acc_empty` barrier, then
-//               convert and store through a per-warp 4 KB staging area so that every global store
-//               instruction writes whole 128-byte (FP32) or 64-byte (bf16) row segments
+//               convert and store: straight from registers in 32-byte pieces (256-wide tiles), or through a
+//               per-warp staging area so that every store or atomic add covers whole row segments
 template <int BN>
 struct PairCfg {
   // BN = 256: one 256x256 tile per CTA pair, two accumulators that overlap in 48 tensor-memory columns
@@ -545,6 +545,32 @@ __device__ __forceinline__ bool sched_wait(u32 sched0, u32 k, volatile int* abor
       if (t0 == 0) t0 = now;
       else if (now - t0 > kWaitLimitNs) { *abort_flag = 1; return false; }
       __nanosleep(100);
+    }
+  }
+}
+
+// A lane's NCOLS values of one row of C, straight from its registers in 32-byte pieces (whole sectors).
+template <int NCOLS>
+__device__ __forceinline__ void direct_store(const u32 (&r)[NCOLS], float alpha, void* row, bool fp32, int valid_cols) {
+  auto st32 = [](void* p, const u32 (&o)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]),
+                 "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < NCOLS; i += 8) {
+    if (i >= valid_cols) break;               // columns beyond N (multiples of 32): nothing to store
+    u32 o[8];
+    if (fp32) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) o[k] = __float_as_uint(__uint_as_float(r[i + k]) * alpha);
+      st32(static_cast<float*>(row) + i, o);
+    } else if (!(i & 8)) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(r[i + 2 * k]) * alpha, __uint_as_float(r[i + 2 * k + 1]) * alpha);
+        o[k] = *reinterpret_cast<const u32*>(&h);
+      }
+      st32(static_cast<__nv_bfloat16*>(row) + i, o);
     }
   }
 }
@@ -922,12 +948,21 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       else if (p.alpha_mode == NVFP4_ALPHA_AMAX) alpha = ld_cg_f32(p.pa) * ld_cg_f32(p.pb) * p.kscale;
       else if (p.alpha_mode == NVFP4_ALPHA_ROW) alpha = ld_cg_f32(p.pa + row0 + lane) * ld_cg_f32(p.pb);   // each lane stages its own row
       const long long col0 = (long long)nt * BN + half * NC;
+      const int valid = (int)min((long long)NC, (long long)p.N - col0);
       // (a warp's 32 rows never straddle two owners: rows_per_owner is a multiple of 128)
       float* cf = p.rows_per_owner ? p.owner_c[(int)row0 / p.rows_per_owner] : static_cast<float*>(p.c);
       void* cbase = p.c_fp32 ? static_cast<void*>(cf + row0 * p.ldc + col0)
                              : static_cast<void*>(static_cast<__nv_bfloat16*>(p.c) + row0 * p.ldc + col0);
-      staged_store<NC, C::kStageRowBytes>(r, alpha, sw, lane, cbase, p.ldc, p.c_fp32 != 0, p.atomic != 0,
-                                          (int)min((long long)NC, (long long)p.N - col0));
+      // Finished output of the 256-wide tile leaves straight from registers: through the staging area every value
+      // crosses shared memory twice more, which costs cycles and, the chip being power-limited here, clock
+      // ([16384, 11264, 2048] 195 -> 186 us, [4096, 11264, 2048] 53.7 -> 49.1, FP32 [49152, 2048, 4096] 215 -> 202,
+      // sustained; TMA stores from the staging area: 213, 55.2, 218).  Atomic adds stay coalesced, and so do the narrower
+      // tiles' stores (a lane's piece of a row is not whole 128-byte lines there: [8192, 3072, 2048] 31.3 against 32.2).
+      if (BN == 256 && !p.atomic && !(reinterpret_cast<uintptr_t>(cbase) & 31u) && !((p.ldc * (p.c_fp32 ? 4 : 2)) & 31))
+        direct_store<NC>(r, alpha, p.c_fp32 ? static_cast<void*>(static_cast<float*>(cbase) + lane * p.ldc)
+                                            : static_cast<void*>(static_cast<__nv_bfloat16*>(cbase) + lane * p.ldc), p.c_fp32 != 0, valid);
+      else
+        staged_store<NC, C::kStageRowBytes>(r, alpha, sw, lane, cbase, p.ldc, p.c_fp32 != 0, p.atomic != 0, valid);
     }
     if (!ok && lane == 0 && p.status) atomicExch(p.status, 13);
   }
