@@ -73,6 +73,7 @@ struct GemmParams {
   int atomic;         // 1: add into C with FP32 atomics
   int splitk;         // number of K slices
   int ktiles_per_split;
+  int wide_store;     // C and its rows are 32-byte aligned
 };
 
 // ---------------------------------------------------------------------------------------- PTX wrappers
@@ -147,7 +148,74 @@ __device__ __forceinline__ u64 pack64(u32 lo, u32 hi) {
 constexpr u32 kDescHiAB = (1024u >> 4) | (1u << 14) | (2u << 29);
 constexpr u32 kDescHiSF = (128u >> 4) | (1u << 14);
 
-template <int BN>
+__device__ __forceinline__ u32 cluster_ctarank() { u32 r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ u32 map_to_cta(u32 saddr, u32 rank) {
+  u32 r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ float alpha_of(const GemmParams& p, long long row) {
+  if (p.alpha_mode == NVFP4_ALPHA_GS) return ld_cg_f32(p.pa) * ld_cg_f32(p.pb);
+  if (p.alpha_mode == NVFP4_ALPHA_AMAX) return ld_cg_f32(p.pa) * ld_cg_f32(p.pb) * p.kscale;
+  if (p.alpha_mode == NVFP4_ALPHA_ROW) return ld_cg_f32(p.pa + row) * ld_cg_f32(p.pb);
+  return 1.f;
+}
+
+// N finished values of one row of C (alpha applied): stores in 32-byte pieces where C's rows are aligned to them (half the
+// store instructions), else in 16-byte pieces, or FP32 atomic adds.
+template <int N>
+__device__ __forceinline__ void store_row(const float (&v)[N], const GemmParams& p, long long row, long long col) {
+  constexpr int W = N < 16 ? N / 2 : 8;                  // words of a piece of a bf16 row
+  if (p.c_fp32) {
+    float* dst = static_cast<float*>(p.c) + row * p.ldc + col;
+#pragma unroll
+    for (int i = 0; i < N; i += 8) {
+      if (!p.atomic && p.wide_store) {
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + i), "f"(v[i]), "f"(v[i + 1]), "f"(v[i + 2]),
+                     "f"(v[i + 3]), "f"(v[i + 4]), "f"(v[i + 5]), "f"(v[i + 6]), "f"(v[i + 7]) : "memory");
+      } else {
+#pragma unroll
+        for (int j = i; j < i + 8; j += 4) {
+          if (p.atomic)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + j), "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]) : "memory");
+          else
+            *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
+      }
+    }
+  } else {
+    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.c) + row * p.ldc + col;
+#pragma unroll
+    for (int i = 0; i < N; i += 2 * W) {
+      u32 o[W];
+#pragma unroll
+      for (int k = 0; k < W; k++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[i + 2 * k], v[i + 2 * k + 1]);
+        o[k] = *reinterpret_cast<const u32*>(&h);
+      }
+      if constexpr (W == 8) {
+        if (p.wide_store) {
+          asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + i), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]),
+                       "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
+          continue;
+        }
+        *reinterpret_cast<uint4*>(dst + i + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+      *reinterpret_cast<uint4*>(dst + i) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
+// Contractions with few output tiles (a short prompt, a weight gradient of a small layer): S > 1 CTAs of a cluster share
+// one 128 x 128 tile, each multiplying every S-th part of K; the partial sums meet in shared memory.  What bounds the
+// plain kernel there is one tensor core working through all of K beside 130 idle ones: [256, 2048] x K = 5632 took 14.5 us
+// on 16 CTAs of 128 x 256, in slices 8.8.
+template <int BN, int S>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_nvf4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
   using C = Cfg<BN>;
@@ -167,6 +235,10 @@ gemm_nvf4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const int tiles_m = p.M / kBM, tiles_n = p.N / BN;
   const int ktiles = (p.K + kBK - 1) / kBK;
   const int num_work = tiles_m * tiles_n * p.splitk;
+  // S == 1: work items dealt out in turn.  S > 1: one item, this CTA's slice of its cluster's tile (splitk == S).
+  const u32 rank = S > 1 ? cluster_ctarank() : 0u;
+  const int first = S > 1 ? (int)rank * tiles_m * tiles_n + (int)(blockIdx.x / S) : (int)blockIdx.x;
+  const int step = S > 1 ? num_work : (int)gridDim.x;
   const u32 smem_base = smem_u32(smem);
   const u32 full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
 
@@ -200,13 +272,13 @@ gemm_nvf4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     u32 st_addr = smem_base;
     const long long sf_row_bytes = (long long)(p.K >> 6) * 512;   // scale bytes of one 128-row block
     bool ok = true;
-    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
+    for (int w = first; w < num_work && ok; w += step) {
       const int mt = w % tiles_m;
       const int rest = w / tiles_m;
       const int nt = rest % tiles_n;
       const int z = rest / tiles_n;
-      const int kt0 = z * p.ktiles_per_split;
-      const int kt1 = min(ktiles, kt0 + p.ktiles_per_split);
+      const int kt0 = S > 1 ? ktiles * z / S : z * p.ktiles_per_split;
+      const int kt1 = S > 1 ? ktiles * (z + 1) / S : min(ktiles, kt0 + p.ktiles_per_split);
       const unsigned char* sfa = p.sfa + (long long)mt * sf_row_bytes + (long long)kt0 * 2048;
       const unsigned char* sfb = p.sfb + (long long)(nt * (BN / 128)) * sf_row_bytes + (long long)kt0 * 2048;
       const int ya = mt * kBM, yb = nt * BN;
@@ -242,10 +314,10 @@ gemm_nvf4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     u32 a_lo = a_lo0;
     int acc = 0; u32 acc_phase = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
+    for (int w = first; w < num_work && ok; w += step) {
       const int z = w / (tiles_m * tiles_n);
-      const int kt0 = z * p.ktiles_per_split;
-      const int kt1 = min(ktiles, kt0 + p.ktiles_per_split);
+      const int kt0 = S > 1 ? ktiles * z / S : z * p.ktiles_per_split;
+      const int kt1 = S > 1 ? ktiles * (z + 1) / S : min(ktiles, kt0 + p.ktiles_per_split);
       // the epilogue must have drained this accumulator
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(acc_empty + acc), acc_phase ^ 1u, abort_flag))) { ok = false; break; }
       tc_fence_after();
@@ -306,7 +378,7 @@ gemm_nvf4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int half = (warp - 2) >> 2;                  // which half of the tile's columns
     int acc = 0; u32 acc_phase = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
+    for (int w = first; w < num_work && ok; w += step) {
       const int mt = w % tiles_m;
       const int nt = (w / tiles_m) % tiles_n;
       // the decision must be warp-uniform: the tensor-memory loads below are warp-collective
@@ -322,41 +394,58 @@ gemm_nvf4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (lane == 0) mbar_arrive(smem_u32(acc_empty + acc));
       if (++acc == C::kAccStages) { acc = 0; acc_phase ^= 1u; }
 
+      if constexpr (S > 1) {
+        // this CTA's MMAs and loads are complete: its stages hold the partial sums, [warp][4 columns][lane] x 16 bytes
+        const u32 mine = smem_base + (u32)(warp - 2) * (kEpiCols * 128) + (u32)lane * 16u;
+#pragma unroll
+        for (int i = 0; i < kEpiCols; i += 4)
+          asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(mine + i * 128), "r"(r[i]), "r"(r[i + 1]), "r"(r[i + 2]),
+                       "r"(r[i + 3]) : "memory");
+        break;
+      }
       const long long row = (long long)mt * kBM + quad * 32 + lane;
-      float alpha = 1.f;
-      if (p.alpha_mode == NVFP4_ALPHA_GS) alpha = ld_cg_f32(p.pa) * ld_cg_f32(p.pb);
-      else if (p.alpha_mode == NVFP4_ALPHA_AMAX) alpha = ld_cg_f32(p.pa) * ld_cg_f32(p.pb) * p.kscale;
-      else if (p.alpha_mode == NVFP4_ALPHA_ROW) alpha = ld_cg_f32(p.pa + row) * ld_cg_f32(p.pb);   // this lane's row
-      const long long col = (long long)nt * BN + half * kEpiCols;
-      if (p.c_fp32) {
-        float* dst = static_cast<float*>(p.c) + row * p.ldc + col;
-        if (p.atomic) {
+      const float alpha = alpha_of(p, row);
 #pragma unroll
-          for (int i = 0; i < kEpiCols; i += 4)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + i),
-                         "f"(__uint_as_float(r[i]) * alpha), "f"(__uint_as_float(r[i + 1]) * alpha),
-                         "f"(__uint_as_float(r[i + 2]) * alpha), "f"(__uint_as_float(r[i + 3]) * alpha) : "memory");
-        } else {
+      for (int i = 0; i < kEpiCols; i += 16) {
+        float v[16];
 #pragma unroll
-          for (int i = 0; i < kEpiCols; i += 4)
-            *reinterpret_cast<float4*>(dst + i) = make_float4(__uint_as_float(r[i]) * alpha, __uint_as_float(r[i + 1]) * alpha,
-                                                              __uint_as_float(r[i + 2]) * alpha, __uint_as_float(r[i + 3]) * alpha);
-        }
-      } else {
-        __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.c) + row * p.ldc + col;
-#pragma unroll
-        for (int i = 0; i < kEpiCols; i += 8) {
-          uint4 o;
-          __nv_bfloat162 h;
-          h = __floats2bfloat162_rn(__uint_as_float(r[i]) * alpha, __uint_as_float(r[i + 1]) * alpha); o.x = *reinterpret_cast<u32*>(&h);
-          h = __floats2bfloat162_rn(__uint_as_float(r[i + 2]) * alpha, __uint_as_float(r[i + 3]) * alpha); o.y = *reinterpret_cast<u32*>(&h);
-          h = __floats2bfloat162_rn(__uint_as_float(r[i + 4]) * alpha, __uint_as_float(r[i + 5]) * alpha); o.z = *reinterpret_cast<u32*>(&h);
-          h = __floats2bfloat162_rn(__uint_as_float(r[i + 6]) * alpha, __uint_as_float(r[i + 7]) * alpha); o.w = *reinterpret_cast<u32*>(&h);
-          *reinterpret_cast<uint4*>(dst + i) = o;
-        }
+        for (int k = 0; k < 16; k++) v[k] = __uint_as_float(r[i + k]) * alpha;
+        store_row<16>(v, p, row, (long long)nt * BN + half * kEpiCols + i);
       }
     }
     if (!ok && lane == 0 && p.status) atomicExch(p.status, 3);
+  }
+
+  if constexpr (S > 1) {
+    // every CTA of the cluster gets here (each wait above is bounded); each sums BN / S columns over all slices, in
+    // slice order, and stores them
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= 2) {
+      constexpr int kCols = BN / 2 / S;                  // of this warp's 64 columns
+      const int tile = blockIdx.x / S, mt = tile % tiles_m, nt = tile / tiles_m;
+      const int quad = warp & 3, half = (warp - 2) >> 2;
+      const u32 at = smem_base + (u32)(warp - 2) * (BN / 2 * 128) + rank * (kCols * 128) + (u32)lane * 16u;
+      float v[kCols];
+#pragma unroll
+      for (int z = 0; z < S; z++) {
+        const u32 src = map_to_cta(at, (u32)z);
+#pragma unroll
+        for (int i = 0; i < kCols; i += 4) {
+          float4 f;
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "r"(src + i * 128) : "memory");
+          v[i] = z ? v[i] + f.x : f.x; v[i + 1] = z ? v[i + 1] + f.y : f.y;
+          v[i + 2] = z ? v[i + 2] + f.z : f.z; v[i + 3] = z ? v[i + 3] + f.w : f.w;
+        }
+      }
+      const long long row = (long long)mt * kBM + quad * 32 + lane;
+      const float alpha = alpha_of(p, row);
+#pragma unroll
+      for (int i = 0; i < kCols; i++) v[i] *= alpha;
+      if (!*abort_flag) store_row<kCols>(v, p, row, (long long)nt * BN + half * (BN / 2) + rank * kCols);
+    }
+    __syncwarp();
+    cluster_sync_all();                                  // nobody leaves while its partial sums are being read
   }
 
   // ------------------------------------------------------------------ teardown
@@ -418,16 +507,6 @@ struct PairCfg {
 };
 
 
-__device__ __forceinline__ u32 cluster_ctarank() { u32 r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ u32 map_to_cta(u32 saddr, u32 rank) {
-  u32 r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // Arrival on a (possibly remote) barrier that hands tensor memory back to the MMA warp.  Relaxed on
 // purpose: the hand-off is ordered by tcgen05.fence::before_thread_sync; a releasing arrive would
 // also wait for this thread's earlier global stores (the previous tile's output) to become visible.
@@ -1014,7 +1093,7 @@ static bool make_sf_map(CUtensorMap* map, const void* base, long long rows, long
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-struct DevInfo { int sms; bool attr128, attr256, attr_pair, attr_pair128, attr_pair192; unsigned* counters; };
+struct DevInfo { int sms; int clusters[3]; bool attr128, attr256, attr_slices[3], attr_pair, attr_pair128, attr_pair192; unsigned* counters; };
 static DevInfo* dev_info() {
   static DevInfo info[64];
   static bool init[64] = {false};
@@ -1023,7 +1102,10 @@ static DevInfo* dev_info() {
   if (!init[dev]) {
     int n = 0;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return nullptr;
-    info[dev].sms = n; info[dev].attr128 = info[dev].attr256 = info[dev].attr_pair = info[dev].attr_pair128 = info[dev].attr_pair192 = false;
+    info[dev].sms = n;
+    info[dev].clusters[0] = info[dev].clusters[1] = info[dev].clusters[2] = -1;
+    info[dev].attr_slices[0] = info[dev].attr_slices[1] = info[dev].attr_slices[2] = false;
+    info[dev].attr128 = info[dev].attr256 = info[dev].attr_pair = info[dev].attr_pair128 = info[dev].attr_pair192 = false;
     void* ctr = nullptr;
     if (cudaGetSymbolAddress(&ctr, g_tile_counters) != cudaSuccess) return nullptr;
     info[dev].counters = static_cast<unsigned*>(ctr);
@@ -1032,22 +1114,45 @@ static DevInfo* dev_info() {
   return &info[dev];
 }
 
-template <int BN>
+template <int BN, int S = 1>
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sms, bool& attr_done,
                        cudaStream_t st) {
   using C = Cfg<BN>;
   if (!attr_done) {
-    if (cudaFuncSetAttribute(gemm_nvf4_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_nvf4_kernel<BN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess)
       return NVFP4_ERR_CUDA;
     attr_done = true;
   }
   const long long work = (long long)(p.M / kBM) * (p.N / BN) * p.splitk;
-  const unsigned grid = (unsigned)(work < sms ? work : sms);
-  if (nvfp4_launch_kernel(gemm_nvf4_kernel<BN>, dim3(grid), dim3(kThreads), C::kSmemBytes, st, ma, mb, p) != cudaSuccess) {
+  const unsigned grid = (unsigned)(work < sms || S > 1 ? work : sms);
+  if (nvfp4_launch_grouped(gemm_nvf4_kernel<BN, S>, S, false, dim3(grid), dim3(kThreads), C::kSmemBytes, st, ma, mb, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return NVFP4_ERR_CUDA;
   }
   return NVFP4_OK;
+}
+
+// How many clusters of S CTAs of the sliced kernel the device runs at the same time.
+template <int S>
+static int query_clusters() {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(S); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = Cfg<128>::kSmemBytes;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaFuncSetAttribute(gemm_nvf4_kernel<128, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<128>::kSmemBytes) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, gemm_nvf4_kernel<128, S>, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+static int clusters_at_once(DevInfo* di, int S) {
+  int& n = di->clusters[S == 2 ? 0 : S == 4 ? 1 : 2];
+  if (n < 0) n = S == 2 ? query_clusters<2>() : S == 4 ? query_clusters<4>() : query_clusters<8>();
+  return n;
 }
 
 }  // namespace nvfp4
@@ -1070,6 +1175,7 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   if ((accumulate || splitk > 1) && c_dtype != NVFP4_DTYPE_FP32) return NVFP4_ERR_ENUM;
   const bool auto_split = splitk == 0;      // the library picks the number of K slices (FP32 output only)
   if (auto_split) splitk = 1;
+  if (splitk > 1) accumulate = 1;           // slices asked for are added to C, however many there turn out to be
   if (!al16(a) || !al16(b) || !al16(sa) || !al16(sb) || !al16(c) || (lda & 15) || (ldb & 15) || (ldc & 7))
     return NVFP4_ERR_ALIGN;
   if (M == 0 || N == 0) return NVFP4_OK;
@@ -1088,7 +1194,21 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   if (g_sm_budget > 0 && g_sm_budget < sms) sms = g_sm_budget >= 2 ? (g_sm_budget & ~1) : 2;
 
   const int ktiles = (K + kBK - 1) / kBK;
-  if (auto_split && c_dtype == NVFP4_DTYPE_FP32 && g_force_bn == 0 && ktiles >= 16) {
+  const long long tiles128 = (long long)(M / kBM) * (N / 128), pairs = (long long)((M + 255) / 256) * ((N + 255) / 256);
+  // Few output tiles: one-CTA tiles with K in `slices` over a cluster fill more SMs than CTA pairs.  As many slices as run
+  // at once (not quite all SMs for clusters of 4 and 8: an SM group holds whole ones only; a second round costs more than
+  // it gives, [128, 2048] x K = 5632 took 14.8 us in 16 clusters of 8, 8.1 in clusters of 4), with two K tiles or more
+  // each, and enough of them saved to pay for the exchange (about 1.5 us, 0.27 us per K tile).
+  bool few = g_force_bn == 0 && !owners && pairs < sms / 4;
+  int slices = 1;
+  if (few) {
+    while (slices < 8 && ktiles >= 4 * slices && tiles128 * 2 * slices <= sms && tiles128 <= clusters_at_once(di, 2 * slices)) slices *= 2;
+    if (ktiles * (slices - 1) < 6 * slices) slices = 1;
+    // where atomic adds are allowed, CTA pairs in more slices win once a slice is long ([2048, 512] x K = 16384, 32 K tiles
+    // in each of two slices: 16.6 against 15.0 us; 16 in each of four, [640, 640]: 11.6 against 12.3)
+    if ((auto_split || splitk > 1) && c_dtype == NVFP4_DTYPE_FP32 && ktiles > 20 * slices) few = false;
+  }
+  if (auto_split && c_dtype == NVFP4_DTYPE_FP32 && g_force_bn == 0 && ktiles >= 16 && !few) {
     // Weight-gradient shapes have few output tiles and a long contraction: 96 or 176 tiles over 74 SM pairs leave
     // a third of the machine idle in the last round.  Slicing K evens that out; the price is the per-tile fixed
     // cost once more per slice, FP32 atomic adds instead of stores, and a zero fill when the call overwrites C.
@@ -1114,20 +1234,37 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
     }
   }
   if (splitk > ktiles) splitk = ktiles;
+  if (splitk > 1 && g_force_bn == 0 && !owners && !auto_split) {
+    // The caller's number of slices is an upper bound.  A slice that adds no parallelism costs a pass of atomic adds over
+    // C (3 TB/s) and the per-tile fixed cost once more: [3072, 1024] x K = 2048 in 8 slices took 32 us, in one 11 us.
+    // Same cost model as the tile-width choice below, in units of 0.72 us.
+    const long long ncl = sms / 2;
+    const int most = few ? 1 : splitk;
+    double best = 0;
+    int pick = 1;
+    for (int s = 1; s <= most; s++) {
+      const int per_s = (ktiles + s - 1) / s;
+      if ((ktiles + per_s - 1) / per_s != s) continue;
+      const long long t192 = (long long)((M + 255) / 256) * ((N + 191) / 192) * s;
+      double cost = (double)((t192 + ncl - 1) / ncl) * (1.88 + 0.3255 * per_s);
+      if (N % 256 == 0) cost = fmin(cost, (double)((pairs * s + ncl - 1) / ncl) * (2.98 + 0.346 * per_s));
+      if (s > 1) cost = fmax(cost, (double)s * (double)M * (double)N * 4.0 / (3.0e6 * 0.72));
+      if (s == 1 || cost < best * 0.97) { best = cost; pick = s; }
+    }
+    splitk = pick;
+  }
   int per = (ktiles + splitk - 1) / splitk;
   splitk = (ktiles + per - 1) / per;
+  // CTA-pair kernels (an SM pair per 256-row tile): the fast path unless there are too few tiles for it
+  bool use_pair = g_force_bn != 128 && g_force_bn != 256 && !(g_force_bn == 0 && pairs * splitk < sms / 4);
+  if (owners) use_pair = true;                    // the scatter lives in the pair kernel's epilogue only
 
-  // 256-wide tiles move fewer operand bytes per FLOP and need fewer issue slots; fall back to 128
-  // when N demands it or when wide tiles would leave SMs without work
-  bool wide = (N % 256 == 0) && ((long long)(M / kBM) * (N / 256) * splitk >= sms || (long long)(M / kBM) * (N / 128) * splitk <= sms);
+  // one-CTA tiles: 256-wide ones only where they keep every SM busy
+  bool wide = (N % 256 == 0) && (long long)(M / kBM) * (N / 256) * splitk >= sms;
   if (g_force_bn == 128) wide = false;
   if (g_force_bn == 256 && N % 256 == 0) wide = true;
   const int bn = wide ? 256 : 128;
 
-  // CTA-pair kernels (an SM pair per 256-row tile): the fast path whenever M allows it
-  bool use_pair = g_force_bn != 128 && g_force_bn != 256;
-  if (g_force_bn == 0 && (long long)((M + 255) / 256) * ((N + 255) / 256) * splitk < sms / 4) use_pair = false;   // too few tiles: finer tiles fill more SMs
-  if (owners) use_pair = true;                    // the scatter lives in the pair kernel's epilogue only
   if (use_pair) {
     // tile width: 256 moves the fewest operand bytes per FLOP but consecutive tiles wait for each other's
     // epilogue hand-off; 192 has two independent accumulators and handles any N; 128 as well, more bytes
@@ -1202,6 +1339,13 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   p.atomic = (accumulate || splitk > 1) ? 1 : 0;
   p.splitk = splitk;
   p.ktiles_per_split = per;
+  p.wide_store = !(reinterpret_cast<uintptr_t>(c) & 31u) && !((ldc * (p.c_fp32 ? 4 : 2)) & 31);
+  if (splitk == 1) {
+    p.splitk = slices;
+    if (slices == 2) return launch_gemm<128, 2>(ma, mb, p, sms, di->attr_slices[0], st);
+    if (slices == 4) return launch_gemm<128, 4>(ma, mb, p, sms, di->attr_slices[1], st);
+    if (slices == 8) return launch_gemm<128, 8>(ma, mb, p, sms, di->attr_slices[2], st);
+  }
   if (wide) return launch_gemm<256>(ma, mb, p, sms, di->attr256, st);
   return launch_gemm<128>(ma, mb, p, sms, di->attr128, st);
 }

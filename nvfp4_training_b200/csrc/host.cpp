@@ -705,13 +705,13 @@ Tensor k_gemm(const Tensor& ad, const Tensor& as, const OptTensor& asw, const Te
   if (!fp32) {
     out = empty({M, N}, at::kBFloat16, ad);
   } else {
-    out = out_ ? *out_ : at::zeros({M, N}, ad.options().dtype(at::kFloat));
+    out = out_ ? *out_ : empty({M, N}, at::kFloat, ad);       // a fresh result is stored, the library slices K as it sees fit
     REQUIRE(out.scalar_type() == at::kFloat && out.stride(1) == 1, "gemm: out is FP32 with contiguous rows");
   }
   const Tensor sa = asw ? *asw : k_swizzle(as, std::nullopt), sb = bsw ? *bsw : k_swizzle(bs, std::nullopt);
   check(lib.nvfp4_gemm(ad.const_data_ptr(), sa.const_data_ptr(), ad.stride(0), bd.const_data_ptr(), sb.const_data_ptr(), bd.stride(0),
                        out.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16, out.stride(0), (int)M, (int)N, (int)K,
-                       NVFP4_ALPHA_AMAX, word(aam), word(bam), ak, bk, fp32, splitk, status_word(ad), stream()), "gemm");
+                       NVFP4_ALPHA_AMAX, word(aam), word(bam), ak, bk, fp32 && out_, fp32 && !out_ ? 0 : splitk, status_word(ad), stream()), "gemm");
   return out;
 }
 
