@@ -372,11 +372,17 @@ static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t
 // this one.  Ids are never given out twice.
 static bool stream_id(cudaStream_t st, int& dev, unsigned long long& id) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cudaStreamGetId(st, &id) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+  if (st == cudaStreamPerThread) return false;              // one handle, a stream per thread
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
     (void)cudaGetLastError();
     return false;
   }
-  return cap == cudaStreamCaptureStatusNone && dev >= 0 && dev < 64;
+  if (cap != cudaStreamCaptureStatusNone) return false;     // asking a capturing stream for its id would end the capture
+  if (cudaStreamGetId(st, &id) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return dev >= 0 && dev < 64;
 }
 
 template <typename T>

@@ -61,3 +61,32 @@ def test_host_errors_keep_their_types():
     q = nvq.quant_rows(torch.ones(128, 64, dtype=torch.bfloat16, device="cuda"))
     with pytest.raises(AssertionError):
         nvq.mm(q, nvq.quant_rows(torch.ones(128, 128, dtype=torch.bfloat16, device="cuda")))
+
+
+@pytest.mark.parametrize("T,K,N", [(128, 128, 256), (1024, 2048, 640)])
+def test_calls_that_need_an_amax_can_be_captured(T, K, N):
+    from nvfp4_training_b200 import fp4ops, nvq
+    lin, x, gy = _layer(T, K, N, False)
+    w32 = lin.weight.detach().float()
+
+    def run():
+        xg = x.clone().requires_grad_(True)
+        y = lin(xg)
+        q, qt = nvq.quant_w2d(lin.weight)
+        k, kt = fp4ops.quant_w2d(w32)
+        r, c = nvq.quant_rows(x), nvq.quant_cols_rht(x, 0xA6B1)
+        return [y.detach(), *torch.autograd.grad(y, (xg, lin.weight), gy), nvq.amax(x), fp4ops.amax_of(w32), q.gs, k.s, kt.d, fp4ops.quant_rows(x).s,
+                q.d.view(torch.uint8), qt.s.view(torch.uint8), r.d.view(torch.uint8), c.d.view(torch.uint8)]
+    want = run()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run()
+    for _ in range(2):
+        for t in got:
+            t.zero_()
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
