@@ -495,6 +495,10 @@ struct LinearNode : torch::autograd::Node {
 Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py::handle cache, unsigned signs) {
   require_cuda(x_);
   const Tensor w_ = w_opt.value_or(Tensor());
+  if (torch::autograd::isFwGradDefined(x_) || torch::autograd::isFwGradDefined(w_opt)) {
+    PyErr_SetString(PyExc_NotImplementedError, "the NVFP4 linear has no jvp: forward-mode AD is not supported");
+    throw py::error_already_set();
+  }
   const bool cached = !cache.is_none();
   const bool grad = at::GradMode::is_enabled();
   const bool need_x = grad && x_.requires_grad(), need_w = grad && w_.defined() && w_.requires_grad();

@@ -90,3 +90,11 @@ def test_calls_that_need_an_amax_can_be_captured(T, K, N):
             t.zero_()
         graph.replay()
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_forward_mode_is_refused():
+    import torch.autograd.forward_ad as fwd
+    lin, x, _ = _layer(128, 128, 128, False)
+    with fwd.dual_level():
+        with pytest.raises(NotImplementedError):
+            lin(fwd.make_dual(x, torch.ones_like(x)))
