@@ -129,13 +129,15 @@ __device__ __forceinline__ u32 e2m1x4_rs(float v0, float v1, float v2, float v3,
 // Stochastic rounding onto the E2M1 grid by adding 22 random bits below the kept mantissa bit
 // and truncating (the reference's method, llm-1b/nvq.cu:32-39).  The result is exactly
 // representable, so the round-to-nearest convert that follows is exact.
+// (a <= 6 and the bits of 6.0 plus 22 set bits truncate to 6.0 again, so the result needs no second clamp; the lift of
+// values below 1 is added, not selected.  The quantizers in this mode are bound by the integer and compare pipe:
+// [16384, 5632], both operands, 192 -> 162 us.)
 __device__ __forceinline__ float sr_dither(float v, u32 rnd) {
-  float a = fminf(fabsf(v), 6.f);
-  bool sub = a < 1.f;
-  float b = sub ? __fadd_rn(a, 1.f) : a;
-  u32 bits = (__float_as_uint(b) + (rnd & 0x3FFFFFu)) & ~0x3FFFFFu;
-  float r = __fsub_rn(__uint_as_float(bits), sub ? 1.f : 0.f);
-  return copysignf(fminf(r, 6.f), v);
+  const float a = fminf(fabsf(v), 6.f);
+  float lift;
+  asm("set.lt.f32.f32 %0, %1, 0f3F800000;" : "=f"(lift) : "f"(a));
+  const u32 bits = (__float_as_uint(__fadd_rn(a, lift)) + (rnd & 0x3FFFFFu)) & ~0x3FFFFFu;
+  return __uint_as_float(__float_as_uint(__fsub_rn(__uint_as_float(bits), lift)) | (__float_as_uint(v) & 0x80000000u));
 }
 
 // Internal modes of the operand emitters (llm-1b/emit.cu arithmetic: block scale and values by
