@@ -144,9 +144,12 @@ __device__ __forceinline__ void q_settle_copies() {
   while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
 }
 
-// Walks the tiles of one CTA in (token tile, column tile) coordinates without a division per tile.
+// Walks the tiles of one CTA in (token tile, column tile) coordinates without a division per tile, the last token
+// rows first: the amax kernel has read the tensor front to back, so of a tensor larger than L2 the end is still there
+// (weight gradient of [16384, 5632] and [16384, 2048] with its quantizers and amax passes: 214.4 -> 210.2 us).
 struct TcWalk {
   int mt, ct, dq, dr, nct, nmt;
+  __device__ __forceinline__ int row_tile() const { return nmt - 1 - mt; }
   __device__ __forceinline__ TcWalk(int M, int C) {
     nct = C / kQCol; nmt = M / kQTok;
     mt = (int)blockIdx.x / nct; ct = (int)blockIdx.x - mt * nct;
@@ -186,8 +189,8 @@ __global__ void __launch_bounds__(kQThreads, 2) quant_tc_kernel(const __grid_con
     if (elect_one()) {
       const u32 bar = full0 + 8 * stage, dst = tiles0 + stage * kQTileBytes;
       mbar_arrive_expect_tx(bar, kQTileBytes);
-      tma_load_2d(dst, &map, tw.ct * kQCol, tw.mt * kQTok, bar);
-      tma_load_2d(dst + kQBoxBytes, &map, tw.ct * kQCol + 64, tw.mt * kQTok, bar);
+      tma_load_2d(dst, &map, tw.ct * kQCol, tw.row_tile() * kQTok, bar);
+      tma_load_2d(dst + kQBoxBytes, &map, tw.ct * kQCol + 64, tw.row_tile() * kQTok, bar);
     }
     __syncwarp();
   };
@@ -362,7 +365,7 @@ __global__ void __launch_bounds__(kQThreads, 2) quant_tc_kernel(const __grid_con
       if (ROWS) q_ld16(t_lane, first16); else q_ld32(t_lane, first32);
     }
     for (; alive && tw.valid(); n++) {
-      const int mt = tw.mt, ct = tw.ct;
+      const int mt = tw.row_tile(), ct = tw.ct;
       const u32 buf0 = BOTH ? 0u : (n & 1u), par = BOTH ? (n & 1u) : ((n >> 1) & 1u);
       tw.next();
       const bool more = tw.valid();
