@@ -157,6 +157,18 @@ int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void* codes_r, 
                      unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
                      const unsigned* seed_r_dev, const unsigned* seed_c_dev, void* stream);
 
+/*
+ * nvfp4_quant_tile for a small tensor whose amax nobody has computed yet: one launch of one thread-block cluster that
+ * keeps the tensor in shared memory, finds max|x| (NaN counts as infinity, as in nvfp4_amax_bf16) and quantizes from
+ * there.  amax_out (optional) receives it.  *launched (a host variable) is 1 where that has been enqueued, and 0, with
+ * nothing enqueued and NVFP4_OK, where the two separate calls are needed: more than 8 tiles of 128 x 128, shapes of the
+ * scalar kernel, launches the device refuses.  Same bits as the two calls.  No reference counterpart.
+ */
+int nvfp4_quant_tile_amax(const void* x, long long ldx, int M, int C, void* codes_r, void* scales_r, void* codes_c,
+                          void* scales_c, int scale_layout, float* amax_out, int* launched, float* gs_r_out, float* gs_c_out,
+                          unsigned signs, int rounding, unsigned seed_r, unsigned seed_c, const unsigned* seed_r_dev,
+                          const unsigned* seed_c_dev, void* stream);
+
 /* Tuning / test hook: 0 = nvfp4_quant_tile picks the tensor-core-fed kernel where it applies (default),
  * 1 = always the scalar tile kernel, 2 = the tensor-core-fed kernel with the 16-point Hadamard transform of the
  * transposed operand computed by the MMA itself (B operand = rows of H diag(signs)) instead of FP32 butterflies, as

@@ -35,7 +35,7 @@ namespace {
 
 // ------------------------------------------------------------------------------------------ library entry points
 #define NVFP4_API(X)                                                                                                        \
-  X(nvfp4_amax_bf16) X(nvfp4_amax_bf16_update) X(nvfp4_quant_rows) X(nvfp4_quant_cols_rht) X(nvfp4_quant_tile)             \
+  X(nvfp4_amax_bf16) X(nvfp4_amax_bf16_update) X(nvfp4_quant_rows) X(nvfp4_quant_cols_rht) X(nvfp4_quant_tile) X(nvfp4_quant_tile_amax)             \
   X(nvfp4_quant_w2d) X(nvfp4_gemm) X(nvfp4_error_string) X(nvfp4_amax_f32) X(nvfp4_amax_bf16_word) X(nvfp4_swizzle_scales) X(nvfp4_emit_rows)        \
   X(nvfp4_emit_cols) X(nvfp4_rms_emit) X(nvfp4_swiglu_emit) X(nvfp4_mom_acc)
 struct Api {
@@ -160,6 +160,17 @@ void run_tile(const Tensor& x, const PackedOut* row, const PackedOut* col, const
                              seed_cols.host, seed.dev, seed_cols.dev, stream()), "quant_tile");
 }
 
+// The same with the tensor's amax found on the way (into `amax_out`, unless that is null); false: not launched
+bool run_tile_amax(const Tensor& x, const PackedOut* row, const PackedOut* col, float* amax_out, unsigned signs, int mode, const Seed& seed,
+                   const Seed& seed_cols) {
+  int launched = 0;
+  check(lib.nvfp4_quant_tile_amax(x.const_data_ptr(), x.stride(0), (int)x.size(0), (int)x.size(1), row ? row->d : nullptr,
+                                  row ? row->s : nullptr, col ? col->d : nullptr, col ? col->s : nullptr, NVFP4_SCALES_SWIZZLED, amax_out,
+                                  &launched, row ? row->gs : nullptr, col ? col->gs : nullptr, signs & 0xFFFFu, mode, seed.host,
+                                  seed_cols.host, seed.dev, seed_cols.dev, stream()), "quant_tile_amax");
+  return launched != 0;
+}
+
 void run_w2d(const Tensor& w, const PackedOut* q, const PackedOut* qt, const float* am) {
   check(lib.nvfp4_quant_w2d(w.const_data_ptr(), NVFP4_DTYPE_BF16, (int)w.size(0), (int)w.size(1), q ? q->d : nullptr,
                             q ? q->s : nullptr, qt ? qt->d : nullptr, qt ? qt->s : nullptr, NVFP4_SCALES_SWIZZLED, am,
@@ -224,6 +235,7 @@ py::tuple nvq_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, py::han
   const Seed seed(seed_);
   PackedTensors q(C, M, x);
   const PackedOut o = q.out();
+  if (!am_ && M % 128 == 0 && run_tile_amax(x, nullptr, &o, nullptr, signs, mode, Seed(), seed)) return q.tuple();
   Tensor keep;
   const float* am = amax_or(am_, x, keep);
   // the tile kernel takes whole 128-token tiles: same bits, faster than the register-tiled kernel
@@ -244,9 +256,11 @@ py::tuple nvq_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py:
   PackedOut r, c;
   if (want_rows) { qr.emplace(M, C, x); r = qr->out(); }
   if (want_cols) { qc.emplace(C, M, x); c = qc->out(); }
-  Tensor keep;
-  const float* am = amax_or(am_, x, keep);
-  run_tile(x, want_rows ? &r : nullptr, want_cols ? &c : nullptr, am, signs, mode, seed, seed_cols);
+  if (am_ || !(want_rows || want_cols) || !run_tile_amax(x, want_rows ? &r : nullptr, want_cols ? &c : nullptr, nullptr, signs, mode, seed, seed_cols)) {
+    Tensor keep;
+    const float* am = amax_or(am_, x, keep);
+    run_tile(x, want_rows ? &r : nullptr, want_cols ? &c : nullptr, am, signs, mode, seed, seed_cols);
+  }
   return py::make_tuple(qr ? py::object(qr->tuple()) : py::none(), qc ? py::object(qc->tuple()) : py::none());
 }
 
@@ -318,15 +332,25 @@ Tensor nvq_mm(const Tensor& ad, const Tensor& as, const Tensor& ag, const Tensor
 }
 
 // ------------------------------------------------------------------------------------------ the linear layer
-// y = Q_rn(x) Q(W)^T with the row operand of x in scratch; `xt` (optional) receives the transposed operand.
-Tensor forward_core(const Tensor& x, const float* am, const Packed& w, int64_t N, const PackedOut* xt, unsigned signs) {
+// y = Q_rn(x) Q(W)^T with the row operand of x in scratch; `xt` (optional) receives the transposed operand.  `am`: the
+// caller's amax(x); null: it is found here, into `am_out` (unless that is null too).
+Tensor forward_core(const Tensor& x, const float* am, float* am_out, const Packed& w, int64_t N, const PackedOut* xt, unsigned signs) {
   const int64_t T = x.size(0), K = x.size(1);
   Carver size;
   carve_packed(size, T, K);
   const Tensor scratch = empty({(int64_t)size.used}, at::kByte, x);
   Carver c{static_cast<char*>(scratch.data_ptr())};
   const PackedOut qx = carve_packed(c, T, K);
-  run_tile(x, &qx, xt, am, signs, NVFP4_ROUND_NEAREST, Seed(), Seed());
+  if (am || !run_tile_amax(x, &qx, xt, am_out, signs, NVFP4_ROUND_NEAREST, Seed(), Seed())) {
+    Tensor keep;
+    if (!am && am_out) {
+      run_amax(x.contiguous(), am_out);
+      am = am_out;
+    } else if (!am) {
+      am = amax_or(std::nullopt, x, keep);
+    }
+    run_tile(x, &qx, xt, am, signs, NVFP4_ROUND_NEAREST, Seed(), Seed());
+  }
   Tensor y = empty({T, N}, at::kBFloat16, x);
   run_mm(qx, w, y, K, false, 1);
   return y;
@@ -361,12 +385,13 @@ std::pair<Tensor, Tensor> backward_core(const Tensor& gy, const Packed& wt, cons
   const Tensor scratch = empty({(int64_t)size.used}, at::kByte, gy);
   Carver c{static_cast<char*>(scratch.data_ptr())};
   carve(c, qg, qgt, own_am);
-  const float* am = a.am ? word(*a.am) : a.am_out ? word(*a.am_out) : own_am;
-  if (!a.am) {
-    if (a.am_out) run_amax(gy, const_cast<float*>(am), false);
-    else am = passing_amax(gy, own_am);
+  const PackedOut *row = a.want_x ? &qg : nullptr, *col = a.want_w ? &qgt : nullptr;
+  if (a.am || a.am_out || !run_tile_amax(gy, row, col, nullptr, a.signs, a.mode, seed, seed_cols)) {
+    const float* am = a.am ? word(*a.am) : a.am_out ? word(*a.am_out) : own_am;
+    if (!a.am && a.am_out) run_amax(gy, const_cast<float*>(am), false);
+    else if (!a.am && gy.numel()) am = passing_amax(gy, own_am);
+    run_tile(gy, row, col, am, a.signs, a.mode, seed, seed_cols);
   }
-  run_tile(gy, a.want_x ? &qg : nullptr, a.want_w ? &qgt : nullptr, am, a.signs, a.mode, seed, seed_cols);
   if (a.want_x) {
     gx = empty({T, a.K}, at::kBFloat16, gy);
     run_mm(qg, wt, gx, N, false, 1);
@@ -392,10 +417,11 @@ py::tuple linear_fwd(const Tensor& x, const Tensor& wd, const Tensor& ws, const 
   at::NoGradGuard no_grad;
   const int64_t T = x.size(0), K = x.size(1), N = wd.size(0);
   require_packed(wd, N, K, "linear_fwd: quantized weight");
-  const Tensor am = am_out ? nvq_amax(x.contiguous(), am_out, false) : nvq_amax(x.contiguous(), std::nullopt, true);
+  REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16, "linear_fwd: a bf16 matrix");
+  const Tensor am = am_out ? nvq_amax(x.contiguous(), am_out, false) : empty({1}, at::kFloat, x);
   PackedTensors xt(K, T, x);
   const PackedOut o = xt.out();
-  Tensor y = forward_core(x, word(am), packed_of(wd, ws, wg), N, &o, signs);
+  Tensor y = forward_core(x, am_out ? word(am) : nullptr, am_out ? nullptr : am.data_ptr<float>(), packed_of(wd, ws, wg), N, &o, signs);
   return py::make_tuple(y, am, xt.d, xt.s, xt.gs);
 }
 
@@ -536,24 +562,23 @@ Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py
     const Kept kept(kc, T, K, N, need_w, keep_w);
 
     PackedOut wq;
-    auto carve = [&](Carver& c, float*& am_x, float*& am_w) {
-      am_x = c.take<float>(4);
-      if (!cached) { am_w = c.take<float>(4); wq = carve_packed(c, N, K); }
-    };
-    float *am_x = nullptr, *am_w = nullptr;
-    Carver size;
-    carve(size, am_x, am_w);
-    const Tensor scratch = empty({(int64_t)size.used}, at::kByte, x);
-    Carver c{static_cast<char*>(scratch.data_ptr())};
-    carve(c, am_x, am_w);
-    const float* amx = passing_amax(x.contiguous(), am_x);
+    Tensor scratch;
     if (!cached) {
-      const float* amw = passing_amax(w, am_w);
+      auto carve = [&](Carver& c) {
+        float* am_w = c.take<float>(4);
+        wq = carve_packed(c, N, K);
+        return am_w;
+      };
+      Carver size;
+      carve(size);
+      scratch = empty({(int64_t)size.used}, at::kByte, x);
+      Carver c{static_cast<char*>(scratch.data_ptr())};
+      const float* amw = passing_amax(w, carve(c));
       if (keep_w) wq.gs = kept.wt.gs;         // both orientations share one tensor scale, which the backward pass reads
       run_w2d(w, &wq, keep_w ? &kept.wt : nullptr, amw);
       qw = wq;
     }
-    y = forward_core(x, amx, qw, N, need_w ? &kept.xt : nullptr, signs);
+    y = forward_core(x, nullptr, nullptr, qw, N, need_w ? &kept.xt : nullptr, signs);
   }
   if (need_x || need_w) {
     node = std::shared_ptr<LinearNode>(new LinearNode(), torch::autograd::deleteNode);
@@ -645,10 +670,21 @@ py::tuple k_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py::h
   const int64_t M = x.size(0), C = x.size(1);
   REQUIRE(M % 128 == 0 && C % 64 == 0, shape_of(M, C));
   const Seed seed(seed_), seed_cols(seed_cols_);
-  const Tensor am = k_amax_or(am_, x);
   const bool both = whole_tiles(M, C);
   Tensor dr = empty({M, C / 2}, at::kByte, x), dc = empty({C, M / 2}, at::kByte, x);
   LinearScales sr(M, C, both, x), sc(C, M, both, x);
+  Tensor am;
+  int launched = 0;
+  if (am_ || !x.is_contiguous()) {
+    am = k_amax_or(am_, x);
+  } else {
+    am = empty({1}, at::kFloat, x);
+    check(lib.nvfp4_quant_tile_amax(x.const_data_ptr(), x.stride(0), (int)M, (int)C, dr.data_ptr(), sr.s.data_ptr(), dc.data_ptr(),
+                                    sc.s.data_ptr(), sr.layout, am.data_ptr<float>(), &launched, nullptr, nullptr, signs, mode, seed.host,
+                                    seed_cols.host, seed.dev, seed_cols.dev, stream()), "quant_tile_amax");
+    if (!launched) am = k_amax(x);
+  }
+  if (!launched)
   check(lib.nvfp4_quant_tile(x.const_data_ptr(), x.stride(0), (int)M, (int)C, dr.data_ptr(), sr.s.data_ptr(), dc.data_ptr(),
                              sc.s.data_ptr(), sr.layout, word(am), nullptr, nullptr, signs, mode, seed.host, seed_cols.host,
                              seed.dev, seed_cols.dev, stream()), "quant_tile");

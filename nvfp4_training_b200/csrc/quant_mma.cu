@@ -60,6 +60,7 @@ struct TcParams {
   u32 signs;
   u32 seed_r, seed_c;
   const u32* seed_r_dev; const u32* seed_c_dev;
+  float* amax_out;  // amax null: the kernel finds it (cluster_amax); optionally receives it
   int tc_rht;       // 1: the 16-point Hadamard transform itself runs in the MMA (B = signed Hadamard rows), see below
 };
 
@@ -159,7 +160,57 @@ struct TcWalk {
   __device__ __forceinline__ void next() { mt += dq; ct += dr; if (ct >= nct) { ct -= nct; mt++; } }
 };
 
-template <int ROUNDING, bool ROWS, bool COLS, bool TCRHT>
+// The tensor's largest magnitude, of a tensor of one tile per CTA of a cluster: each CTA reads its tile where TMA has put
+// it, the CTAs exchange their maxima through shared memory, and quantization goes on from there.
+// An amax kernel in front costs a launch and more time than the exchange.  NaN patterns count as +inf, as in that
+// kernel.  Called by all threads of all CTAs of the only cluster.
+__device__ __forceinline__ float cluster_amax(const TcParams& p, u32 tiles0, u32 full0, volatile int* abort_flag) {
+  __shared__ u32 warp_max[1 + kQConsumerWarps];
+  __shared__ u32 cta_max;
+  u32 m = 0u;
+  if (threadIdx.x >= 32) {                       // the consumer warps
+    if (!mbar_wait(full0, 0u, abort_flag)) {
+      atomicCAS(&g_quant_tc_status, 0, 2);
+    } else {
+      const u32 at = tiles0 + (threadIdx.x - 32u) * 16u;
+#pragma unroll
+      for (u32 k = 0; k < kQTileBytes / (kQConsumerWarps * 512); k++) {
+        u32 a, b, c, d;
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at + k * (kQConsumerWarps * 512)));
+        m = __vmaxu2(__vmaxu2(m, a & 0x7FFF7FFFu), b & 0x7FFF7FFFu);
+        m = __vmaxu2(__vmaxu2(m, c & 0x7FFF7FFFu), d & 0x7FFF7FFFu);
+      }
+    }
+  }
+  __syncwarp();
+  const u32 wm = __reduce_max_sync(0xffffffffu, min(max(m & 0xFFFFu, m >> 16), 0x7F80u) << 16);
+  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = wm;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    u32 cta = 0u;
+#pragma unroll
+    for (int w = 1; w <= kQConsumerWarps; w++) cta = max(cta, warp_max[w]);
+    cta_max = cta;
+  }
+  __syncwarp();
+  // (each wait above is bounded, so every CTA gets to the barriers)
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  u32 all = 0u;
+  for (u32 r = 0; r < gridDim.x; r++) {
+    u32 at, v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(&cta_max)), "r"(r));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+    all = max(all, v);
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");        // all have read
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const float amax = __uint_as_float(all);
+  if (p.amax_out && blockIdx.x == 0 && threadIdx.x == 0) *p.amax_out = amax;
+  return amax;
+}
+
+template <int ROUNDING, bool ROWS, bool COLS, bool TCRHT, bool FIND>
 __global__ void __launch_bounds__(kQThreads, 2) quant_tc_kernel(const __grid_constant__ CUtensorMap map, const TcParams p) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) float lut_r[kLutFloats];
@@ -236,10 +287,12 @@ __global__ void __launch_bounds__(kQThreads, 2) quant_tc_kernel(const __grid_con
     q_tmem_alloc(smem_u32(&tmem_slot), kQTmemCols);
     q_tmem_relinquish();
   }
-  // everything above touches shared and tensor memory only; the tensor's amax is the previous kernel's result
-  pdl_wait();
-  const float amax = ld_cg_f32(p.amax);
   const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  // everything above touches shared and tensor memory only; the tensor's amax may be the previous kernel's result
+  pdl_wait();
+  float amax;
+  if constexpr (FIND) amax = cluster_amax(p, tiles0, full0, abort_flag);
+  else amax = ld_cg_f32(p.amax);
   TensorScale ts_r, ts_c;
   if (ROWS) ts_r = make_tensor_scale<ROUNDING>(amax, 1.f, lut_r, first ? p.gs_r_out : nullptr);
   // the x0.25 that follows the butterflies is folded into the tensor scale (a power of two)
@@ -482,32 +535,38 @@ static bool make_tc_map(CUtensorMap* map, const void* x, long long M, long long 
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int ROUNDING, bool ROWS, bool COLS, bool TCRHT = false>
+template <int ROUNDING, bool ROWS, bool COLS, bool TCRHT, bool FIND>
 static int launch_tc(const CUtensorMap& map, const TcParams& p, int grid, cudaStream_t st) {
   static bool configured[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return NVFP4_ERR_CUDA;
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (cudaFuncSetAttribute(quant_tc_kernel<ROUNDING, ROWS, COLS, TCRHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQSmem) != cudaSuccess)
+    if (cudaFuncSetAttribute(quant_tc_kernel<ROUNDING, ROWS, COLS, TCRHT, FIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQSmem) != cudaSuccess)
       return NVFP4_ERR_CUDA;
     configured[dev] = true;
   }
-  if (nvfp4_launch_kernel(quant_tc_kernel<ROUNDING, ROWS, COLS, TCRHT>, dim3((unsigned)grid), dim3(kQThreads), kQSmem, st, map, p) != cudaSuccess) {
+  if (nvfp4_launch_grouped(quant_tc_kernel<ROUNDING, ROWS, COLS, TCRHT, FIND>, FIND ? (unsigned)grid : 1u, false, dim3((unsigned)grid), dim3(kQThreads),
+                           kQSmem, st, map, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return NVFP4_ERR_CUDA;
   }
   return NVFP4_OK;
 }
 
-template <int ROUNDING>
+template <int ROUNDING, bool FIND>
 static int launch_tc_mode(const CUtensorMap& map, const TcParams& p, int grid, cudaStream_t st) {
-  if (p.tc_rht && p.codes_c) {
-    if (p.codes_r) return launch_tc<ROUNDING, true, true, true>(map, p, grid, st);
-    return launch_tc<ROUNDING, false, true, true>(map, p, grid, st);
+  if (!FIND && p.tc_rht && p.codes_c) {
+    if (p.codes_r) return launch_tc<ROUNDING, true, true, true, false>(map, p, grid, st);
+    return launch_tc<ROUNDING, false, true, true, false>(map, p, grid, st);
   }
-  if (p.codes_r && p.codes_c) return launch_tc<ROUNDING, true, true>(map, p, grid, st);
-  if (p.codes_c) return launch_tc<ROUNDING, false, true>(map, p, grid, st);
-  return launch_tc<ROUNDING, true, false>(map, p, grid, st);
+  if (p.codes_r && p.codes_c) return launch_tc<ROUNDING, true, true, false, FIND>(map, p, grid, st);
+  if (p.codes_c) return launch_tc<ROUNDING, false, true, false, FIND>(map, p, grid, st);
+  return launch_tc<ROUNDING, true, false, false, FIND>(map, p, grid, st);
+}
+
+template <int ROUNDING>
+static int launch_tc_rounding(const CUtensorMap& map, const TcParams& p, int grid, cudaStream_t st) {
+  return p.amax ? launch_tc_mode<ROUNDING, false>(map, p, grid, st) : launch_tc_mode<ROUNDING, true>(map, p, grid, st);
 }
 
 }  // namespace nvfp4
@@ -529,10 +588,20 @@ static int g_tc_rht = 0;
 // 1: the Hadamard transform of the transposed operand runs inside the MMA instead of FP32 butterflies
 void nvfp4_quant_tc_set_rht(int on) { g_tc_rht = on ? 1 : 0; }
 
-// Arguments as nvfp4_quant_tile, already validated by it.
+// CTAs of the one cluster that finds the amax of such a tensor itself, 0 where it is too large for that: a tile per CTA.
+// us against amax kernel + quantizer, both operands, round to nearest: 1 tile 6.4 / 8.1, 8 tiles 7.5 / 8.2; 16 tiles, two
+// per CTA, 10.1 / 8.3.
+static int cluster_of(int M, int C) {
+  const long long ntiles = (long long)(M / kQTok) * (C / kQCol);
+  return ntiles > 8 ? 0 : (int)ntiles;
+}
+bool nvfp4_quant_tc_finds_amax(int M, int C) { return cluster_of(M, C) > 0; }
+
+// Arguments as nvfp4_quant_tile, already validated by it.  `amax` null: the launch finds it (nvfp4_quant_tc_finds_amax
+// sizes only) and hands it out in `amax_out`, unless that is null.
 int nvfp4_quant_tc_launch(const void* x, long long ldx, int M, int C, void* codes_r, void* scales_r, void* codes_c,
-                          void* scales_c, int scale_layout, const float* amax, float* gs_r_out, float* gs_c_out,
-                          unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
+                          void* scales_c, int scale_layout, const float* amax, float* amax_out, float* gs_r_out,
+                          float* gs_c_out, unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
                           const unsigned* seed_r_dev, const unsigned* seed_c_dev, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap map;
@@ -540,7 +609,7 @@ int nvfp4_quant_tc_launch(const void* x, long long ldx, int M, int C, void* code
   TcParams p = {};
   p.codes_r = static_cast<unsigned char*>(codes_r); p.scales_r = static_cast<unsigned char*>(scales_r);
   p.codes_c = static_cast<unsigned char*>(codes_c); p.scales_c = static_cast<unsigned char*>(scales_c);
-  p.amax = amax; p.gs_r_out = gs_r_out; p.gs_c_out = gs_c_out;
+  p.amax = amax; p.amax_out = amax_out; p.gs_r_out = gs_r_out; p.gs_c_out = gs_c_out;
   p.M = M; p.C = C; p.layout = scale_layout;
   p.signs = signs & 0xFFFFu;
   p.seed_r = seed_r; p.seed_c = seed_c; p.seed_r_dev = seed_r_dev; p.seed_c_dev = seed_c_dev;
@@ -552,13 +621,13 @@ int nvfp4_quant_tc_launch(const void* x, long long ldx, int M, int C, void* code
   }
   const long long ntiles = (long long)(M / kQTok) * (C / kQCol);
   { const int b = nvfp4_sm_budget_value(); if (b > 0 && b < sms) sms = b; }   // SMs left to a collective running beside this kernel
-  int grid = 2 * sms;
+  int grid = amax ? 2 * sms : cluster_of(M, C);
   if (ntiles < grid) grid = (int)ntiles;
   switch (rounding) {
-    case NVFP4_ROUND_NEAREST: return launch_tc_mode<NVFP4_ROUND_NEAREST>(map, p, grid, st);
-    case NVFP4_ROUND_SR_DITHER: return launch_tc_mode<NVFP4_ROUND_SR_DITHER>(map, p, grid, st);
-    case NVFP4_ROUND_SR_DITHER_K: return launch_tc_mode<NVFP4_ROUND_SR_DITHER_K>(map, p, grid, st);
-    default: return launch_tc_mode<NVFP4_ROUND_SR_HW>(map, p, grid, st);
+    case NVFP4_ROUND_NEAREST: return launch_tc_rounding<NVFP4_ROUND_NEAREST>(map, p, grid, st);
+    case NVFP4_ROUND_SR_DITHER: return launch_tc_rounding<NVFP4_ROUND_SR_DITHER>(map, p, grid, st);
+    case NVFP4_ROUND_SR_DITHER_K: return launch_tc_rounding<NVFP4_ROUND_SR_DITHER_K>(map, p, grid, st);
+    default: return launch_tc_rounding<NVFP4_ROUND_SR_HW>(map, p, grid, st);
   }
 }
 

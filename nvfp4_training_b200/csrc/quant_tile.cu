@@ -313,9 +313,10 @@ int nvfp4_sm_budget_value();   // gemm.cu: nvfp4_gemm_set_sm_budget
 bool nvfp4_quant_tc_accepts(const void* x, long long ldx, int M, int C, const void* codes_r, const void* scales_r,
                             const void* codes_c, const void* scales_c);
 int nvfp4_quant_tc_launch(const void* x, long long ldx, int M, int C, void* codes_r, void* scales_r, void* codes_c,
-                          void* scales_c, int scale_layout, const float* amax, float* gs_r_out, float* gs_c_out,
-                          unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
+                          void* scales_c, int scale_layout, const float* amax, float* amax_out, float* gs_r_out,
+                          float* gs_c_out, unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
                           const unsigned* seed_r_dev, const unsigned* seed_c_dev, void* stream);
+bool nvfp4_quant_tc_finds_amax(int M, int C);
 int nvfp4_quant_tc_status(int* out, int reset);
 void nvfp4_quant_tc_set_rht(int on);
 int nvfp4_emit_rows_ring_status(int* out, int reset);
@@ -332,11 +333,10 @@ extern "C" int nvfp4_quant_tile_set_path(int path) {
   return NVFP4_OK;
 }
 
-extern "C" int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void* codes_r, void* scales_r, void* codes_c,
-                                void* scales_c, int scale_layout, const float* amax, float* gs_r_out, float* gs_c_out,
-                                unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
-                                const unsigned* seed_r_dev, const unsigned* seed_c_dev, void* stream) {
-  if (!x || !amax || (!codes_r && !codes_c) || (codes_r && !scales_r) || (codes_c && !scales_c)) return NVFP4_ERR_NULL;
+// The checks of nvfp4_quant_tile and nvfp4_quant_tile_amax: NVFP4_OK, or the status to return.
+static int check_tile_args(const void* x, long long ldx, int M, int C, const void* codes_r, const void* scales_r, const void* codes_c,
+                           const void* scales_c, int scale_layout, int rounding) {
+  if (!x || (!codes_r && !codes_c) || (codes_r && !scales_r) || (codes_c && !scales_c)) return NVFP4_ERR_NULL;
   if (scale_layout < NVFP4_SCALES_SWIZZLED || scale_layout > NVFP4_SCALES_BOTH) return NVFP4_ERR_ENUM;
   if (rounding < NVFP4_ROUND_NEAREST || rounding > NVFP4_ROUND_SR_HW) return NVFP4_ERR_ENUM;
   if (M < 0 || C < 0 || (M % kTileTok) || (C % kTileCol) || ldx < C) return NVFP4_ERR_SHAPE;
@@ -344,10 +344,33 @@ extern "C" int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void
   if ((reinterpret_cast<uintptr_t>(x) & 15u) || (ldx & 7) || (reinterpret_cast<uintptr_t>(codes_r) & 7u) ||
       (reinterpret_cast<uintptr_t>(codes_c) & 15u) || (reinterpret_cast<uintptr_t>(scales_c) & 7u))
     return NVFP4_ERR_ALIGN;
-  if (M == 0 || C == 0) return NVFP4_OK;
+  return NVFP4_OK;
+}
+
+extern "C" int nvfp4_quant_tile_amax(const void* x, long long ldx, int M, int C, void* codes_r, void* scales_r, void* codes_c,
+                                     void* scales_c, int scale_layout, float* amax_out, int* launched, float* gs_r_out,
+                                     float* gs_c_out, unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
+                                     const unsigned* seed_r_dev, const unsigned* seed_c_dev, void* stream) {
+  if (!launched) return NVFP4_ERR_NULL;
+  *launched = 0;
+  const int rc = check_tile_args(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c, scale_layout, rounding);
+  if (rc != NVFP4_OK || M == 0 || C == 0) return rc;
+  if (g_tile_path != 0 || !nvfp4_quant_tc_accepts(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c) || !nvfp4_quant_tc_finds_amax(M, C))
+    return NVFP4_OK;
+  *launched = nvfp4_quant_tc_launch(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c, scale_layout, nullptr, amax_out, gs_r_out, gs_c_out,
+                                    signs, rounding, seed_r, seed_c, seed_r_dev, seed_c_dev, stream) == NVFP4_OK;
+  return NVFP4_OK;                      // a refused launch: the caller takes two kernels
+}
+
+extern "C" int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void* codes_r, void* scales_r, void* codes_c,
+                                void* scales_c, int scale_layout, const float* amax, float* gs_r_out, float* gs_c_out,
+                                unsigned signs, int rounding, unsigned seed_r, unsigned seed_c,
+                                const unsigned* seed_r_dev, const unsigned* seed_c_dev, void* stream) {
+  if (!amax) return NVFP4_ERR_NULL;
+  const int bad = check_tile_args(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c, scale_layout, rounding);
+  if (bad != NVFP4_OK || M == 0 || C == 0) return bad;
   if (g_tile_path != 1 && nvfp4_quant_tc_accepts(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c))
-    return nvfp4_quant_tc_launch(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c, scale_layout, amax, gs_r_out, gs_c_out,
-                                 signs, rounding, seed_r, seed_c, seed_r_dev, seed_c_dev, stream);
+    return nvfp4_quant_tc_launch(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c, scale_layout, amax, nullptr, gs_r_out, gs_c_out, signs, rounding, seed_r, seed_c, seed_r_dev, seed_c_dev, stream);
   if (scale_layout == NVFP4_SCALES_BOTH) return NVFP4_ERR_SHAPE;       // the scalar kernel writes one layout
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap map;
