@@ -97,11 +97,12 @@ int nvfp4_amax_bf16_word(const void* x, long long n, float* fallback, const floa
 int nvfp4_amax_f32(const float* x, long long n, float* out, void* stream);
 
 /*
- * Programmatic dependent launch of this library's amax, one-read quantizer and GEMM kernels: when on, such a kernel
- * may become resident and run its set-up (barriers, tensor-memory allocation, constant tables) while the previous
- * kernel of the stream drains; it waits for that kernel's completion before it touches global memory, and reads
- * global memory past L1 only.  Off by default (measured gain on the 81-linear step: 0.2-0.6 %); the environment
- * variable NVFP4_PDL=1 or this call switch it on.  Process-wide; no reference counterpart.
+ * Programmatic dependent launch of this library's amax, one-read quantizer, whole-tile weight quantizer and GEMM
+ * kernels: such a kernel may become resident and run its set-up (barriers, tensor-memory allocation, constant tables)
+ * while the previous kernel of the stream drains; it waits for that kernel's completion before it touches global memory,
+ * and reads global memory past L1 only.  0: off.  1: all these launches.  2 (the default): the short ones, which move at
+ * most 48 MB or are GEMMs of at most 1e11 multiply-adds.  The environment variable NVFP4_PDL (0, 1, 2) sets the start
+ * value.  Process-wide; no reference counterpart.
  */
 int nvfp4_set_pdl(int on);
 

@@ -26,20 +26,20 @@ typedef uint64_t u64;
 // memory only past the L1 cache (ld.global.cg, TMA, atomics): it is launched, and its SM's L1 invalidated, while
 // older kernels still run, so a line one of them reads afterwards (say a scale word at an address the allocator
 // hands out again) would otherwise still sit in L1, stale, when the staged kernel gets to read the new value.
-bool nvfp4_pdl_enabled();
+// `brief`: see nvfp4_set_pdl.
+bool nvfp4_pdl_enabled(bool brief);
 
-// `cluster`: blocks of a cluster.  `cooperative`: the blocks wait for one another; all of them are resident or the launch
-// is refused.
+// Short enough for its launch latency to matter: a launch that moves this many bytes (measured at nvfp4_pdl_enabled).
+static inline bool nvfp4_brief(long long bytes) { return bytes <= (48ll << 20); }
+
+// `cluster`: blocks of a cluster.
 template <typename... KArgs, typename... Args>
-static inline cudaError_t nvfp4_launch_grouped(void (*kernel)(KArgs...), unsigned cluster, bool cooperative, dim3 grid, dim3 block, size_t smem,
+static inline cudaError_t nvfp4_launch_grouped(void (*kernel)(KArgs...), unsigned cluster, bool brief, dim3 grid, dim3 block, size_t smem,
                                                cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  if (cooperative) {
-    attr[cfg.numAttrs].id = cudaLaunchAttributeCooperative;
-    attr[cfg.numAttrs++].val.cooperative = 1;
-  } else if (nvfp4_pdl_enabled()) {
+  if (nvfp4_pdl_enabled(brief)) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
   }
@@ -54,9 +54,9 @@ static inline cudaError_t nvfp4_launch_grouped(void (*kernel)(KArgs...), unsigne
 }
 
 template <typename... KArgs, typename... Args>
-static inline cudaError_t nvfp4_launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+static inline cudaError_t nvfp4_launch_kernel(void (*kernel)(KArgs...), bool brief, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                               Args&&... args) {
-  return nvfp4_launch_grouped(kernel, 1, false, grid, block, smem, st, args...);
+  return nvfp4_launch_grouped(kernel, 1, brief, grid, block, smem, st, args...);
 }
 
 namespace nvfp4 {

@@ -1114,6 +1114,9 @@ static DevInfo* dev_info() {
   return &info[dev];
 }
 
+// about 40 us or less
+static bool brief_gemm(int M, int N, int K) { return (double)M * N * K <= 1e11; }
+
 template <int BN, int S = 1>
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sms, bool& attr_done,
                        cudaStream_t st) {
@@ -1125,7 +1128,7 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
   }
   const long long work = (long long)(p.M / kBM) * (p.N / BN) * p.splitk;
   const unsigned grid = (unsigned)(work < sms || S > 1 ? work : sms);
-  if (nvfp4_launch_grouped(gemm_nvf4_kernel<BN, S>, S, false, dim3(grid), dim3(kThreads), C::kSmemBytes, st, ma, mb, p) != cudaSuccess) {
+  if (nvfp4_launch_grouped(gemm_nvf4_kernel<BN, S>, S, brief_gemm(p.M, p.N, p.K), dim3(grid), dim3(kThreads), C::kSmemBytes, st, ma, mb, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return NVFP4_ERR_CUDA;
   }
@@ -1311,7 +1314,7 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
           return NVFP4_ERR_CUDA;                                                                                           \
         di->FLAG = true;                                                                                                   \
       }                                                                                                                    \
-      if (nvfp4_launch_kernel(gemm_nvf4_pair_kernel<BN_>, dim3(grid), dim3(kPairThreads), PairCfg<BN_>::kSmemBytes, st, ma, mb,\
+      if (nvfp4_launch_kernel(gemm_nvf4_pair_kernel<BN_>, brief_gemm(M, N, K), dim3(grid), dim3(kPairThreads), PairCfg<BN_>::kSmemBytes, st, ma, mb,\
                               msa, msb, pp) != cudaSuccess) {                                                               \
         (void)cudaGetLastError();                                                                                          \
         return NVFP4_ERR_CUDA;                                                                                             \

@@ -385,16 +385,20 @@ static int sm_count() {
 
 using namespace nvfp4;
 
-static int g_pdl = -1;      // -1: not decided yet (environment NVFP4_PDL=1 switches it on), else 0 / 1
-bool nvfp4_pdl_enabled() {
+// -1: not decided yet (environment variable NVFP4_PDL, else 2), else as nvfp4_set_pdl.  2: short launches only, us per
+// pass off -> on: forward [256, 5632, 2048] 20.5 -> 15.6, weight refresh of a block 77 -> 67, layer [4096, 2048, 3072]
+// 131 -> 125.  With every launch in it the long ones lose (weight gradient of 16384 tokens 204 -> 218): a staged grid
+// crowds onto the SMs that come free first.
+static int g_pdl = -1;
+bool nvfp4_pdl_enabled(bool brief) {
   if (g_pdl < 0) {
     const char* e = getenv("NVFP4_PDL");
-    g_pdl = (e && e[0] == '1') ? 1 : 0;
+    g_pdl = !e || !e[0] ? 2 : e[0] == '1' ? 1 : e[0] == '2' ? 2 : 0;
   }
-  return g_pdl != 0;
+  return g_pdl == 1 || (g_pdl == 2 && brief);
 }
 extern "C" int nvfp4_set_pdl(int on) {
-  g_pdl = on ? 1 : 0;
+  g_pdl = on == 2 ? 2 : on ? 1 : 0;
   return NVFP4_OK;
 }
 
@@ -485,7 +489,7 @@ static cudaError_t amax_start(const void* x, long long nv, float* out, float* ne
   long long blocks = (nv + 256 * 4 - 1) / (256 * 4);
   const long long cap = (long long)sm_count() * 4;
   if (blocks > cap) blocks = cap;
-  const cudaError_t rc = nvfp4_launch_kernel(amax_kernel<F32>, dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const uint4*>(x), nv, out, next, slot);
+  const cudaError_t rc = nvfp4_launch_kernel(amax_kernel<F32>, nvfp4_brief(nv * 16), dim3((unsigned)blocks), dim3(256), 0, st, static_cast<const uint4*>(x), nv, out, next, slot);
   if (rc != cudaSuccess) (void)cudaGetLastError();
   return rc;
 }
@@ -635,7 +639,7 @@ extern "C" int nvfp4_quant_w2d(const void* w, int w_dtype, int N, int K, void* q
   unsigned char *qp = static_cast<unsigned char*>(q), *sp = static_cast<unsigned char*>(s);
   unsigned char *qtp = static_cast<unsigned char*>(qt), *stp = static_cast<unsigned char*>(st_);
   cudaError_t rc;
-#define NVFP4_W2D(T) nvfp4_launch_kernel(quant_w2d_kernel<T>, grid, dim3(256), 0, stm, static_cast<const T*>(w), qp, sp, qtp, stp, amax, N, K, scale_layout, gs_out)
+#define NVFP4_W2D(T) nvfp4_launch_kernel(quant_w2d_kernel<T>, nvfp4_brief((long long)N * K * (long long)sizeof(T)), grid, dim3(256), 0, stm, static_cast<const T*>(w), qp, sp, qtp, stp, amax, N, K, scale_layout, gs_out)
   if (w_dtype == NVFP4_DTYPE_BF16) rc = NVFP4_W2D(__nv_bfloat16);
   else rc = NVFP4_W2D(float);
 #undef NVFP4_W2D

@@ -545,7 +545,7 @@ static int launch_tc(const CUtensorMap& map, const TcParams& p, int grid, cudaSt
       return NVFP4_ERR_CUDA;
     configured[dev] = true;
   }
-  if (nvfp4_launch_grouped(quant_tc_kernel<ROUNDING, ROWS, COLS, TCRHT, FIND>, FIND ? (unsigned)grid : 1u, false, dim3((unsigned)grid), dim3(kQThreads),
+  if (nvfp4_launch_grouped(quant_tc_kernel<ROUNDING, ROWS, COLS, TCRHT, FIND>, FIND ? (unsigned)grid : 1u, nvfp4_brief(2ll * p.M * p.C), dim3((unsigned)grid), dim3(kQThreads),
                            kQSmem, st, map, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return NVFP4_ERR_CUDA;

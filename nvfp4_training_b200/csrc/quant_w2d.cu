@@ -221,7 +221,7 @@ static int launch_w2d(const void* w, void* q, void* qt, const W2dParams& p, cuda
   }
   const long long ntiles = (long long)(p.N / kWRows) * (p.K / KT);
   const unsigned grid = (unsigned)(ntiles < 2 * sms[dev] ? ntiles : 2 * sms[dev]);
-  if (nvfp4_launch_kernel(quant_w2d_tile_kernel<T>, dim3(grid), dim3(256), kWSmem, st, mw, mq, mt, p) != cudaSuccess) {
+  if (nvfp4_launch_kernel(quant_w2d_tile_kernel<T>, nvfp4_brief((long long)p.N * p.K * (long long)sizeof(T)), dim3(grid), dim3(256), kWSmem, st, mw, mq, mt, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return NVFP4_ERR_CUDA;
   }
