@@ -84,3 +84,30 @@ def test_gemm_multiplies_with_the_scales_as_they_stand(write):
         assert torch.equal(fp4ops.gemm(q, b), want)
         if write is not _in_place:
             assert not want.any()
+
+
+def test_an_sw_can_be_given_in_inference_mode():
+    with torch.inference_mode():
+        s = torch.zeros(128, 8, dtype=torch.uint8)
+        q = fp4ops.Q(None, s, None, 1.0, s.flatten())
+        assert q.swizzled() is q.sw
+        _replace(q)
+        assert q.swizzled() is None
+
+
+@pytest.mark.gpu
+def test_inference_mode():
+    from nvfp4_training_b200 import fp4torch
+    x, w = torch.randn(128, 256, device="cuda").bfloat16(), torch.randn(256, 256, device="cuda") * 0.02
+
+    def run():
+        fw = fp4torch.FP4Weight(w)
+        fw.refresh()
+        a, c = fp4ops.quant_rows_cols_rht(x, 0xA6B1)
+        return [fp4torch.fp4_fwd(x, fw.wd, fw.ws, fw.amax), fp4torch.fp4_linear(x, w, fw.wd, fw.ws, fw.wtd, fw.wts, fw.amax),
+                fp4ops.gemm(a, fp4ops.quant_w2d(w)[0]), fp4ops.gemm(c, c, splitk=2),
+                fp4ops.gemm(fp4ops.quant_rows(x), fp4ops.quant_rows(w.bfloat16())), fp4ops.quant_cols_rht(x, 0xA6B1).s]
+    want = run()
+    with torch.inference_mode():
+        got = run()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
