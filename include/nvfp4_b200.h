@@ -149,8 +149,8 @@ int nvfp4_quant_cols_rht(const void* x, int M, int C, void* codes, void* scales,
  *     tensor memory, the quantizing warps read it with tcgen05.ld.  One documented difference: an input
  *     that is exactly -0 gives code 0x0 (the scalar kernels and the reference's convert give 0x8);
  *   - scalar (any other accepted shape): TMA tiles of 128 x 64 in a shared-memory ring, read by the
- *     quantizing warps.  NVFP4_SCALES_BOTH is written by the first kernel only.
- * Requires M % 128 == 0, C % 64 == 0 (C % 128 == 0 with SWIZZLED scales and codes_c), ldx % 8 == 0,
+ *     quantizing warps.  With NVFP4_SCALES_BOTH two launches of the re-swizzle kernel follow (scales 4-byte aligned).
+ * Requires M % 128 == 0, C % 64 == 0 (C % 128 == 0 with SWIZZLED or BOTH scales and codes_c), ldx % 8 == 0,
  * x and codes_c 16-byte aligned, codes_r and scales_c 8-byte aligned.  A wait that expires inside the kernel (1 s) is reported by nvfp4_quant_tile_status.
  */
 int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void* codes_r, void* scales_r, void* codes_c,

@@ -340,7 +340,7 @@ static int check_tile_args(const void* x, long long ldx, int M, int C, const voi
   if (scale_layout < NVFP4_SCALES_SWIZZLED || scale_layout > NVFP4_SCALES_BOTH) return NVFP4_ERR_ENUM;
   if (rounding < NVFP4_ROUND_NEAREST || rounding > NVFP4_ROUND_SR_HW) return NVFP4_ERR_ENUM;
   if (M < 0 || C < 0 || (M % kTileTok) || (C % kTileCol) || ldx < C) return NVFP4_ERR_SHAPE;
-  if (codes_c && scale_layout == NVFP4_SCALES_SWIZZLED && (C & 127)) return NVFP4_ERR_SHAPE;
+  if (codes_c && scale_layout != NVFP4_SCALES_LINEAR && (C & 127)) return NVFP4_ERR_SHAPE;
   if ((reinterpret_cast<uintptr_t>(x) & 15u) || (ldx & 7) || (reinterpret_cast<uintptr_t>(codes_r) & 7u) ||
       (reinterpret_cast<uintptr_t>(codes_c) & 15u) || (reinterpret_cast<uintptr_t>(scales_c) & 7u))
     return NVFP4_ERR_ALIGN;
@@ -371,7 +371,9 @@ extern "C" int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void
   if (bad != NVFP4_OK || M == 0 || C == 0) return bad;
   if (g_tile_path != 1 && nvfp4_quant_tc_accepts(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c))
     return nvfp4_quant_tc_launch(x, ldx, M, C, codes_r, scales_r, codes_c, scales_c, scale_layout, amax, nullptr, gs_r_out, gs_c_out, signs, rounding, seed_r, seed_c, seed_r_dev, seed_c_dev, stream);
-  if (scale_layout == NVFP4_SCALES_BOTH) return NVFP4_ERR_SHAPE;       // the scalar kernel writes one layout
+  // the scalar kernel writes one layout: the row-major bytes first, the swizzled ones from them
+  const bool both = scale_layout == NVFP4_SCALES_BOTH;
+  if (both && ((reinterpret_cast<uintptr_t>(scales_r) | reinterpret_cast<uintptr_t>(scales_c)) & 3u)) return NVFP4_ERR_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   CUtensorMap map;
   if (!make_tile_map(&map, x, M, C, ldx)) return NVFP4_ERR_CUDA;
@@ -379,7 +381,7 @@ extern "C" int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void
   p.codes_r = static_cast<uint2*>(codes_r); p.scales_r = static_cast<unsigned char*>(scales_r);
   p.codes_c = static_cast<unsigned char*>(codes_c); p.scales_c = static_cast<unsigned char*>(scales_c);
   p.amax = amax; p.gs_r_out = gs_r_out; p.gs_c_out = gs_c_out;
-  p.M = M; p.C = C; p.linear = scale_layout == NVFP4_SCALES_LINEAR;
+  p.M = M; p.C = C; p.linear = scale_layout != NVFP4_SCALES_SWIZZLED;
   p.signs = signs & 0xFFFFu;
   p.seed_r = seed_r; p.seed_c = seed_c; p.seed_r_dev = seed_r_dev; p.seed_c_dev = seed_c_dev;
   int dev = 0, sms = 148;
@@ -391,12 +393,17 @@ extern "C" int nvfp4_quant_tile(const void* x, long long ldx, int M, int C, void
   { const int b = nvfp4_sm_budget_value(); if (b > 0 && b < sms) sms = b; }   // SMs left to a collective running beside this kernel
   int grid = 2 * sms;
   if (ntiles < grid) grid = (int)ntiles;
+  int rc;
   switch (rounding) {
-    case NVFP4_ROUND_NEAREST: return launch_tile_mode<NVFP4_ROUND_NEAREST>(map, p, grid, st);
-    case NVFP4_ROUND_SR_DITHER: return launch_tile_mode<NVFP4_ROUND_SR_DITHER>(map, p, grid, st);
-    case NVFP4_ROUND_SR_DITHER_K: return launch_tile_mode<NVFP4_ROUND_SR_DITHER_K>(map, p, grid, st);
-    default: return launch_tile_mode<NVFP4_ROUND_SR_HW>(map, p, grid, st);
+    case NVFP4_ROUND_NEAREST: rc = launch_tile_mode<NVFP4_ROUND_NEAREST>(map, p, grid, st); break;
+    case NVFP4_ROUND_SR_DITHER: rc = launch_tile_mode<NVFP4_ROUND_SR_DITHER>(map, p, grid, st); break;
+    case NVFP4_ROUND_SR_DITHER_K: rc = launch_tile_mode<NVFP4_ROUND_SR_DITHER_K>(map, p, grid, st); break;
+    default: rc = launch_tile_mode<NVFP4_ROUND_SR_HW>(map, p, grid, st);
   }
+  const size_t n = (size_t)M * (size_t)(C >> 4);
+  if (rc == NVFP4_OK && both && codes_r) rc = nvfp4_swizzle_scales(scales_r, C >> 4, M, C >> 4, p.scales_r + n, stream);
+  if (rc == NVFP4_OK && both && codes_c) rc = nvfp4_swizzle_scales(scales_c, M >> 4, C, M >> 4, p.scales_c + n, stream);
+  return rc;
 }
 
 extern "C" int nvfp4_emit_cols(const void* x, long long ldx, int M, int C, void* codes, void* scales,

@@ -265,6 +265,20 @@ def test_tile_quantizer_matches_both_oracles(mods, tile_path, mode, M, C):
     assert nvq.quant_tile_status() == 0
 
 
+@pytest.mark.parametrize("M,C", [(128, 128), (256, 640), (128, 192)])
+def test_row_major_scales_from_both_tile_kernels(mods, tile_path, M, C):
+    """`fp4ops.quant_rows_cols_rht` on whichever kernel the path switch selects: row-major scales as the oracle has them
+    and, for whole 128 x 128 tiles, the same scales swizzled."""
+    _, fp4ops, _ = mods
+    x = make_dy(M * C, M, C)
+    r, c = O.quant_rows(x), O.quant_cols_rht(x, 0x9C3A)
+    for q, want in zip(fp4ops.quant_rows_cols_rht(to_dev(x), 0x9C3A), (r, c)):
+        sw = q.sw
+        assert np.array_equal(u8(q.d), want[0]) and np.array_equal(u8(q.s), want[1])
+        assert (sw is not None) == (C % 128 == 0)
+        assert sw is None or torch.equal(sw, fp4ops.swizzle_scales(q.s))
+
+
 def test_tile_quantizer_tensor_core_path_negative_zero_inputs(mods):
     """The tensor-core-fed kernel moves values through an MMA with a 0/1 matrix; an input that is exactly -0
     comes out as +0, so its code may be 0x0 where the convert instruction gives 0x8.  Everything else --
