@@ -415,9 +415,9 @@ void require_packed(const Tensor& d, int64_t R, int64_t C, const char* what) {
 py::tuple linear_fwd(const Tensor& x, const Tensor& wd, const Tensor& ws, const Tensor& wg, unsigned signs, const OptTensor& am_out) {
   require_cuda(x);
   at::NoGradGuard no_grad;
+  REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "linear_fwd: a bf16 matrix with contiguous rows");
   const int64_t T = x.size(0), K = x.size(1), N = wd.size(0);
   require_packed(wd, N, K, "linear_fwd: quantized weight");
-  REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16, "linear_fwd: a bf16 matrix");
   const Tensor am = am_out ? nvq_amax(x.contiguous(), am_out, false) : empty({1}, at::kFloat, x);
   PackedTensors xt(K, T, x);
   const PackedOut o = xt.out();

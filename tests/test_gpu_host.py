@@ -63,6 +63,20 @@ def test_host_errors_keep_their_types():
         nvq.mm(q, nvq.quant_rows(torch.ones(128, 128, dtype=torch.bfloat16, device="cuda")))
 
 
+def test_linear_fwd_wants_contiguous_rows():
+    from nvfp4_training_b200 import linear, nvq
+    base = torch.randn(128, 512, device="cuda").bfloat16()
+    qw = nvq.quant_w2d(torch.randn(256, 256, device="cuda").bfloat16())[0]
+    with pytest.raises(AssertionError):
+        linear.linear_fwd(base[:, ::2], qw, keep_xt=True)              # every other column
+    with pytest.raises(AssertionError):
+        linear.linear_fwd(base[:, :256].reshape(256, 128).t(), qw, keep_xt=True)
+    for x in (base[:, :256], base[:, 256:]):                           # rows with a stride
+        y, am, qxt = linear.linear_fwd(x, qw, keep_xt=True)
+        y2, am2, qxt2 = linear.linear_fwd(x.contiguous(), qw, keep_xt=True)
+        assert torch.equal(y, y2) and torch.equal(am, am2) and torch.equal(qxt.d.view(torch.uint8), qxt2.d.view(torch.uint8))
+
+
 @pytest.mark.parametrize("T,K,N", [(128, 128, 256), (1024, 2048, 640)])
 def test_calls_that_need_an_amax_can_be_captured(T, K, N):
     from nvfp4_training_b200 import fp4ops, nvq
