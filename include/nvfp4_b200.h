@@ -296,7 +296,8 @@ int nvfp4_swizzle_scales(const void* s_linear, long long lds, int R, int C16, vo
  *   pa, pb    device FP32 scalars used by alpha_mode (may be null for NVFP4_ALPHA_ONE); NVFP4_ALPHA_ROW: pa = FP32 [M]
  *   accumulate  0: C = result; 1: C += result (fp32 only, atomic adds)
  *   splitk    >= 1: the K range is cut into at most that many slices of whole 256-element tiles (as many as help), each
- *             added atomically into C; needs accumulate = 1 or C zeroed by the caller when > 1.
+ *             added atomically into C; needs accumulate = 1 or C zeroed by the caller when > 1.  (A K of one tile has
+ *             one slice: C is stored unless accumulate = 1.)
  *             0 (fp32 C only; bf16 C runs unsliced): the library picks the slice count from its tile cost model --
  *             weight-gradient shapes with few output tiles and a long K fill the SMs better in slices -- and, when it
  *             slices a call with accumulate = 0, zero-fills C itself first.  Slices add in no fixed order, so the

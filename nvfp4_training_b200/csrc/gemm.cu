@@ -1178,7 +1178,6 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   if ((accumulate || splitk > 1) && c_dtype != NVFP4_DTYPE_FP32) return NVFP4_ERR_ENUM;
   const bool auto_split = splitk == 0;      // the library picks the number of K slices (FP32 output only)
   if (auto_split) splitk = 1;
-  if (splitk > 1) accumulate = 1;           // slices asked for are added to C, however many there turn out to be
   if (!al16(a) || !al16(b) || !al16(sa) || !al16(sb) || !al16(c) || (lda & 15) || (ldb & 15) || (ldc & 7))
     return NVFP4_ERR_ALIGN;
   if (M == 0 || N == 0) return NVFP4_OK;
@@ -1237,6 +1236,7 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
     }
   }
   if (splitk > ktiles) splitk = ktiles;
+  if (splitk > 1) accumulate = 1;           // slices that K has room for are added to C, however many are taken below
   if (splitk > 1 && g_force_bn == 0 && !owners && !auto_split) {
     // The caller's number of slices is an upper bound.  A slice that adds no parallelism costs a pass of atomic adds over
     // C (3 TB/s) and the per-tile fixed cost once more: [3072, 1024] x K = 2048 in 8 slices took 32 us, in one 11 us.

@@ -56,3 +56,21 @@ def test_requested_slices_add_into_c(M, N, K, splitk):
     for got, want in ((out, y + 2), (fresh, y)):
         assert float((got.double() - want).norm() / want.norm()) <= 1e-5
     L.check_status()
+
+
+@pytest.mark.parametrize("K", [64, 256])
+def test_slices_of_a_single_k_tile_store(K):
+    """K of one tile has one slice whatever the caller asks for: without `accumulate` it is stored, not added."""
+    from nvfp4_training_b200 import _lib as L, nvq
+    a, b = nvq.quant_rows(to_dev(make_x(5, 256, K))), nvq.quant_rows(to_dev(make_w(6, 384, K)))
+    want = nvq.mm(a, b, out_dtype=torch.float32)
+    out = torch.full((256, 384), 7.0, device="cuda")
+    assert torch.equal(nvq.mm(a, b, out_dtype=torch.float32, out=out, splitk=4), want)
+    out.fill_(7.0)
+    nvq.mm(a, b, out_dtype=torch.float32, out=out, splitk=4, accumulate=True)
+    assert float((out - 7 - want).abs().max()) <= 2 ** -22 * float(want.abs().max() + 7)      # the sum and the difference round
+    # an empty contraction leaves zeros
+    out.fill_(7.0)
+    p = out.data_ptr()
+    assert L.load().nvfp4_gemm(p, p, 16, p, p, 16, p, L.DTYPE_FP32, 384, 256, 384, 0, L.ALPHA_ONE, None, None, 1.0, 1.0, 0, 4, None, L.stream()) == 0
+    assert not out.any()
