@@ -303,7 +303,8 @@ void nvq_quant_w2d_into(const Tensor& w_, const OptTensor& am_, const OptTensor&
   run_w2d(w, d ? &q : nullptr, dt ? &qt : nullptr, amax_or(am_, w, keep));
 }
 
-// A block-scaled GEMM into `out` (or a fresh tensor): alpha = product of the two words as `alpha_mode` says.
+// A block-scaled GEMM into `out` (or a fresh tensor): alpha = product of the two words as `alpha_mode` says.  Slices asked
+// for are added to `out`; a fresh tensor has nothing to add to, so there the library picks the slices and clears it first.
 Tensor gemm(const Tensor& ad, const Tensor& as, const Tensor& bd, const Tensor& bs, const OptTensor& out_, bool fp32, int alpha_mode,
             const OptTensor& pa, const OptTensor& pb, float ka, float kb, bool accumulate, int splitk, const char* what) {
   require_cuda(ad); require_cuda(bd);
@@ -321,7 +322,7 @@ Tensor gemm(const Tensor& ad, const Tensor& as, const Tensor& bd, const Tensor& 
   check(lib.nvfp4_gemm(ad.const_data_ptr(), as.const_data_ptr(), ad.stride(0), bd.const_data_ptr(), bs.const_data_ptr(), bd.stride(0),
                        out.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16, out.stride(0), (int)M, (int)N, (int)K, alpha_mode,
                        static_cast<const float*>(cptr(pa)), static_cast<const float*>(cptr(pb)), ka, kb, accumulate,
-                       fp32 ? splitk : 1, status_word(ad), stream()), what);
+                       !fp32 ? 1 : !out_ && splitk > 1 ? 0 : splitk, status_word(ad), stream()), what);
   return out;
 }
 

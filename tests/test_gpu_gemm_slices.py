@@ -74,3 +74,16 @@ def test_slices_of_a_single_k_tile_store(K):
     p = out.data_ptr()
     assert L.load().nvfp4_gemm(p, p, 16, p, p, 16, p, L.DTYPE_FP32, 384, 256, 384, 0, L.ALPHA_ONE, None, None, 1.0, 1.0, 0, 4, None, L.stream()) == 0
     assert not out.any()
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 128, 256), (256, 384, 4096), (2048, 1024, 8192)])
+def test_slices_of_a_fresh_result(M, N, K):
+    """`nvq.mm` without `out` gives the product, whatever the memory of its result held before."""
+    from nvfp4_training_b200 import nvq
+    a, b = nvq.quant_rows(to_dev(make_x(7, M, K))), nvq.quant_rows(to_dev(make_w(8, N, K)))
+    want = nvq.dequant(a).double() @ nvq.dequant(b).double().t()
+    for splitk in (1, 4):
+        junk = [torch.full((M, N), 1e6, device="cuda") for _ in range(4)]
+        del junk
+        got = nvq.mm(a, b, out_dtype=torch.float32, splitk=splitk)
+        assert float((got.double() - want).norm() / want.norm()) <= 1e-5
