@@ -752,7 +752,7 @@ Tensor k_gemm(const Tensor& ad, const Tensor& as, const OptTensor& asw, const Te
   const Tensor sa = asw ? *asw : k_swizzle(as, std::nullopt), sb = bsw ? *bsw : k_swizzle(bs, std::nullopt);
   check(lib.nvfp4_gemm(ad.const_data_ptr(), sa.const_data_ptr(), ad.stride(0), bd.const_data_ptr(), sb.const_data_ptr(), bd.stride(0),
                        out.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16, out.stride(0), (int)M, (int)N, (int)K,
-                       NVFP4_ALPHA_AMAX, word(aam), word(bam), ak, bk, fp32 && out_, fp32 && !out_ ? 0 : splitk, status_word(ad), stream()), "gemm");
+                       NVFP4_ALPHA_AMAX, word(aam), word(bam), ak, bk, fp32 && out_, fp32 && !out_ && splitk > 1 ? 0 : splitk, status_word(ad), stream()), "gemm");
   return out;
 }
 

@@ -260,3 +260,15 @@ def test_scatter_rows_rejects_bad_requests(mods):
     assert call([p] * 3) == 0                    # 256 rows each
     torch.cuda.synchronize()
     L.check_status()
+
+
+def test_a_negative_slice_count_is_refused(mods):
+    nvq, fp4ops, L = mods
+    x = to_dev(make_x(1, 128, 256))
+    a, q = fp4ops.quant_rows(x), nvq.quant_rows(x)
+    out = torch.zeros(128, 128, device="cuda")
+    for o in (None, out):
+        with pytest.raises(L.Nvfp4Error):
+            fp4ops.gemm(a, a, out=o, splitk=-3)
+        with pytest.raises(L.Nvfp4Error):
+            nvq.mm(q, q, out_dtype=torch.float32, out=o, splitk=-3)
