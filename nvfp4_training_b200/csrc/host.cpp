@@ -749,7 +749,11 @@ Tensor k_gemm(const Tensor& ad, const Tensor& as, const OptTensor& asw, const Te
     out = out_ ? *out_ : empty({M, N}, at::kFloat, ad);       // a fresh result is stored, the library slices K as it sees fit
     REQUIRE(out.scalar_type() == at::kFloat && out.stride(1) == 1, "gemm: out is FP32 with contiguous rows");
   }
-  const Tensor sa = asw ? *asw : k_swizzle(as, std::nullopt), sb = bsw ? *bsw : k_swizzle(bs, std::nullopt);
+  // scales of the operand's rows; more may be there (a slice of the codes with the scales of the whole)
+  auto swizzled = [](const Tensor& s, const OptTensor& sw, int64_t rows) {
+    return sw ? *sw : k_swizzle(s.size(0) == rows ? s : s.narrow(0, 0, rows), std::nullopt);
+  };
+  const Tensor sa = swizzled(as, asw, M), sb = swizzled(bs, bsw, N);
   check(lib.nvfp4_gemm(ad.const_data_ptr(), sa.const_data_ptr(), ad.stride(0), bd.const_data_ptr(), sb.const_data_ptr(), bd.stride(0),
                        out.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16, out.stride(0), (int)M, (int)N, (int)K,
                        NVFP4_ALPHA_AMAX, word(aam), word(bam), ak, bk, fp32 && out_, fp32 && !out_ && splitk > 1 ? 0 : splitk, status_word(ad), stream()), "gemm");

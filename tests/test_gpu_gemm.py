@@ -272,3 +272,14 @@ def test_a_negative_slice_count_is_refused(mods):
             fp4ops.gemm(a, a, out=o, splitk=-3)
         with pytest.raises(L.Nvfp4Error):
             nvq.mm(q, q, out_dtype=torch.float32, out=o, splitk=-3)
+
+
+def test_fp4ops_gemm_on_the_first_rows_of_an_operand(mods):
+    """Codes of 128 rows with the scale tensor of all 144 (no whole tiles) or 256: the rows' own scales count."""
+    _, fp4ops, _ = mods
+    b = fp4ops.quant_rows(to_dev(make_x(2, 256, 256)))
+    for R in (144, 256):
+        a = fp4ops.quant_rows(to_dev(make_x(1, R, 256)))
+        want = fp4ops.gemm(fp4ops.Q(a.d[:128].clone(), a.s[:128].clone(), a.amax), b)
+        assert torch.equal(fp4ops.gemm(fp4ops.Q(a.d[:128], a.s, a.amax), b), want)
+        assert torch.equal(fp4ops.gemm(b, fp4ops.Q(a.d[:128], a.s, a.amax)), want.t())
