@@ -823,7 +823,8 @@ void e_mom(const Tensor& m, const Tensor& g, const Tensor& alpha, float scale, c
 // raw = A B^T with block scales only (alpha_mode ONE), or times the words of `pa`, `pb`
 Tensor e_mm(const Tensor& ad, const Tensor& as, const Tensor& bd, const Tensor& bs, bool fp32, int alpha_mode, const OptTensor& pa,
             const OptTensor& pb, const OptTensor& out, bool accumulate, int splitk) {
-  return gemm(ad, as, bd, bs, out, fp32, alpha_mode, pa, pb, 1.f, 1.f, accumulate, splitk, "gemm");
+  auto bytes = [](const Tensor& t) { return t.element_size() == 1 ? t : t.view(at::kByte); };     // codes in wider words
+  return gemm(bytes(ad), as, bytes(bd), bs, out, fp32, alpha_mode, pa, pb, 1.f, 1.f, accumulate, splitk, "gemm");
 }
 
 void bind(const py::dict& addresses, py::object error, py::object lin, py::object nvq, py::object status) {

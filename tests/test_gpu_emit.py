@@ -322,3 +322,13 @@ def test_row_emit_hardware_sr_warp_per_row_and_long_rows():
     q = emit.row_emit(to_dev(g), emit.RowQ(128, 49152), rng, sr="hw", salt=9)
     _check(q, O.emit_rows(g, seed=41, sr="hw", salt=9), 128, 49152)
     _lib.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.float4_e2m1fn_x2, torch.int16, torch.int32])
+def test_mm_takes_codes_of_any_width(dtype):
+    """The operands are bytes; a tensor that holds them in wider words is the same operand."""
+    from nvfp4_training_b200 import emit, nvq
+    a, b = (nvq.quant_rows(torch.randn(r, 256, device="cuda").bfloat16()) for r in (128, 256))
+    want = emit.mm(a.d, a.s, b.d, b.s)
+    codes = [q.d.view(torch.uint8).view(dtype) for q in (a, b)]
+    assert torch.equal(emit.mm(codes[0], a.s, codes[1], b.s), want)
