@@ -115,13 +115,14 @@ struct Carver {
   }
 };
 
-// A packed matrix [R, C]: codes, swizzled scales, tensor scale.
+// A packed matrix [R, C]: codes, bytes from row to row of them, swizzled scales, tensor scale.
 struct Packed {
-  const void* d; const void* s; const float* gs;
+  const void* d; int64_t ld; const void* s; const float* gs;
 };
+// One of whole rows, as the quantizers write it.
 struct PackedOut {
   void* d; void* s; float* gs;
-  operator Packed() const { return {d, s, gs}; }
+  Packed in(int64_t C) const { return {d, C / 2, s, gs}; }
 };
 PackedOut carve_packed(Carver& c, int64_t R, int64_t C) {
   void* d = c.take(R * C / 2);
@@ -177,10 +178,10 @@ void run_w2d(const Tensor& w, const PackedOut* q, const PackedOut* qt, const flo
                             (q ? q : qt)->gs, stream()), "quant_w2d");
 }
 
-// contiguous packed operands a [M, K], b [N, K] -> c [M, N]
+// packed operands a [M, K], b [N, K] -> c [M, N]
 void run_mm(const Packed& a, const Packed& b, const Tensor& c, int64_t K, bool accumulate, int splitk) {
   const bool fp32 = c.scalar_type() == at::kFloat;
-  check(lib.nvfp4_gemm(a.d, a.s, K / 2, b.d, b.s, K / 2, c.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16,
+  check(lib.nvfp4_gemm(a.d, a.s, a.ld, b.d, b.s, b.ld, c.data_ptr(), fp32 ? NVFP4_DTYPE_FP32 : NVFP4_DTYPE_BF16,
                        c.stride(0), (int)c.size(0), (int)c.size(1), (int)K, NVFP4_ALPHA_GS, a.gs, b.gs, 1.f, 1.f, accumulate,
                        fp32 ? splitk : 1, status_word(c), stream()), "mm");
 }
@@ -353,12 +354,12 @@ Tensor forward_core(const Tensor& x, const float* am, float* am_out, const Packe
     run_tile(x, &qx, xt, am, signs, NVFP4_ROUND_NEAREST, Seed(), Seed());
   }
   Tensor y = empty({T, N}, at::kBFloat16, x);
-  run_mm(qx, w, y, K, false, 1);
+  run_mm(qx.in(K), w, y, K, false, 1);
   return y;
 }
 
 struct BackwardArgs {
-  int64_t K;                       // in-features
+  int64_t K, Kw;                   // columns of gx and of gW: in-features
   unsigned signs;
   int mode;
   bool want_x = true, want_w = true;
@@ -395,22 +396,20 @@ std::pair<Tensor, Tensor> backward_core(const Tensor& gy, const Packed& wt, cons
   }
   if (a.want_x) {
     gx = empty({T, a.K}, at::kBFloat16, gy);
-    run_mm(qg, wt, gx, N, false, 1);
+    run_mm(qg.in(N), wt, gx, N, false, 1);
   }
   if (a.want_w) {
-    gw = a.gw_out ? *a.gw_out : empty({N, a.K}, a.gw_dtype, gy);
-    run_mm(qgt, xt, gw, T, a.gw_out && !a.overwrite, a.gw_out ? 0 : 1);
+    gw = a.gw_out ? *a.gw_out : empty({N, a.Kw}, a.gw_dtype, gy);
+    run_mm(qgt.in(T), xt, gw, T, a.gw_out && !a.overwrite, a.gw_out ? 0 : 1);
   }
   return {gx, gw};
 }
 
-Packed packed_of(const Tensor& d, const Tensor& s, const Tensor& gs) {
-  return {d.const_data_ptr(), s.const_data_ptr(), word(gs)};
-}
-// whole [R, C/2] code matrices only: the layer addresses them by their sizes
-void require_packed(const Tensor& d, int64_t R, int64_t C, const char* what) {
+// a code matrix [R, C/2] (its rows may have a stride) with its scales; R < 0: any number of rows
+Packed packed_of(const Tensor& d, const Tensor& s, const Tensor& gs, int64_t R, int64_t C, const char* what) {
   require_cuda(d);
-  REQUIRE(d.dim() == 2 && d.size(0) == R && d.size(1) * 2 == C && d.is_contiguous(), what);
+  REQUIRE(d.dim() == 2 && (R < 0 || d.size(0) == R) && d.size(1) * 2 == C && d.stride(1) == 1, what);
+  return {d.const_data_ptr(), d.stride(0), s.const_data_ptr(), word(gs)};
 }
 
 py::tuple linear_fwd(const Tensor& x, const Tensor& wd, const Tensor& ws, const Tensor& wg, unsigned signs, const OptTensor& am_out) {
@@ -418,11 +417,11 @@ py::tuple linear_fwd(const Tensor& x, const Tensor& wd, const Tensor& ws, const 
   at::NoGradGuard no_grad;
   REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "linear_fwd: a bf16 matrix with contiguous rows");
   const int64_t T = x.size(0), K = x.size(1), N = wd.size(0);
-  require_packed(wd, N, K, "linear_fwd: quantized weight");
+  const Packed w = packed_of(wd, ws, wg, N, K, "linear_fwd: quantized weight");
   const Tensor am = am_out ? nvq_amax(x.contiguous(), am_out, false) : empty({1}, at::kFloat, x);
   PackedTensors xt(K, T, x);
   const PackedOut o = xt.out();
-  Tensor y = forward_core(x, am_out ? word(am) : nullptr, am_out ? nullptr : am.data_ptr<float>(), packed_of(wd, ws, wg), N, &o, signs);
+  Tensor y = forward_core(x, am_out ? word(am) : nullptr, am_out ? nullptr : am.data_ptr<float>(), w, N, &o, signs);
   return py::make_tuple(y, am, xt.d, xt.s, xt.gs);
 }
 
@@ -435,16 +434,17 @@ py::tuple linear_bwd(const Tensor& gy_, const Tensor& wd, const Tensor& ws, cons
   REQUIRE(gy.dim() == 2 && gy.scalar_type() == at::kBFloat16, "linear_bwd: bf16 output gradient");
   BackwardArgs a;
   a.K = wd.size(0);
-  require_packed(wd, a.K, gy.size(1), "linear_bwd: quantized transposed weight");
-  require_packed(xd, a.K, gy.size(0), "linear_bwd: transposed operand of x");
+  a.Kw = xd.size(0);
+  const Packed wt = packed_of(wd, ws, wg, -1, gy.size(1), "linear_bwd: quantized transposed weight");
+  const Packed xt = packed_of(xd, xs, xg, -1, gy.size(0), "linear_bwd: transposed operand of x");
   a.signs = signs; a.mode = mode; a.gw_out = gw_out; a.overwrite = overwrite; a.am = am; a.am_out = am_out;
   a.gw_dtype = gw_fp32 ? at::kFloat : at::kBFloat16;
   if (gw_out) {
     require_cuda(gw_out);
-    REQUIRE(gw_out->dim() == 2 && gw_out->size(0) == gy.size(1) && gw_out->size(1) == a.K && gw_out->scalar_type() == at::kFloat &&
+    REQUIRE(gw_out->dim() == 2 && gw_out->size(0) == gy.size(1) && gw_out->size(1) == a.Kw && gw_out->scalar_type() == at::kFloat &&
                 gw_out->stride(1) == 1, "linear_bwd: gw_out is fp32 [N, K]");
   }
-  auto [gx, gw] = backward_core(gy, packed_of(wd, ws, wg), packed_of(xd, xs, xg), Seed(seed), Seed(seed_cols), a);
+  auto [gx, gw] = backward_core(gy, wt, xt, Seed(seed), Seed(seed_cols), a);
   return py::make_tuple(gx, gw);
 }
 
@@ -485,7 +485,7 @@ struct LinearNode : torch::autograd::Node {
     w.unpack(getptr());                         // raises when the graph was freed or the weight changed in place
     const Tensor buf = kept.unpack(getptr());
     BackwardArgs a;
-    a.K = K; a.signs = signs;
+    a.K = a.Kw = K; a.signs = signs;
     a.want_x = task_should_compute_output(0);
     a.want_w = task_should_compute_output(1);
     if (!a.want_x && !a.want_w) return out;
@@ -505,13 +505,9 @@ struct LinearNode : torch::autograd::Node {
     REQUIRE(a.gw_dtype == at::kFloat || a.gw_dtype == at::kBFloat16, "LinCtx.wgrad_dtype: float32 or bfloat16");
     Carver c{static_cast<char*>(buf.data_ptr())};
     const Kept k(c, T, K, N, keep_x, keep_w);
-    Packed wt = k.wt;
-    if (cached.d.defined()) {
-      require_packed(cached.d, K, N, "cached transposed weight");
-      wt = packed_of(cached.d, cached.s, cached.gs);
-    }
+    const Packed wt = cached.d.defined() ? packed_of(cached.d, cached.s, cached.gs, K, N, "cached transposed weight") : k.wt.in(N);
     const Tensor gy = grads[0].contiguous();
-    std::tie(out[0], out[1]) = backward_core(gy, wt, k.xt, Seed(seed), Seed(seed ^ 0x5bd1e995u), a);
+    std::tie(out[0], out[1]) = backward_core(gy, wt, k.xt.in(T), Seed(seed), Seed(seed ^ 0x5bd1e995u), a);
     return out;
   }
 };
@@ -545,8 +541,7 @@ Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py
     if (cached) {
       cq = q_of(cache.attr("q"));
       N = cq.d.size(0);
-      require_packed(cq.d, N, K, "cached weight");
-      qw = packed_of(cq.d, cq.s, cq.gs);
+      qw = packed_of(cq.d, cq.s, cq.gs, N, K, "cached weight");
     } else {
       REQUIRE(w_.defined(), "linear: no weight");
       require_cuda(w_);
@@ -577,7 +572,7 @@ Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py
       const float* amw = passing_amax(w, carve(c));
       if (keep_w) wq.gs = kept.wt.gs;         // both orientations share one tensor scale, which the backward pass reads
       run_w2d(w, &wq, keep_w ? &kept.wt : nullptr, amw);
-      qw = wq;
+      qw = wq.in(K);
     }
     y = forward_core(x, nullptr, nullptr, qw, N, need_w ? &kept.xt : nullptr, signs);
   }

@@ -77,6 +77,28 @@ def test_linear_fwd_wants_contiguous_rows():
         assert torch.equal(y, y2) and torch.equal(am, am2) and torch.equal(qxt.d.view(torch.uint8), qxt2.d.view(torch.uint8))
 
 
+def test_packed_operands_may_have_a_row_stride():
+    """Codes with padding between their rows: the same results from the pair and from a layer whose cache holds them."""
+    from nvfp4_training_b200 import linear, nvq
+
+    def padded(q):
+        wide = torch.full((q.d.shape[0], q.d.shape[1] + 32), 0x77, dtype=torch.uint8, device="cuda")
+        wide[:, :q.d.shape[1]] = q.d.view(torch.uint8)
+        return nvq.Q(wide[:, :q.d.shape[1]].view(q.d.dtype), q.s, q.gs)
+    lin, x, gy = _layer(384, 256, 640, True)
+    qw, qwt = lin.cache.q, lin.cache.qt
+    y, am, qxt = linear.linear_fwd(x, qw, keep_xt=True)
+    gx, gw = linear.linear_bwd(None, am, gy, qwt, 1, 2, qxt=qxt)
+    y2, am2, _ = linear.linear_fwd(x, padded(qw), keep_xt=True)
+    gx2, gw2 = linear.linear_bwd(None, am2, gy, padded(qwt), 1, 2, qxt=padded(qxt))
+    assert torch.equal(y, y2) and torch.equal(gx, gx2) and torch.equal(gw, gw2)
+    xg = x.clone().requires_grad_(True)
+    want = torch.autograd.grad(lin(xg), (xg, lin.weight), gy)
+    lin.cache.q, lin.cache.qt = padded(qw), padded(qwt)
+    got = torch.autograd.grad(lin(xg), (xg, lin.weight), gy)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("T,K,N", [(128, 128, 256), (1024, 2048, 640)])
 def test_calls_that_need_an_amax_can_be_captured(T, K, N):
     from nvfp4_training_b200 import fp4ops, nvq
