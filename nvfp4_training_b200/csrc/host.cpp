@@ -121,7 +121,7 @@ struct Packed {
 };
 // One of whole rows, as the quantizers write it.
 struct PackedOut {
-  void* d; void* s; float* gs;
+  void* d = nullptr; void* s = nullptr; float* gs = nullptr;
   Packed in(int64_t C) const { return {d, C / 2, s, gs}; }
 };
 PackedOut carve_packed(Carver& c, int64_t R, int64_t C) {

@@ -83,6 +83,7 @@ def linear_bwd(x, am_x, gy, qwt, seed, seed_cols, gw_out=None, wgrad_dtype=torch
     rank; the product is added into the row slab each rank owns (`nvq.mm(owners=)`; `overwrite` is then ignored: the
     caller clears the slabs once per step)."""
     if qxt is not None and gw_owners is None and (gw_out is None or wgrad_stream is None) and _tileable(gy):
+        assert gw_out is not None or wgrad_dtype in (torch.bfloat16, torch.float32)
         return (L._host or L.host()).linear_bwd(gy, qwt.d, qwt.s, qwt.gs, qxt.d, qxt.s, qxt.gs, seed, seed_cols, signs & 0xFFFF,
                                                 sr_mode or nvq.SR_MODE, gw_out, overwrite, wgrad_dtype == torch.float32, am_gy, am_out)
     gy = gy.contiguous()

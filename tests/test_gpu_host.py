@@ -77,6 +77,20 @@ def test_linear_fwd_wants_contiguous_rows():
         assert torch.equal(y, y2) and torch.equal(am, am2) and torch.equal(qxt.d.view(torch.uint8), qxt2.d.view(torch.uint8))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.int32, None, "float32"])
+def test_linear_bwd_refuses_other_gradient_types(dtype):
+    from nvfp4_training_b200 import linear, nvq
+    x, gy = (torch.randn(128, 128, device="cuda").bfloat16() for _ in range(2))
+    qw, qwt = nvq.quant_w2d(x)
+    _, am, qxt = linear.linear_fwd(x, qw, keep_xt=True)
+    with pytest.raises(AssertionError):
+        linear.linear_bwd(None, am, gy, qwt, 1, 2, qxt=qxt, wgrad_dtype=dtype)
+    gw = torch.zeros(128, 128, device="cuda")                          # `gw_out` decides the type where it is given
+    assert linear.linear_bwd(None, am, gy, qwt, 1, 2, qxt=qxt, wgrad_dtype=dtype, gw_out=gw)[1] is gw
+    for ok in (torch.float32, torch.bfloat16):
+        assert linear.linear_bwd(None, am, gy, qwt, 1, 2, qxt=qxt, wgrad_dtype=ok)[1].dtype == ok
+
+
 def test_packed_operands_may_have_a_row_stride():
     """Codes with padding between their rows: the same results from the pair and from a layer whose cache holds them."""
     from nvfp4_training_b200 import linear, nvq
