@@ -16,6 +16,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <pybind11/pybind11.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -478,7 +479,34 @@ struct LinearNode : torch::autograd::Node {
   std::string name() const override { return "FP4LinearBackward"; }
   void release_variables() override { w.reset_data(); kept.reset_data(); }
 
+  // Exceptions leave through the autograd engine, not through this module: as Python errors of their types
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    try {
+      return backward(std::move(grads));
+    } catch (const AssertionFailure& e) {
+      throw_as(PyExc_AssertionError, e.what());
+    } catch (const LibraryError& e) {
+      throw_as(error_class.ptr(), e.what());
+    } catch (py::error_already_set& e) {
+      py::gil_scoped_acquire gil;
+      e.restore();
+      throw_python_error_set();
+    }
+  }
+
+ private:
+  [[noreturn]] static void throw_python_error_set() {
+    python_error error;
+    error.persist();
+    throw std::move(error);
+  }
+  [[noreturn]] static void throw_as(PyObject* type, const char* what) {
+    py::gil_scoped_acquire gil;
+    PyErr_SetString(type, what);
+    throw_python_error_set();
+  }
+
+  torch::autograd::variable_list backward(torch::autograd::variable_list&& grads) {
     torch::autograd::variable_list out(2);
     if (!grads[0].defined()) return out;
     at::NoGradGuard no_grad;

@@ -77,6 +77,22 @@ def test_linear_fwd_wants_contiguous_rows():
         assert torch.equal(y, y2) and torch.equal(am, am2) and torch.equal(qxt.d.view(torch.uint8), qxt2.d.view(torch.uint8))
 
 
+def test_errors_in_the_backward_pass_keep_their_types(monkeypatch):
+    from nvfp4_training_b200 import _lib
+    from nvfp4_training_b200.linear import LinCtx
+    lin, x, gy = _layer(128, 128, 256, False)
+    xg = x.clone().requires_grad_(True)
+    off = torch.zeros(128 * 256 + 8, dtype=torch.bfloat16, device="cuda")[4:-4].view(128, 256)     # off its 16-byte boundary
+    for cuda_grad, name, value, error in ((off, "seed", 1, _lib.Nvfp4Error), (gy, "wgrad_dtype", torch.float16, AssertionError),
+                                          (gy, "seed", "one", TypeError)):
+        with monkeypatch.context() as m:
+            m.setattr(LinCtx, name, value)
+            with pytest.raises(error) as caught:
+                torch.autograd.grad(lin(xg), (xg, lin.weight), cuda_grad)
+            assert caught.type is error
+    torch.autograd.grad(lin(xg), (xg, lin.weight), gy)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.int32, None, "float32"])
 def test_linear_bwd_refuses_other_gradient_types(dtype):
     from nvfp4_training_b200 import linear, nvq
