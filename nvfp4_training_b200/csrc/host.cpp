@@ -526,7 +526,7 @@ struct LinearNode : torch::autograd::Node {
       seed = (unsigned)PyLong_AsUnsignedLongLongMask(s.ptr()) * 1000003u + lid * 7919u;
       if (PyErr_Occurred()) throw py::error_already_set();
       const py::object dtype = lin_ctx.attr("wgrad_dtype");
-      a.gw_dtype = reinterpret_cast<THPDtype*>(dtype.ptr())->scalar_type;
+      a.gw_dtype = THPDtype_Check(dtype.ptr()) ? reinterpret_cast<THPDtype*>(dtype.ptr())->scalar_type : at::kByte;
       a.mode = py::cast<int>(nvq_module.attr("SR_MODE"));
       if (cache && a.want_x) cached = q_of(py::handle(cache).attr("qt"));
     }

@@ -84,6 +84,7 @@ def test_errors_in_the_backward_pass_keep_their_types(monkeypatch):
     xg = x.clone().requires_grad_(True)
     off = torch.zeros(128 * 256 + 8, dtype=torch.bfloat16, device="cuda")[4:-4].view(128, 256)     # off its 16-byte boundary
     for cuda_grad, name, value, error in ((off, "seed", 1, _lib.Nvfp4Error), (gy, "wgrad_dtype", torch.float16, AssertionError),
+                                          (gy, "wgrad_dtype", None, AssertionError), (gy, "wgrad_dtype", "float32", AssertionError),
                                           (gy, "seed", "one", TypeError)):
         with monkeypatch.context() as m:
             m.setattr(LinCtx, name, value)
