@@ -24,7 +24,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
-#include <mutex>
+#include <atomic>
 
 #include "../../include/nvfp4_b200.h"
 
@@ -72,7 +72,8 @@ Tensor empty(at::IntArrayRef size, at::ScalarType dtype, const Tensor& like) {
 }
 const void* cptr(const OptTensor& t) { return t ? t->const_data_ptr() : nullptr; }
 
-// Host seed or a device word: a CUDA int32 / uint32 tensor selects the device-side seed.
+// Host seed or a device word: a CUDA int32 / uint32 tensor selects the device-side seed.  (Constructed from a Python
+// object with the interpreter lock held, by the caster at the end of this file.)
 struct Seed {
   unsigned host = 0;
   const unsigned* dev = nullptr;
@@ -94,14 +95,16 @@ struct Seed {
 // Per-device status word of the GEMM, created and owned by the Python binding.
 int* status_word(const Tensor& like) {
   constexpr int kDevices = 64;
-  static int* words[kDevices] = {};
+  static std::atomic<int*> words[kDevices];
   const int dev = like.get_device();
   TORCH_CHECK(dev >= 0 && dev < kDevices);
-  if (!words[dev]) {
+  int* p = words[dev].load(std::memory_order_relaxed);
+  if (!p) {
     py::gil_scoped_acquire gil;
-    words[dev] = static_cast<int*>(py::cast<Tensor>(status_word_fn(like.device())).data_ptr());
+    p = static_cast<int*>(py::cast<Tensor>(status_word_fn(like.device())).data_ptr());
+    words[dev].store(p, std::memory_order_relaxed);
   }
-  return words[dev];
+  return p;
 }
 
 // Carves sub-buffers, each at a multiple of 256 bytes, out of one allocation; in a dry run it only adds up sizes.
@@ -131,6 +134,9 @@ PackedOut carve_packed(Carver& c, int64_t R, int64_t C) {
   return {d, s, c.take<float>(4)};
 }
 
+using Packed3 = std::tuple<Tensor, Tensor, Tensor>;          // the `d`, `s`, `gs` of a Q
+using OptPacked3 = std::optional<Packed3>;
+
 // Fresh output tensors of a packed matrix (the `d`, `s`, `gs` of a Q).
 struct PackedTensors {
   Tensor d, s, gs;
@@ -138,7 +144,7 @@ struct PackedTensors {
       : d(empty({R, C / 2}, at::kFloat4_e2m1fn_x2, like)), s(empty({R * C / 16}, at::kFloat8_e4m3fn, like)),
         gs(empty({1}, at::kFloat, like)) {}
   PackedOut out() const { return {d.data_ptr(), s.data_ptr(), gs.data_ptr<float>()}; }
-  py::tuple tuple() const { return py::make_tuple(d, s, gs); }
+  Packed3 tuple() const { return {d, s, gs}; }
 };
 
 // ------------------------------------------------------------------------------------------ launches
@@ -212,12 +218,11 @@ const float* amax_or(const OptTensor& am, const Tensor& x, Tensor& keep) {
   return word(keep);
 }
 
-py::tuple nvq_quant_rows(const Tensor& x, int mode, py::handle seed_, const OptTensor& am_) {
+Packed3 nvq_quant_rows(const Tensor& x, int mode, const Seed& seed, const OptTensor& am_) {
   require_cuda(x);
   REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16, "quant_rows: a bf16 matrix");
   const int64_t R = x.size(0), C = x.size(1);
   REQUIRE(x.stride(1) == 1 && C % 64 == 0 && R % 128 == 0, shape_of(R, C));
-  const Seed seed(seed_);
   PackedTensors q(R, C, x);
   const PackedOut o = q.out();
   Tensor keep;
@@ -227,14 +232,13 @@ py::tuple nvq_quant_rows(const Tensor& x, int mode, py::handle seed_, const OptT
   return q.tuple();
 }
 
-py::tuple nvq_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, py::handle seed_, const OptTensor& am_) {
+Packed3 nvq_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, const Seed& seed, const OptTensor& am_) {
   require_cuda(x_);
   REQUIRE(x_.dim() == 2 && x_.scalar_type() == at::kBFloat16, "quant_cols_rht: a bf16 matrix");
   at::NoGradGuard no_grad;
   const Tensor x = x_.contiguous();
   const int64_t M = x.size(0), C = x.size(1);
   REQUIRE(M % 64 == 0 && C % 128 == 0, shape_of(M, C));
-  const Seed seed(seed_);
   PackedTensors q(C, M, x);
   const PackedOut o = q.out();
   if (!am_ && M % 128 == 0 && run_tile_amax(x, nullptr, &o, nullptr, signs, mode, Seed(), seed)) return q.tuple();
@@ -247,13 +251,12 @@ py::tuple nvq_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, py::han
   return q.tuple();
 }
 
-py::tuple nvq_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py::handle seed_, py::handle seed_cols_,
-                                  const OptTensor& am_, bool want_rows, bool want_cols) {
+std::pair<OptPacked3, OptPacked3> nvq_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, const Seed& seed, const Seed& seed_cols,
+                                                          const OptTensor& am_, bool want_rows, bool want_cols) {
   require_cuda(x);
   REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "quant_rows_cols_rht: a bf16 matrix with contiguous rows");
   const int64_t M = x.size(0), C = x.size(1);
   REQUIRE(M % 128 == 0 && C % 128 == 0, shape_of(M, C));
-  const Seed seed(seed_), seed_cols(seed_cols_);
   std::optional<PackedTensors> qr, qc;
   PackedOut r, c;
   if (want_rows) { qr.emplace(M, C, x); r = qr->out(); }
@@ -263,11 +266,11 @@ py::tuple nvq_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py:
     const float* am = amax_or(am_, x, keep);
     run_tile(x, want_rows ? &r : nullptr, want_cols ? &c : nullptr, am, signs, mode, seed, seed_cols);
   }
-  return py::make_tuple(qr ? py::object(qr->tuple()) : py::none(), qc ? py::object(qc->tuple()) : py::none());
+  return {qr ? OptPacked3(qr->tuple()) : std::nullopt, qc ? OptPacked3(qc->tuple()) : std::nullopt};
 }
 
 // Fresh outputs, the two operands sharing one tensor scale; a skipped operand is None.
-py::tuple nvq_quant_w2d(const Tensor& w_, const OptTensor& am_, bool want, bool want_t) {
+std::pair<OptPacked3, OptPacked3> nvq_quant_w2d(const Tensor& w_, const OptTensor& am_, bool want, bool want_t) {
   require_cuda(w_);
   REQUIRE(w_.dim() == 2 && w_.scalar_type() == at::kBFloat16, "quant_w2d: a bf16 matrix");
   at::NoGradGuard no_grad;
@@ -286,8 +289,7 @@ py::tuple nvq_quant_w2d(const Tensor& w_, const OptTensor& am_, bool want, bool 
   if (want_t) qt = alloc(K, N, dt, st);
   Tensor keep;
   run_w2d(w, want ? &q : nullptr, want_t ? &qt : nullptr, amax_or(am_, w, keep));
-  return py::make_tuple(want ? py::object(py::make_tuple(d, s, gs)) : py::none(),
-                        want_t ? py::object(py::make_tuple(dt, st, gs)) : py::none());
+  return {want ? OptPacked3({d, s, gs}) : std::nullopt, want_t ? OptPacked3({dt, st, gs}) : std::nullopt};
 }
 
 // In place into an earlier call's buffers.
@@ -413,7 +415,7 @@ Packed packed_of(const Tensor& d, const Tensor& s, const Tensor& gs, int64_t R, 
   return {d.const_data_ptr(), d.stride(0), s.const_data_ptr(), word(gs)};
 }
 
-py::tuple linear_fwd(const Tensor& x, const Tensor& wd, const Tensor& ws, const Tensor& wg, unsigned signs, const OptTensor& am_out) {
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> linear_fwd(const Tensor& x, const Tensor& wd, const Tensor& ws, const Tensor& wg, unsigned signs, const OptTensor& am_out) {
   require_cuda(x);
   at::NoGradGuard no_grad;
   REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "linear_fwd: a bf16 matrix with contiguous rows");
@@ -423,12 +425,12 @@ py::tuple linear_fwd(const Tensor& x, const Tensor& wd, const Tensor& ws, const 
   PackedTensors xt(K, T, x);
   const PackedOut o = xt.out();
   Tensor y = forward_core(x, am_out ? word(am) : nullptr, am_out ? nullptr : am.data_ptr<float>(), w, N, &o, signs);
-  return py::make_tuple(y, am, xt.d, xt.s, xt.gs);
+  return {y, am, xt.d, xt.s, xt.gs};
 }
 
-py::tuple linear_bwd(const Tensor& gy_, const Tensor& wd, const Tensor& ws, const Tensor& wg, const Tensor& xd, const Tensor& xs,
-                     const Tensor& xg, py::handle seed, py::handle seed_cols, unsigned signs, int mode, const OptTensor& gw_out,
-                     bool overwrite, bool gw_fp32, const OptTensor& am, const OptTensor& am_out) {
+std::pair<Tensor, Tensor> linear_bwd(const Tensor& gy_, const Tensor& wd, const Tensor& ws, const Tensor& wg, const Tensor& xd,
+                                     const Tensor& xs, const Tensor& xg, const Seed& seed, const Seed& seed_cols, unsigned signs, int mode,
+                                     const OptTensor& gw_out, bool overwrite, bool gw_fp32, const OptTensor& am, const OptTensor& am_out) {
   require_cuda(gy_); require_cuda(am_out);
   at::NoGradGuard no_grad;
   const Tensor gy = gy_.contiguous();
@@ -445,8 +447,7 @@ py::tuple linear_bwd(const Tensor& gy_, const Tensor& wd, const Tensor& ws, cons
     REQUIRE(gw_out->dim() == 2 && gw_out->size(0) == gy.size(1) && gw_out->size(1) == a.Kw && gw_out->scalar_type() == at::kFloat &&
                 gw_out->stride(1) == 1, "linear_bwd: gw_out is fp32 [N, K]");
   }
-  auto [gx, gw] = backward_core(gy, wt, xt, Seed(seed), Seed(seed_cols), a);
-  return py::make_tuple(gx, gw);
+  return backward_core(gy, wt, xt, seed, seed_cols, a);
 }
 
 // Offsets inside the one buffer a forward pass keeps for its backward pass.
@@ -556,18 +557,21 @@ Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py
   REQUIRE(x_.dim() == 2 && x_.scalar_type() == at::kBFloat16 && x_.stride(1) == 1, "linear: x is bf16 [T, K] with contiguous rows");
   const int64_t T = x_.size(0), K = x_.size(1);
   REQUIRE(T % 128 == 0 && K % 128 == 0, shape_of(T, K));
+  const unsigned layer = (unsigned)PyLong_AsUnsignedLongLongMask(lid.ptr());
+  if (PyErr_Occurred()) throw py::error_already_set();
+  Q3 cq;
+  if (cached) cq = q_of(cache.attr("q"));
   Tensor y;
   std::shared_ptr<LinearNode> node;
   Tensor kept_buf;
   int64_t N;
   {
+    py::gil_scoped_release unlocked;
     at::NoGradGuard no_grad;
     const Tensor x = x_.detach();
     Packed qw;
-    Q3 cq;
     Tensor w;
     if (cached) {
-      cq = q_of(cache.attr("q"));
       N = cq.d.size(0);
       qw = packed_of(cq.d, cq.s, cq.gs, N, K, "cached weight");
     } else {
@@ -608,8 +612,7 @@ Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py
     node = std::shared_ptr<LinearNode>(new LinearNode(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x_, w_));
     node->T = T; node->K = K; node->N = N;
-    node->lid = (unsigned)PyLong_AsUnsignedLongLongMask(lid.ptr());
-    if (PyErr_Occurred()) throw py::error_already_set();
+    node->lid = layer;
     node->signs = signs; node->keep_x = need_w; node->keep_w = !cached && need_x;
     if (cached) { node->cache = cache.ptr(); Py_INCREF(node->cache); }
     node->w = torch::autograd::SavedVariable(w_, false);
@@ -656,44 +659,42 @@ struct LinearScales {
 };
 bool whole_tiles(int64_t R, int64_t C) { return R % 128 == 0 && C % 128 == 0 && R > 0 && C > 0; }
 
-py::tuple k_quant_rows(const Tensor& x_, int mode, py::handle seed_, const OptTensor& am_) {
+using Scaled = std::tuple<Tensor, Tensor, Tensor, OptTensor>;          // d, s, amax, swizzled s
+Scaled k_quant_rows(const Tensor& x_, int mode, const Seed& seed, const OptTensor& am_) {
   require_cuda(x_);
   at::NoGradGuard no_grad;
   REQUIRE(x_.dim() == 2 && x_.scalar_type() == at::kBFloat16 && x_.size(1) % 16 == 0, "quant_rows: a bf16 matrix, columns a multiple of 16");
   const Tensor x = x_.contiguous();
   const int64_t R = x.size(0), C = x.size(1);
-  const Seed seed(seed_);
   const Tensor am = k_amax_or(am_, x);
   Tensor d = empty({R, C / 2}, at::kByte, x);
   LinearScales s(R, C, whole_tiles(R, C), x);
   check(lib.nvfp4_quant_rows(x.const_data_ptr(), C, (int)R, (int)C, d.data_ptr(), s.s.data_ptr(), s.layout, word(am), nullptr, mode,
                              seed.host, seed.dev, stream()), "quant_rows");
-  return py::make_tuple(d, s.s, am, s.sw);
+  return {d, s.s, am, s.sw};
 }
 
-py::tuple k_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, py::handle seed_, const OptTensor& am_) {
+Scaled k_quant_cols_rht(const Tensor& x_, unsigned signs, int mode, const Seed& seed, const OptTensor& am_) {
   require_cuda(x_);
   at::NoGradGuard no_grad;
   const Tensor x = x_.contiguous();
   REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.size(0) % 16 == 0 && x.size(1) % 8 == 0,
           "quant_cols_rht: a bf16 matrix, rows a multiple of 16, columns of 8");
   const int64_t M = x.size(0), C = x.size(1);
-  const Seed seed(seed_);
   const Tensor am = k_amax_or(am_, x);
   Tensor d = empty({C, M / 2}, at::kByte, x);
   LinearScales s(C, M, whole_tiles(C, M), x);
   check(lib.nvfp4_quant_cols_rht(x.const_data_ptr(), (int)M, (int)C, d.data_ptr(), s.s.data_ptr(), s.layout, word(am), nullptr, signs,
                                  mode, seed.host, seed.dev, stream()), "quant_cols_rht");
-  return py::make_tuple(d, s.s, am, s.sw);
+  return {d, s.s, am, s.sw};
 }
 
-py::tuple k_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py::handle seed_, py::handle seed_cols_, const OptTensor& am_) {
+std::pair<Scaled, Scaled> k_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, const Seed& seed, const Seed& seed_cols, const OptTensor& am_) {
   require_cuda(x);
   at::NoGradGuard no_grad;
   REQUIRE(x.dim() == 2 && x.scalar_type() == at::kBFloat16 && x.stride(1) == 1, "quant_rows_cols_rht: a bf16 matrix with contiguous rows");
   const int64_t M = x.size(0), C = x.size(1);
   REQUIRE(M % 128 == 0 && C % 64 == 0, shape_of(M, C));
-  const Seed seed(seed_), seed_cols(seed_cols_);
   const bool both = whole_tiles(M, C);
   Tensor dr = empty({M, C / 2}, at::kByte, x), dc = empty({C, M / 2}, at::kByte, x);
   LinearScales sr(M, C, both, x), sc(C, M, both, x);
@@ -709,10 +710,10 @@ py::tuple k_quant_rows_cols_rht(const Tensor& x, unsigned signs, int mode, py::h
     if (!launched) am = k_amax(x);
   }
   if (!launched)
-  check(lib.nvfp4_quant_tile(x.const_data_ptr(), x.stride(0), (int)M, (int)C, dr.data_ptr(), sr.s.data_ptr(), dc.data_ptr(),
-                             sc.s.data_ptr(), sr.layout, word(am), nullptr, nullptr, signs, mode, seed.host, seed_cols.host,
-                             seed.dev, seed_cols.dev, stream()), "quant_tile");
-  return py::make_tuple(py::make_tuple(dr, sr.s, am, sr.sw), py::make_tuple(dc, sc.s, am, sc.sw));
+    check(lib.nvfp4_quant_tile(x.const_data_ptr(), x.stride(0), (int)M, (int)C, dr.data_ptr(), sr.s.data_ptr(), dc.data_ptr(),
+                               sc.s.data_ptr(), sr.layout, word(am), nullptr, nullptr, signs, mode, seed.host, seed_cols.host,
+                               seed.dev, seed_cols.dev, stream()), "quant_tile");
+  return {{dr, sr.s, am, sr.sw}, {dc, sc.s, am, sc.sw}};
 }
 
 Tensor k_swizzle(const Tensor& s, const OptTensor& out_) {
@@ -724,13 +725,13 @@ Tensor k_swizzle(const Tensor& s, const OptTensor& out_) {
 }
 
 // Buffers of one weight: (d, s, sw) of W and of W^T and the shared amax.
-py::tuple k_w2d_buffers(const Tensor& w) {
+std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, OptTensor, Tensor> k_w2d_buffers(const Tensor& w) {
   require_cuda(w);
   REQUIRE(w.dim() == 2 && w.scalar_type() == at::kFloat && w.size(0) % 16 == 0 && w.size(1) % 16 == 0, "quant_w2d: an FP32 matrix, sides multiples of 16");
   const int64_t N = w.size(0), K = w.size(1);
   const bool both = whole_tiles(N, K);
   LinearScales s(N, K, both, w), st(K, N, both, w);
-  return py::make_tuple(empty({N, K / 2}, at::kByte, w), s.s, s.sw, empty({K, N / 2}, at::kByte, w), st.s, st.sw, empty({1}, at::kFloat, w));
+  return {empty({N, K / 2}, at::kByte, w), s.s, s.sw, empty({K, N / 2}, at::kByte, w), st.s, st.sw, empty({1}, at::kFloat, w)};
 }
 
 void k_quant_w2d(const Tensor& w_, const Tensor& d, const Tensor& s, const OptTensor& sw, const Tensor& dt, const Tensor& st,
@@ -862,6 +863,16 @@ void bind(const py::dict& addresses, py::object error, py::object lin, py::objec
 
 }  // namespace
 
+namespace pybind11::detail {
+template <> struct type_caster<Seed> {
+  PYBIND11_TYPE_CASTER(Seed, const_name("Seed"));
+  bool load(handle src, bool) {
+    value = Seed(src);
+    return true;
+  }
+};
+}  // namespace pybind11::detail
+
 PYBIND11_MODULE(_host, m) {
   py::register_exception_translator([](std::exception_ptr p) {
     try {
@@ -880,28 +891,31 @@ PYBIND11_MODULE(_host, m) {
 #undef X
     return names;
   });
-  m.def("amax", &nvq_amax);
-  m.def("quant_rows", &nvq_quant_rows);
-  m.def("quant_cols_rht", &nvq_quant_cols_rht);
-  m.def("quant_rows_cols_rht", &nvq_quant_rows_cols_rht);
-  m.def("quant_w2d", &nvq_quant_w2d);
-  m.def("quant_w2d_into", &nvq_quant_w2d_into);
-  m.def("mm", &nvq_mm);
-  m.def("linear_fwd", &linear_fwd);
-  m.def("linear_bwd", &linear_bwd);
+  // Launches wait while the queue of the stream is full, and allocations may: other Python threads go on meanwhile.
+  // (linear_apply, which reads Python objects, lets go of the interpreter lock by itself.)
+  const py::call_guard<py::gil_scoped_release> unlocked;
+  m.def("amax", &nvq_amax, unlocked);
+  m.def("quant_rows", &nvq_quant_rows, unlocked);
+  m.def("quant_cols_rht", &nvq_quant_cols_rht, unlocked);
+  m.def("quant_rows_cols_rht", &nvq_quant_rows_cols_rht, unlocked);
+  m.def("quant_w2d", &nvq_quant_w2d, unlocked);
+  m.def("quant_w2d_into", &nvq_quant_w2d_into, unlocked);
+  m.def("mm", &nvq_mm, unlocked);
+  m.def("linear_fwd", &linear_fwd, unlocked);
+  m.def("linear_bwd", &linear_bwd, unlocked);
   m.def("linear_apply", &linear_apply);
-  m.def("k_amax", &k_amax);
-  m.def("k_quant_rows", &k_quant_rows);
-  m.def("k_quant_cols_rht", &k_quant_cols_rht);
-  m.def("k_quant_rows_cols_rht", &k_quant_rows_cols_rht);
-  m.def("k_swizzle", &k_swizzle);
-  m.def("k_w2d_buffers", &k_w2d_buffers);
-  m.def("k_quant_w2d", &k_quant_w2d);
-  m.def("k_gemm", &k_gemm);
-  m.def("e_rows", &e_rows);
-  m.def("e_cols", &e_cols);
-  m.def("e_rms", &e_rms);
-  m.def("e_swiglu", &e_swiglu);
-  m.def("e_mom", &e_mom);
-  m.def("e_mm", &e_mm);
+  m.def("k_amax", &k_amax, unlocked);
+  m.def("k_quant_rows", &k_quant_rows, unlocked);
+  m.def("k_quant_cols_rht", &k_quant_cols_rht, unlocked);
+  m.def("k_quant_rows_cols_rht", &k_quant_rows_cols_rht, unlocked);
+  m.def("k_swizzle", &k_swizzle, unlocked);
+  m.def("k_w2d_buffers", &k_w2d_buffers, unlocked);
+  m.def("k_quant_w2d", &k_quant_w2d, unlocked);
+  m.def("k_gemm", &k_gemm, unlocked);
+  m.def("e_rows", &e_rows, unlocked);
+  m.def("e_cols", &e_cols, unlocked);
+  m.def("e_rms", &e_rms, unlocked);
+  m.def("e_swiglu", &e_swiglu, unlocked);
+  m.def("e_mom", &e_mom, unlocked);
+  m.def("e_mm", &e_mm, unlocked);
 }

@@ -77,6 +77,45 @@ def test_linear_fwd_wants_contiguous_rows():
         assert torch.equal(y, y2) and torch.equal(am, am2) and torch.equal(qxt.d.view(torch.uint8), qxt2.d.view(torch.uint8))
 
 
+@pytest.mark.parametrize("call", ["amax", "layer"])
+def test_other_threads_run_while_launches_wait(call):
+    """Half a second of work in front of more launches than a stream's queue holds: calls block, the interpreter does not."""
+    import threading
+    import time
+    from nvfp4_training_b200 import nvq
+    lin, x, _ = _layer(128, 128, 128, False)
+    word = torch.zeros(1, device="cuda")
+
+    def launch():
+        if call == "amax":
+            nvq.amax(x, out=word, clear=False)
+        else:
+            with torch.no_grad():
+                lin(x)
+    for _ in range(3):
+        launch()
+    torch.cuda.synchronize()
+    done, gap = threading.Event(), [0.0]
+
+    def beat():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gap[0], last = max(gap[0], now - last), now
+    thread = threading.Thread(target=beat)
+    thread.start()
+    torch.cuda._sleep(int(1e9))                              # cycles
+    t0 = time.perf_counter()
+    for _ in range(4000):
+        launch()
+    waited = time.perf_counter() - t0
+    done.set()
+    thread.join()
+    torch.cuda.synchronize()
+    assert waited > 0.25 and gap[0] < waited / 2
+
+
 def test_errors_in_the_backward_pass_keep_their_types(monkeypatch):
     from nvfp4_training_b200 import _lib
     from nvfp4_training_b200.linear import LinCtx
