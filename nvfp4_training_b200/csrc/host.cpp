@@ -477,7 +477,7 @@ struct LinearNode : torch::autograd::Node {
       Py_DECREF(cache);
     }
   }
-  std::string name() const override { return "FP4LinearBackward"; }
+  std::string name() const override { return "FP4LinearFnBackward"; }
   void release_variables() override { w.reset_data(); kept.reset_data(); }
 
   // Exceptions leave through the autograd engine, not through this module: as Python errors of their types
@@ -544,7 +544,7 @@ struct LinearNode : torch::autograd::Node {
 // The layer on x [T, K], w [N, K] -> y [T, N].  With `cache` the quantized weight is taken from it, else W is quantized
 // here: both orientations in one pass when the backward pass will want W^T (one amax and one read of W instead of two
 // of each).  Without gradients only the row operand of x is produced.
-Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py::handle cache, unsigned signs) {
+Tensor linear_apply(unsigned signs, const Tensor& x_, const OptTensor& w_opt, py::handle lid, py::handle cache) {
   require_cuda(x_);
   const Tensor w_ = w_opt.value_or(Tensor());
   if (torch::autograd::isFwGradDefined(x_) || torch::autograd::isFwGradDefined(w_opt)) {
@@ -621,7 +621,6 @@ Tensor linear_apply(const Tensor& x_, const OptTensor& w_opt, py::handle lid, py
   }
   return y;
 }
-
 
 // ------------------------------------------------------------------------------------------ fp4ops operators
 // max|x| as FP32 [1]: one kernel for contiguous bf16 and FP32, torch's reduction for everything else
@@ -903,7 +902,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("mm", &nvq_mm, unlocked);
   m.def("linear_fwd", &linear_fwd, unlocked);
   m.def("linear_bwd", &linear_bwd, unlocked);
-  m.def("linear_apply", &linear_apply);
+  m.def("linear_apply", &linear_apply, py::arg(), py::arg(), py::arg(), py::arg(), py::arg() = py::none());
   m.def("k_amax", &k_amax, unlocked);
   m.def("k_quant_rows", &k_quant_rows, unlocked);
   m.def("k_quant_cols_rht", &k_quant_cols_rht, unlocked);

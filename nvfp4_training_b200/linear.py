@@ -116,16 +116,36 @@ def linear_bwd(x, am_x, gy, qwt, seed, seed_cols, gw_out=None, wgrad_dtype=torch
     return gx, gw
 
 
-class FP4LinearFn:
-    """x [T, K] bf16, w [N, K] bf16 -> y [T, N] bf16 (llm-1b/model.py:45-69), an autograd function in native code
-    (`linear_apply` of csrc/host.cpp).  `cache`: a `WeightCache`, else w is quantized here.  The forward pass keeps x only
-    as the transposed RHT operand that wgrad needs (0.56 byte per element), and W^T's operand when W was quantized here;
-    the backward pass reads `LinCtx`, `nvq.SR_MODE` and `cache.qt` as they stand when it runs.  Gradients nobody asked
-    for, and operands only they would need, are not computed."""
+class FP4LinearFn(torch.autograd.Function):
+    """x [T, K] bf16, w [N, K] bf16 -> y [T, N] bf16 (llm-1b/model.py:45-69).  `cache`: a `WeightCache`, else w is
+    quantized here.  `apply` runs natively (`linear_apply` of csrc/host.cpp): the forward pass keeps x only as the
+    transposed RHT operand that wgrad needs (0.56 byte per element), and W^T's operand (0.56 byte per weight, until the
+    graph is freed) when W was quantized here; the backward pass reads `LinCtx`, `nvq.SR_MODE` and `cache.qt` as they
+    stand when it runs.  Gradients nobody asked for, and operands only they would need, are not computed.  `forward` and
+    `backward` are the same recipe for functions derived from this one, whose `apply` is autograd's own."""
+
+    @classmethod
+    def apply(cls, *args):
+        if cls is FP4LinearFn:
+            return (L._host or L.host()).linear_apply(_RHT_SIGNS, *args)
+        return super().apply(*args)
 
     @staticmethod
-    def apply(x, w, lid, cache=None):
-        return (L._host or L.host()).linear_apply(x, w, lid, cache, _RHT_SIGNS)
+    def forward(ctx, x, w, lid, cache=None):
+        qw = cache.q if cache is not None else nvq.quant_w2d(w, want=(True, False))[0]
+        y, am, qxt = linear_fwd(x, qw, keep_xt=True)
+        ctx.save_for_backward(w, am, qxt.d, qxt.s, qxt.gs)
+        ctx.lid, ctx.cache = lid, cache
+        return y
+
+    @staticmethod
+    def backward(ctx, gy):
+        w, am, xd, xs, xg = ctx.saved_tensors
+        seed = sr_seed(ctx.lid)
+        qwt = ctx.cache.qt if ctx.cache is not None else nvq.quant_w2d(w, want=(False, True))[1]
+        gx, gw = linear_bwd(None, am, gy, qwt, seed, seed ^ 0x5bd1e995, wgrad_dtype=LinCtx.wgrad_dtype,
+                            qxt=nvq.Q(xd, xs, xg))
+        return gx, gw, None, None
 
 
 class Linear(nn.Module):

@@ -204,3 +204,52 @@ def test_forward_mode_is_refused():
     with fwd.dual_level():
         with pytest.raises(NotImplementedError):
             lin(fwd.make_dual(x, torch.ones_like(x)))
+
+
+@pytest.mark.parametrize("cache", [False, True])
+def test_the_function_is_an_autograd_function(cache):
+    """Derived functions run their own forward and backward; positional arguments only, as autograd's apply takes them."""
+    from nvfp4_training_b200.linear import FP4LinearFn
+    assert issubclass(FP4LinearFn, torch.autograd.Function)
+    lin, x, gy = _layer(256, 128, 384, cache)
+    xg = x.clone().requires_grad_(True)
+    seen = []
+
+    class Doubled(FP4LinearFn):
+        @staticmethod
+        def forward(ctx, *args):
+            seen.append("forward")
+            return FP4LinearFn.forward(ctx, *args) * 2
+
+        @staticmethod
+        def backward(ctx, g):
+            seen.append("backward")
+            return FP4LinearFn.backward(ctx, g)
+    y = FP4LinearFn.apply(xg, lin.weight, lin.lid, lin.cache)
+    want = torch.autograd.grad(y, (xg, lin.weight), gy)
+    y2 = Doubled.apply(xg, lin.weight, lin.lid, lin.cache)
+    got = torch.autograd.grad(y2, (xg, lin.weight), gy)
+    assert seen == ["forward", "backward"] and torch.equal(y2, y * 2)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    for bad in ({"lid": 3}, {"lid": 3, "cache": None}):
+        with pytest.raises(TypeError):
+            FP4LinearFn.apply(x, lin.weight, **bad)
+    for args in ((x,), (x, lin.weight, 3, None, None)):
+        with pytest.raises(TypeError):
+            FP4LinearFn.apply(*args)
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda a: FP4LinearFn.apply(a, lin.weight.detach(), 3, lin.cache).float().sum())(x)
+    with pytest.raises(RuntimeError):
+        torch.vmap(lambda a: FP4LinearFn.apply(a, lin.weight.detach(), 3, lin.cache))(torch.stack([x, x]))
+
+
+def test_a_compiled_model_runs_the_layer():
+    """torch.compile breaks its graph at the layer and runs it as it is."""
+    lin, x, gy = _layer(128, 128, 256, False)
+    xg = x.clone().requires_grad_(True)
+    y = lin(xg.relu())
+    want = torch.autograd.grad(y, (xg, lin.weight), gy)
+    f = torch.compile(lambda a: lin(a.relu()), backend="eager")
+    y2 = f(xg)
+    assert torch.equal(y, y2)
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y2, (xg, lin.weight), gy), want))
