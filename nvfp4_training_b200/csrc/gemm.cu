@@ -1258,29 +1258,38 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   }
   int per = (ktiles + splitk - 1) / splitk;
   splitk = (ktiles + per - 1) / per;
-  // CTA-pair kernels (an SM pair per 256-row tile): the fast path unless there are too few tiles for it
-  bool use_pair = g_force_bn != 128 && g_force_bn != 256 && !(g_force_bn == 0 && pairs * splitk < sms / 4);
-  if (owners) use_pair = true;                    // the scatter lives in the pair kernel's epilogue only
-
-  // one-CTA tiles: 256-wide ones only where they keep every SM busy
-  bool wide = (N % 256 == 0) && (long long)(M / kBM) * (N / 256) * splitk >= sms;
-  if (g_force_bn == 128) wide = false;
-  if (g_force_bn == 256 && N % 256 == 0) wide = true;
+  // Relative per-tile cost of a CTA pair fitted to measurements, 256-wide 2.98 + 0.346 per K tile, 192-wide 1.88 + 0.3255
+  // (0.78 of the 256-wide tile at K = 2048, 0.89 at K = 11264), in units of 0.70 us: what decides is mostly how evenly the
+  // tile count divides over the SM pairs.
+  auto rounds = [](long long tiles, long long at_once) { return (double)((tiles + at_once - 1) / at_once); };
+  const double cost256 = N % 256 ? 1e30 : rounds(pairs * splitk, sms / 2) * (2.98 + 0.346 * per);
+  const double cost192 = rounds((long long)((M + 255) / 256) * ((N + 191) / 192) * splitk, sms / 2) * (1.88 + 0.3255 * per);
+  // CTA pairs (an SM pair per 256-row tile) are the fast path; `one` is the width of one-CTA tiles where those are taken
+  int one = 0;
+  if (g_force_bn == 128 || g_force_bn == 256) {
+    one = g_force_bn == 256 && N % 256 == 0 ? 256 : 128;
+  } else if (g_force_bn == 0 && !owners) {
+    if (pairs * splitk < sms / 4) {
+      one = 128;                                  // too few tiles for pairs
+    } else if (M % 256 && splitk == 1 && !accumulate) {
+      // The last row tile of an odd number would be half empty, which costs a pair as much as a full one.  One row tile
+      // (us, pairs / 128-wide: [128, 16384] x K = 2048 10.2 / 7.9, [128, 49152] 17.5 / 13.8, x K = 5632 36.2 / 31.6,
+      // [128, 9472] x K = 512 6.0 / 4.6): never pairs.  More of them: a 256-wide one-CTA tile takes 1.3 times a pair's
+      // round, so where its rounds are that much fewer ([384, 49152] x K = 5632 67.9 / 59.0, x K = 2048 27.6 / 25.5,
+      // [384, 11264] 11.0 / 9.0; not at [384, 16384] 12.9 / 13.1 nor [640, 49152] 38.6 / 40.7).  Adds into C stay with
+      // pairs, which make them row by row.
+      if (M == 128) one = 128;
+      else if (N % 256 == 0 && rounds((long long)(M / kBM) * (N / 256), sms) * 1.3 * (2.98 + 0.346 * per) < fmin(cost256, cost192)) one = 256;
+    }
+  }
+  const bool use_pair = owners || !one;           // the scatter lives in the pair kernel's epilogue only
+  const bool wide = one == 256;
   const int bn = wide ? 256 : 128;
 
   if (use_pair) {
     // tile width: 256 moves the fewest operand bytes per FLOP but consecutive tiles wait for each other's
     // epilogue hand-off; 192 has two independent accumulators and handles any N; 128 as well, more bytes
-    int pbn = 192;
-    if (N % 256 == 0) {
-      // relative per-tile cost of a CTA pair fitted to measurements: 256-wide 2.98 + 0.346 per K tile, 192-wide
-      // 1.88 + 0.3255 (0.78 of the 256-wide tile at K = 2048, 0.89 at K = 11264); what decides is mostly how
-      // evenly the tile count divides over the SM pairs
-      const long long ncl = sms / 2;
-      const long long r256 = ((long long)((M + 255) / 256) * (N / 256) * splitk + ncl - 1) / ncl;
-      const long long r192 = ((long long)((M + 255) / 256) * ((N + 191) / 192) * splitk + ncl - 1) / ncl;
-      if (r256 * (2.98 + 0.346 * per) <= r192 * (1.88 + 0.3255 * per)) pbn = 256;
-    }
+    int pbn = cost256 <= cost192 ? 256 : 192;
     if (g_pair_bn == 128 || g_pair_bn == 192 || (g_pair_bn == 256 && N % 256 == 0)) pbn = g_pair_bn;   // forced (tuning and tests)
     CUtensorMap ma, mb, msa, msb;
     if (!make_map(&ma, a, M, K / 2, lda, 128) || !make_sf_map(&msa, sa, M, K, 1) ||

@@ -283,3 +283,27 @@ def test_fp4ops_gemm_on_the_first_rows_of_an_operand(mods):
         want = fp4ops.gemm(fp4ops.Q(a.d[:128].clone(), a.s[:128].clone(), a.amax), b)
         assert torch.equal(fp4ops.gemm(fp4ops.Q(a.d[:128], a.s, a.amax), b), want)
         assert torch.equal(fp4ops.gemm(b, fp4ops.Q(a.d[:128], a.s, a.amax)), want.t())
+
+
+# one row tile (128-wide one-CTA tiles); three and five (256-wide ones where they save rounds, else pairs); a last K tile of 64
+@pytest.mark.parametrize("M,N", [(128, 9472), (128, 9600), (128, 19200), (384, 11264), (384, 24576), (384, 16384), (640, 11264), (384, 9600)])
+@pytest.mark.parametrize("K", [128, 2112])
+def test_odd_row_tiles_of_wide_outputs(mods, M, N, K):
+    nvq, _, L = mods
+    a, b = nvq.quant_rows(to_dev(make_x(M + K, M, K))), nvq.quant_rows(to_dev(make_w(K, N, K)))
+    y = nvq.dequant(a).double() @ nvq.dequant(b).double().t()
+    top = y.abs().max()
+
+    def close(c, fro=1e-5, rel=1e-4):                                # the bounds of check_close, on the device
+        err = (c.double() - y).abs()
+        assert err.norm() <= fro * y.norm() and bool((err <= rel * y.abs() + 1e-6 * top).all())
+    close(nvq.mm(a, b), 4e-3, 2.0 ** -8)
+    close(nvq.mm(a, b, out_dtype=torch.float32))
+    wide = torch.full((M, N + 8), 3.0, device="cuda")                # rows off their 32-byte boundaries, padding untouched
+    nvq.mm(a, b, out_dtype=torch.float32, out=wide[:, 4:N + 4])
+    close(wide[:, 4:N + 4])
+    assert bool((wide[:, :4] == 3.0).all()) and bool((wide[:, N + 4:] == 3.0).all())
+    out = torch.zeros(M, N, device="cuda")
+    nvq.mm(a, b, out_dtype=torch.float32, out=out, accumulate=True)
+    close(out)
+    L.check_status()
