@@ -98,7 +98,9 @@ def host():
         if not os.path.exists(HOST_PATH):
             raise Nvfp4Error(f"{HOST_PATH} not found: build it with `python -m nvfp4_training_b200.build` "
                              "(there is no fallback path)")
-        from . import _host as h, linear, nvq
+        from . import _host as h, build, linear, nvq
+        if h.built_for != build.host_tag():
+            raise Nvfp4Error(f"{HOST_PATH} was built for {h.built_for}, this is {build.host_tag()}: build it again")
         h.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in h.entry_points()}, Nvfp4Error,
                linear.LinCtx, nvq, status_word)
         _host = h

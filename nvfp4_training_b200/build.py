@@ -43,9 +43,22 @@ def _run(cmd, what, verbose):
         print(res.stdout + res.stderr)
 
 
+def host_tag():
+    """What the host module is tied to: the C++ interfaces of the installed torch and of the interpreter."""
+    import torch
+    return f"torch {torch.__version__} python {sys.version_info.major}.{sys.version_info.minor}"
+
+
+def host_is_stale():
+    if _stale(HOST, ["host.cpp"]):
+        return True
+    with open(HOST, "rb") as f:
+        return host_tag().encode() not in f.read()           # compiled in below
+
+
 def build_host(force=False, verbose=False):
     """The host module (`csrc/host.cpp`): torch's C++ headers, the CUDA runtime's headers, no device code."""
-    if not force and not _stale(HOST, ["host.cpp"]):
+    if not force and not host_is_stale():
         return HOST
     import torch
     from torch.utils.cpp_extension import include_paths
@@ -53,7 +66,7 @@ def build_host(force=False, verbose=False):
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path()))), "include")
     incs = [*include_paths(), cuda, sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[f"-I{d}" for d in incs],
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f'-DNVFP4_HOST_TAG="{host_tag()}"', *[f"-I{d}" for d in incs],
            os.path.join(CSRC, "host.cpp"), "-o", HOST, f"-L{lib_dir}", f"-Wl,-rpath,{lib_dir}",
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
     _run(cmd, HOST, verbose)

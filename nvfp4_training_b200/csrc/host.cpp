@@ -882,6 +882,7 @@ PYBIND11_MODULE(_host, m) {
       PyErr_SetString(error_class.ptr(), e.what());
     }
   });
+  m.attr("built_for") = NVFP4_HOST_TAG;
   m.def("bind", &bind);
   m.def("entry_points", [] {
     py::list names;
