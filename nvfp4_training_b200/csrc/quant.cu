@@ -11,6 +11,15 @@
 
 namespace nvfp4 {
 
+__device__ __forceinline__ void unpack8(const uint4& q, float* f) {
+  const u32 w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    f[2 * i] = __uint_as_float(w[i] << 16);
+    f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+  }
+}
+
 __device__ __forceinline__ uint4 ldg128(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -252,91 +261,116 @@ __global__ void __launch_bounds__(256, 3) quant_cols_rht_kernel(const __nv_bfloa
 }
 
 // ------------------------------------------------------------------------------------------ 16x16 weights
-// Sixteen values of one row of W, as they travel: bf16 pairs, or FP32.
-template <typename T> struct RawRow;
-template <> struct RawRow<__nv_bfloat16> {
-  uint4 v[2];
-  __device__ __forceinline__ void load(const __nv_bfloat16* p) {
-    v[0] = ld_cg_128(reinterpret_cast<const uint4*>(p)); v[1] = ld_cg_128(reinterpret_cast<const uint4*>(p) + 1);
-  }
-  __device__ __forceinline__ void clear() { v[0] = v[1] = make_uint4(0u, 0u, 0u, 0u); }
-  __device__ __forceinline__ void pairs(u64 (&P)[8]) const {
-    const u32 w[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w};
-#pragma unroll
-    for (int i = 0; i < 8; i++) P[i] = f2_from_bf16x2(w[i]);
-  }
-};
-template <> struct RawRow<float> {
-  uint4 v[4];
-  __device__ __forceinline__ void load(const float* p) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = ld_cg_128(reinterpret_cast<const uint4*>(p) + i);
-  }
-  __device__ __forceinline__ void clear() {
-#pragma unroll
-    for (int i = 0; i < 4; i++) v[i] = make_uint4(0u, 0u, 0u, 0u);
-  }
-  __device__ __forceinline__ void pairs(u64 (&P)[8]) const {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      P[2 * i] = (u64)v[i].x | ((u64)v[i].y << 32);
-      P[2 * i + 1] = (u64)v[i].z | ((u64)v[i].w << 32);
-    }
-  }
-};
-
-// Any N and K that are multiples of 16 (weights in whole 128 x 128 tiles take the TMA-fed kernel of quant_w2d.cu): a
-// half-warp owns 64 rows (N) x 32 columns (K) of W, a lane one row of each 16 x 16 block; block maximum by four
-// shuffles, the transposed block's row of codes by NibbleTranspose, bounds-checked 4-byte stores.  L1-bound: the 32
-// lanes of a load or store are on 32 rows.
+// Any N and K that are multiples of 16 (weights in whole 128 x 128 tiles take the TMA-fed kernel of quant_w2d.cu).
+// Persistent CTAs; one warp per group of four 16x16 blocks that are neighbours along N (same K
+// block): lane = (row, 8-column half) of each block, four independent 16-byte loads in flight per
+// lane.  Block max by warp shuffles, codes for W written as one word per lane and block, codes for
+// W^T gathered with shuffles (lane = (k row, 8-row half)) and, after one exchange inside each lane
+// pair, stored as 16 contiguous bytes per lane: a k row's 32 bytes for the four blocks leave together.
+// L1-bound: the lanes of a load or store are on 16 rows.  A half-warp per patch of 4 x 2 blocks, a lane
+// on whole 16-value rows, leaves too few warps and puts 32 rows into each load (us, that one / this one:
+// FP32 [9616, 336] 32.3 / 10.3, [5008, 1552] 46.0 / 20.5, [20000, 5904] 326 / 222, bf16 [2064, 2064] 30.5 / 14.4).
 template <typename T>
-__global__ void __launch_bounds__(256, 2) quant_w2d_kernel(const T* __restrict__ w, unsigned char* __restrict__ q,
-                                                           unsigned char* __restrict__ s, unsigned char* __restrict__ qt,
-                                                           unsigned char* __restrict__ st, const float* __restrict__ amax,
-                                                           int N, int K, int layout, float* __restrict__ gs_out) {
-  constexpr int NB = 4, KB = 2;                      // blocks of the patch along N and K
-  pdl_trigger();
-  const int lane = threadIdx.x & 31, i = lane & 15;
+__global__ void __launch_bounds__(256) quant_w2d_kernel(const T* __restrict__ w, u32* __restrict__ q,
+                                                         unsigned char* __restrict__ s, u32* __restrict__ qt,
+                                                         unsigned char* __restrict__ st, const float* __restrict__ amax,
+                                                         int N, int K, int layout, float* __restrict__ gs_out) {
+  const int lane = threadIdx.x & 31;
   const int nb = N >> 4, kb = K >> 4;
-  const int kgroups = (kb + 2 * KB - 1) / (2 * KB);
-  const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int gn = (int)(item / kgroups) * NB;         // first block row, block column of this half-warp's patch
-  const int gk = (int)(item % kgroups) * (2 * KB) + (lane >> 4) * KB;
-  __shared__ __align__(8) float lut[kLutFloats];
-  pdl_wait();
-  const TensorScale ts = make_tensor_scale<NVFP4_ROUND_NEAREST>(ld_cg_f32(amax), 1.f, lut,
-                                                               (blockIdx.x == 0 && threadIdx.x == 0) ? gs_out : nullptr);
-  const NibbleTranspose transpose(lane);
+  const int ngrp = (nb + 3) >> 2;
+  const bool linear = layout != NVFP4_SCALES_SWIZZLED, swizzled = layout != NVFP4_SCALES_LINEAR;
   unsigned char* s_sw = layout == NVFP4_SCALES_BOTH ? s + (long long)N * kb : s;
   unsigned char* st_sw = layout == NVFP4_SCALES_BOTH ? st + (long long)K * nb : st;
-  const bool linear = layout != NVFP4_SCALES_SWIZZLED, swizzled = layout != NVFP4_SCALES_LINEAR;
+  __shared__ __align__(8) float lut[kLutFloats];
+  const TensorScale ts = make_tensor_scale<NVFP4_ROUND_NEAREST>(__ldg(amax), 1.f, lut,
+                                                               (blockIdx.x == 0 && threadIdx.x == 0) ? gs_out : nullptr);
+  const u64 G = f2_pack(ts.gs, ts.gs), NRG = f2_pack(ts.nrgs, ts.nrgs);
+  const int r = lane >> 1, c0 = (lane & 1) * 8;
+  const bool wide_t = !(N & 31) && !(reinterpret_cast<uintptr_t>(qt) & 15u);   // 16-byte stores of W^T codes possible
+  const long long nitems = (long long)ngrp * kb;
+  const long long wstride = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < nitems; item += wstride) {
+    // consecutive warps walk K: the loads of a CTA are contiguous along each row
+    const int grp = (int)(item / kb), bk = (int)(item - (long long)grp * kb);
+    float v[4][8];
 #pragma unroll
-  for (int c = 0; c < KB; c++) {
+    for (int j = 0; j < 4; j++) {
+      const int bn = grp * 4 + j;
+      if (bn < nb) {
+        const T* src = w + (long long)(bn * 16 + r) * K + bk * 16 + c0;
+        if constexpr (sizeof(T) == 2) {
+          unpack8(ldg128(src), v[j]);
+        } else {
+          const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+          v[j][0] = a.x; v[j][1] = a.y; v[j][2] = a.z; v[j][3] = a.w; v[j][4] = b.x; v[j][5] = b.y; v[j][6] = b.z; v[j][7] = b.w;
+        }
+      } else {
 #pragma unroll
-    for (int b = 0; b < NB; b++) {
-      const bool in = gn + b < nb && gk + c < kb;
-      const int rn = (gn + b) * 16 + i, rk = (gk + c) * 16 + i;        // this lane's row of W and of W^T
-      RawRow<T> raw;
-      if (in) raw.load(w + (long long)rn * K + (gk + c) * 16); else raw.clear();
-      u64 P[8];
-      raw.pairs(P);
-      float m = absmax16(P);
-#pragma unroll
-      for (int o = 8; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      const u32 sb = block_scale_byte(m, ts);
-      const uint2 wq = quant_block16<NVFP4_ROUND_NEAREST>(P, sb, ts, 0u, 0u, 0u);
-      const uint2 wt = transpose(wq);
-      if (in && q) {
-        u32* dst = reinterpret_cast<u32*>(q + (long long)rn * (K >> 1) + (gk + c) * 8);
-        dst[0] = wq.x; dst[1] = wq.y;
-        if (linear) s[(long long)rn * kb + gk + c] = (unsigned char)sb;
-        if (swizzled) s_sw[sw_off(rn, gk + c, kb >> 2)] = (unsigned char)sb;
+        for (int i = 0; i < 8; i++) v[j][i] = 0.f;
       }
-      if (in && qt) {
-        u32* dst = reinterpret_cast<u32*>(qt + (long long)rk * (N >> 1) + (gn + b) * 8);
-        dst[0] = wt.x; dst[1] = wt.y;
-        if (linear) st[(long long)rk * nb + gn + b] = (unsigned char)sb;
-        if (swizzled) st_sw[sw_off(rk, gn + b, nb >> 2)] = (unsigned char)sb;
+    }
+    u32 wt[4], sbs[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int bn = grp * 4 + j;
+      float bmax = absmax3(v[j][0], v[j][1], v[j][2]);
+      bmax = absmax3(bmax, v[j][3], v[j][4]);
+      bmax = absmax3(bmax, v[j][5], v[j][6]);
+      bmax = absmax3(bmax, v[j][7], bmax);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
+      const u32 sb = block_scale_byte(bmax, ts);
+      sbs[j] = sb;
+      const float2 kf = lut_entry(ts, sb);
+      const u64 NRH = f2_pack(kf.x, kf.x), NRL = f2_pack(kf.y, kf.y);
+      float y[8];
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        const u64 t = f2_div_bs(f2_ndiv(f2_pack(v[j][i], v[j][i + 1]), G, NRG), NRH, NRL);
+        y[i] = f2_lo(t); y[i + 1] = f2_hi(t);
+      }
+      const u32 word = e2m1x8_rn(y);
+      if (q && bn < nb) {
+        q[((long long)(bn * 16 + r) * K + bk * 16 + c0) >> 3] = word;
+        if (!(lane & 1) && linear) s[(long long)(bn * 16 + r) * kb + bk] = (unsigned char)sb;
+        if (!(lane & 1) && swizzled) s_sw[sw_off(bn * 16 + r, bk, kb >> 2)] = (unsigned char)sb;
+      }
+      // transposed block: this lane builds k-row kk = lane>>1, n values (lane&1)*8 .. +7
+      const int kk = lane >> 1;
+      u32 t = 0u;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const u32 ww = __shfl_sync(0xffffffffu, word, 2 * (c0 + i) + (kk >> 3));
+        t |= ((ww >> (4 * (kk & 7))) & 15u) << (4 * i);
+      }
+      wt[j] = t;
+    }
+    if (qt) {
+      const int kk = lane >> 1;
+      const long long krow = (long long)bk * 16 + kk;
+      if (grp * 4 + 3 < nb && wide_t) {
+        // even lane keeps blocks 0,1 (both 8-row halves), odd lane blocks 2,3: 16 contiguous bytes each
+        const bool odd = lane & 1;
+        const u32 give0 = odd ? wt[0] : wt[2], give1 = odd ? wt[1] : wt[3];
+        const u32 got0 = __shfl_xor_sync(0xffffffffu, give0, 1), got1 = __shfl_xor_sync(0xffffffffu, give1, 1);
+        const uint4 o = odd ? make_uint4(got0, wt[2], got1, wt[3]) : make_uint4(wt[0], got0, wt[1], got1);
+        *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(qt) + krow * (N >> 1) + grp * 32 + (odd ? 16 : 0)) = o;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          if (grp * 4 + j < nb) qt[(krow * N + (grp * 4 + j) * 16 + c0) >> 3] = wt[j];
+      }
+      if (!(lane & 1)) {
+        if (grp * 4 + 3 < nb && !(nb & 3)) {
+          // the four blocks' scale bytes are neighbours in both layouts (swizzled: nb is a multiple of 8)
+          const u32 four = sbs[0] | (sbs[1] << 8) | (sbs[2] << 16) | (sbs[3] << 24);
+          if (linear) *reinterpret_cast<u32*>(st + krow * nb + grp * 4) = four;
+          if (swizzled) *reinterpret_cast<u32*>(st_sw + sw_off(krow, grp * 4, nb >> 2)) = four;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (grp * 4 + j < nb) st[krow * nb + grp * 4 + j] = (unsigned char)sbs[j];
+        }
       }
     }
   }
@@ -634,19 +668,17 @@ extern "C" int nvfp4_quant_w2d(const void* w, int w_dtype, int N, int K, void* q
   cudaStream_t stm = static_cast<cudaStream_t>(stream);
   if (nvfp4_quant_w2d_tile_accepts(w, N, K, q, s, qt, st_))
     return nvfp4_quant_w2d_tile_launch(w, w_dtype, N, K, q, s, qt, st_, scale_layout, amax, gs_out, stream);
-  const long long warps = (long long)(((N >> 4) + 3) / 4) * (((K >> 4) + 3) / 4);
-  const dim3 grid((unsigned)((warps + 7) / 8));
-  unsigned char *qp = static_cast<unsigned char*>(q), *sp = static_cast<unsigned char*>(s);
-  unsigned char *qtp = static_cast<unsigned char*>(qt), *stp = static_cast<unsigned char*>(st_);
-  cudaError_t rc;
-#define NVFP4_W2D(T) nvfp4_launch_kernel(quant_w2d_kernel<T>, nvfp4_brief((long long)N * K * (long long)sizeof(T)), grid, dim3(256), 0, stm, static_cast<const T*>(w), qp, sp, qtp, stp, amax, N, K, scale_layout, gs_out)
-  if (w_dtype == NVFP4_DTYPE_BF16) rc = NVFP4_W2D(__nv_bfloat16);
-  else rc = NVFP4_W2D(float);
+  const long long nwarps = (long long)(((N >> 4) + 3) >> 2) * (K >> 4);
+  long long blocks = (nwarps + 7) / 8;
+  const long long cap = (long long)sm_count() * 8;
+  if (blocks > cap) blocks = cap;
+#define NVFP4_W2D(T)                                                                                                     \
+  quant_w2d_kernel<T><<<(unsigned)blocks, 256, 0, stm>>>(static_cast<const T*>(w), static_cast<u32*>(q), static_cast<unsigned char*>(s), \
+      static_cast<u32*>(qt), static_cast<unsigned char*>(st_), amax, N, K, scale_layout, gs_out)
+  if (w_dtype == NVFP4_DTYPE_BF16) NVFP4_W2D(__nv_bfloat16);
+  else NVFP4_W2D(float);
 #undef NVFP4_W2D
-  if (rc != cudaSuccess) {
-    (void)cudaGetLastError();
-    return NVFP4_ERR_CUDA;
-  }
+  NVFP4_LAUNCH_CHECK();
   return NVFP4_OK;
 }
 

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import nvfp4_oracle as O
-from tests.gpu_util import u8
+from tests.gpu_util import make_w, to_dev, u8
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +79,34 @@ def test_fp4ops_quantizers_write_both_scale_layouts(M, C):
         assert torch.equal(q.sw, fp4ops.swizzle_scales(q.s))
         q.s.add_(1)                      # changed in place: the swizzled copy is no longer used
         assert q.swizzled() is None
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("N,K", [(128, 256), (384, 128), (16, 16), (48, 64), (80, 48), (1008, 208)])
+def test_w2d_kernels_agree_in_every_layout(N, K, dtype):
+    """Codes off their 16-byte boundaries take the kernel for any shape: the bits the oracle has, whole tiles in all three
+    scale layouts, other shapes row-major; each operand also by itself."""
+    from nvfp4_training_b200 import _lib as L
+    lib = L.load()
+    w = make_w(N * K, N, K)
+    wd = to_dev(w) if dtype == "bf16" else torch.from_numpy(w).cuda()
+    am = wd.abs().amax().float().reshape(1)
+    codes, scales, codes_t, scales_t, _ = O.quant_w2d(w)
+    whole = N % 128 == 0 and K % 128 == 0
+    for layout in (L.SCALES_SWIZZLED, L.SCALES_LINEAR, L.SCALES_BOTH) if whole else (L.SCALES_LINEAR,):
+        for want in ((True, True), (True, False), (False, True)):
+            for off in (0, 4):
+                bufs = [torch.zeros(N * K // d * m + 16, dtype=torch.uint8, device="cuda") for d, m in ((2, 1), (16, 2), (2, 1), (16, 2))]
+                ptrs = [b.data_ptr() + off if want[i // 2] else None for i, b in enumerate(bufs)]
+                assert lib.nvfp4_quant_w2d(wd.data_ptr(), L.DTYPE_BF16 if dtype == "bf16" else L.DTYPE_FP32, N, K, *ptrs, layout,
+                                           am.data_ptr(), None, L.stream()) == 0
+                for i, (d, s, R, C) in enumerate(((codes, scales, N, K), (codes_t, scales_t, K, N))):
+                    q, sc = u8(bufs[2 * i]), u8(bufs[2 * i + 1])
+                    n, m = (R * C // 2, R * C // 16) if want[i] else (0, 0)
+                    assert np.array_equal(q[off:off + n].reshape(-1), np.asarray(d).reshape(-1)[:n]) and not q[off + n:].any()
+                    if layout != L.SCALES_SWIZZLED:
+                        assert np.array_equal(sc[off:off + m], np.asarray(s).reshape(-1)[:m])
+                    if layout != L.SCALES_LINEAR and m:
+                        at = off + (m if layout == L.SCALES_BOTH else 0)
+                        assert np.array_equal(O.unswizzle_scales(sc[at:at + m], R, C // 16), s)
+                    assert not sc[off + m * (2 if layout == L.SCALES_BOTH else 1):].any()
