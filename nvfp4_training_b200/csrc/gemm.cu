@@ -1271,15 +1271,16 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   } else if (g_force_bn == 0 && !owners) {
     if (pairs * splitk < sms / 4) {
       one = 128;                                  // too few tiles for pairs
-    } else if (M % 256 && splitk == 1 && !accumulate) {
+    } else if (M % 256 && splitk == 1) {
       // The last row tile of an odd number would be half empty, which costs a pair as much as a full one.  One row tile
       // (us, pairs / 128-wide: [128, 16384] x K = 2048 10.2 / 7.9, [128, 49152] 17.5 / 13.8, x K = 5632 36.2 / 31.6,
       // [128, 9472] x K = 512 6.0 / 4.6): never pairs.  More of them: a 256-wide one-CTA tile takes 1.3 times a pair's
       // round, so where its rounds are that much fewer ([384, 49152] x K = 5632 67.9 / 59.0, x K = 2048 27.6 / 25.5,
-      // [384, 11264] 11.0 / 9.0; not at [384, 16384] 12.9 / 13.1 nor [640, 49152] 38.6 / 40.7).  Adds into C stay with
-      // pairs, which make them row by row.
+      // [384, 11264] 11.0 / 9.0; not at [384, 16384] 12.9 / 13.1 nor [640, 49152] 38.6 / 40.7).  Adds into C gain as much with
+      // one row tile ([128, 19200] x K = 2048 12.6 / 10.6, [128, 49152] 19.4 / 16.6), but pairs make whole rows of them, which
+      // counts for more with three ([384, 49152] x K = 2048 40.8 / 63.5).
       if (M == 128) one = 128;
-      else if (N % 256 == 0 && rounds((long long)(M / kBM) * (N / 256), sms) * 1.3 * (2.98 + 0.346 * per) < fmin(cost256, cost192)) one = 256;
+      else if (!accumulate && N % 256 == 0 && rounds((long long)(M / kBM) * (N / 256), sms) * 1.3 * (2.98 + 0.346 * per) < fmin(cost256, cost192)) one = 256;
     }
   }
   const bool use_pair = owners || !one;           // the scatter lives in the pair kernel's epilogue only
