@@ -1202,13 +1202,23 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   // it gives, [128, 2048] x K = 5632 took 14.8 us in 16 clusters of 8, 8.1 in clusters of 4), with two K tiles or more
   // each, and enough of them saved to pay for the exchange (about 1.5 us, 0.27 us per K tile).
   bool few = g_force_bn == 0 && !owners && pairs < sms / 4;
-  int slices = 1;
+  int slices = 1, asked = 0;                // `asked`: atomic slices of one-CTA tiles
   if (few) {
     while (slices < 8 && ktiles >= 4 * slices && tiles128 * 2 * slices <= sms && tiles128 <= clusters_at_once(di, 2 * slices)) slices *= 2;
     if (ktiles * (slices - 1) < 6 * slices) slices = 1;
     // where atomic adds are allowed, CTA pairs in more slices win once a slice is long ([2048, 512] x K = 16384, 32 K tiles
     // in each of two slices: 16.6 against 15.0 us; 16 in each of four, [640, 640]: 11.6 against 12.3)
     if ((auto_split || splitk > 1) && c_dtype == NVFP4_DTYPE_FP32 && ktiles > 20 * slices) few = false;
+    if (few && splitk > slices) {
+      // A caller who allows more slices than a cluster has gets them as atomic adds where that shortens a slice by enough
+      // K tiles to pay for the adds: by four, all slices at once on one-CTA tiles (us, cluster / atomic: [128, 128] x
+      // K = 16384 in 16 8.8 / 6.2, x 32768 in 32 10.9 / 6.1, [384, 384] x 32768 11.7 / 8.3), by eight on CTA pairs
+      // ([512, 512] x 16384 in 8 11.0 / 7.8, [640, 640] 11.5 / 10.0).
+      auto longest = [&](long long s) { return (int)((ktiles + s - 1) / s); };
+      const long long one_cta = splitk < sms / tiles128 ? splitk : sms / tiles128, two = splitk < sms / 2 / pairs ? splitk : sms / 2 / pairs;
+      if (one_cta > slices && longest(slices) - longest(one_cta) >= 4) { slices = 1; asked = (int)one_cta; }
+      else if (two > slices && longest(slices) - longest(two) >= 8) { slices = 1; few = false; }
+    }
   }
   if (auto_split && c_dtype == NVFP4_DTYPE_FP32 && g_force_bn == 0 && ktiles >= 16 && !few) {
     // Weight-gradient shapes have few output tiles and a long contraction: 96 or 176 tiles over 74 SM pairs leave
@@ -1242,9 +1252,9 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
     // C (3 TB/s) and the per-tile fixed cost once more: [3072, 1024] x K = 2048 in 8 slices took 32 us, in one 11 us.
     // Same cost model as the tile-width choice below, in units of 0.72 us.
     const long long ncl = sms / 2;
-    const int most = few ? 1 : splitk;
+    const int most = asked ? 0 : few ? 1 : splitk;
     double best = 0;
-    int pick = 1;
+    int pick = asked ? asked : 1;
     for (int s = 1; s <= most; s++) {
       const int per_s = (ktiles + s - 1) / s;
       if ((ktiles + per_s - 1) / per_s != s) continue;
@@ -1269,7 +1279,7 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   if (g_force_bn == 128 || g_force_bn == 256) {
     one = g_force_bn == 256 && N % 256 == 0 ? 256 : 128;
   } else if (g_force_bn == 0 && !owners) {
-    if (pairs * splitk < sms / 4) {
+    if (asked || pairs * splitk < sms / 4) {
       one = 128;                                  // too few tiles for pairs
     } else if (M % 256 && splitk == 1) {
       // The last row tile of an odd number would be half empty, which costs a pair as much as a full one.  One row tile

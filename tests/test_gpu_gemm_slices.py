@@ -41,8 +41,10 @@ def test_few_tile_gemms(M, N, K):
     L.check_status()
 
 
-@pytest.mark.parametrize("M,N,K", [(128, 512, 4096), (3072, 1024, 2048), (1024, 1024, 16384)])
-@pytest.mark.parametrize("splitk", [2, 16])
+# by pairs and clusters; atomic slices of one-CTA tiles, more than K has tiles for; of CTA pairs; uneven ones
+@pytest.mark.parametrize("M,N,K", [(128, 512, 4096), (3072, 1024, 2048), (1024, 1024, 16384), (128, 128, 16384), (128, 128, 4480), (512, 512, 16384),
+                                   (640, 640, 16384), (384, 384, 32640)])
+@pytest.mark.parametrize("splitk", [2, 8, 16, 64])
 def test_requested_slices_add_into_c(M, N, K, splitk):
     """However many slices the library takes, the product is added once to what C holds."""
     from nvfp4_training_b200 import _lib as L, fp4ops
