@@ -1037,7 +1037,10 @@ gemm_nvf4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       // ([16384, 11264, 2048] 195 -> 186 us, [4096, 11264, 2048] 53.7 -> 49.1, FP32 [49152, 2048, 4096] 215 -> 202,
       // sustained; TMA stores from the staging area: 213, 55.2, 218).  Atomic adds stay coalesced, and so do the narrower
       // tiles' stores (a lane's piece of a row is not whole 128-byte lines there: [8192, 3072, 2048] 31.3 against 32.2).
-      if (BN == 256 && !p.atomic && !(reinterpret_cast<uintptr_t>(cbase) & 31u) && !((p.ldc * (p.c_fp32 ? 4 : 2)) & 31))
+      // FP32 only with 16 K tiles or more: with fewer the kernel is bound by its stores and whole lines are what
+      // counts ([11264, 2048] x K = 1024 31.2 against 24.6 staged, x 2048 32.6 / 30.0, x 4096 43.8 / 44.9; [5632, 11264] x
+      // 2048 81.9 / 76.6, x 4096 116.8 / 124.8).
+      if (BN == 256 && !p.atomic && (!p.c_fp32 || p.ktiles_per_split >= 16) && !(reinterpret_cast<uintptr_t>(cbase) & 31u) && !((p.ldc * (p.c_fp32 ? 4 : 2)) & 31))
         direct_store<NC>(r, alpha, p.c_fp32 ? static_cast<void*>(static_cast<float*>(cbase) + lane * p.ldc)
                                             : static_cast<void*>(static_cast<__nv_bfloat16*>(cbase) + lane * p.ldc), p.c_fp32 != 0, valid);
       else
