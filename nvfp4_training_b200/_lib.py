@@ -147,7 +147,8 @@ def status_word(device):
     """Per-device int32 that GEMM CTAs set when a bounded pipeline wait expires (never expected)."""
     key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
     if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}")
+        # the allocation lets other threads run: the first word to be stored is everybody's
+        _status.setdefault(key, torch.zeros(1, dtype=torch.int32, device=f"cuda:{key}"))
     return _status[key]
 
 
