@@ -25,6 +25,7 @@
 #include <torch/csrc/utils/pybind.h>
 
 #include <atomic>
+#include <mutex>
 
 #include "../../include/nvfp4_b200.h"
 
@@ -478,7 +479,10 @@ struct LinearNode : torch::autograd::Node {
     }
   }
   std::string name() const override { return "FP4LinearFnBackward"; }
-  void release_variables() override { w.reset_data(); kept.reset_data(); }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    w.reset_data(); kept.reset_data();
+  }
 
   // Exceptions leave through the autograd engine, not through this module: as Python errors of their types
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
@@ -511,8 +515,12 @@ struct LinearNode : torch::autograd::Node {
     torch::autograd::variable_list out(2);
     if (!grads[0].defined()) return out;
     at::NoGradGuard no_grad;
-    w.unpack(getptr());                         // raises when the graph was freed or the weight changed in place
-    const Tensor buf = kept.unpack(getptr());
+    Tensor buf;
+    {
+      std::lock_guard<std::mutex> lock(mutex_);   // another thread's backward pass may free the graph
+      w.unpack(getptr());                         // raises when the graph was freed or the weight changed in place
+      buf = kept.unpack(getptr());
+    }
     BackwardArgs a;
     a.K = a.Kw = K; a.signs = signs;
     a.want_x = task_should_compute_output(0);

@@ -253,3 +253,28 @@ def test_a_compiled_model_runs_the_layer():
     y2 = f(xg)
     assert torch.equal(y, y2)
     assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y2, (xg, lin.weight), gy), want))
+
+
+def test_backward_passes_of_several_threads_over_one_graph():
+    """Each gets the gradients, or the error for a graph another thread has freed."""
+    from concurrent.futures import ThreadPoolExecutor
+    lin, x, gy = _layer(128, 128, 256, False)
+    xg = x.clone().requires_grad_(True)
+
+    def grads(y, keep):
+        try:
+            got = torch.autograd.grad(y, (xg, lin.weight), gy, retain_graph=keep)
+            torch.cuda.synchronize()
+            return got
+        except RuntimeError as e:
+            assert "second time" in str(e)
+            return None
+    want = grads(lin(xg), False)
+    with ThreadPoolExecutor(8) as pool:
+        for keep in (True, False):
+            for _ in range(20):
+                y = lin(xg)
+                results = list(pool.map(lambda _: grads(y, keep), range(8)))
+                assert any(r is not None for r in results) and (not keep or None not in results)
+                for r in results:
+                    assert r is None or all(torch.equal(a, b) for a, b in zip(r, want))
