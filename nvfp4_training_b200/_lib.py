@@ -122,14 +122,6 @@ def ptr_array(addresses):
     return (ctypes.c_void_p * len(addresses))(*[int(a) for a in addresses])
 
 
-def seed_args(seed):
-    """(host seed, device seed pointer): a CUDA int32/uint32 tensor selects the device-side seed."""
-    if isinstance(seed, torch.Tensor):
-        assert seed.is_cuda and seed.numel() >= 1 and seed.element_size() == 4
-        return 0, seed.data_ptr()
-    return seed & 0xFFFFFFFF, None
-
-
 def stream():
     return torch.cuda.current_stream().cuda_stream
 

@@ -1227,7 +1227,7 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
     // Weight-gradient shapes have few output tiles and a long contraction: 96 or 176 tiles over 74 SM pairs leave
     // a third of the machine idle in the last round.  Slicing K evens that out; the price is the per-tile fixed
     // cost once more per slice, FP32 atomic adds instead of stores, and a zero fill when the call overwrites C.
-    // Same cost model as the tile-width choice below (units of about half a microsecond).
+    // Same cost model as the tile-width choice below (a unit is 0.70 us; the zero fill is counted at 2 TB/s).
     const long long ncl = sms / 2;
     double best = 0;
     for (int s = 1; s <= 8 && s <= ktiles; s++) {
@@ -1253,7 +1253,7 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
   if (splitk > 1 && g_force_bn == 0 && !owners && !auto_split) {
     // The caller's number of slices is an upper bound.  A slice that adds no parallelism costs a pass of atomic adds over
     // C (3 TB/s) and the per-tile fixed cost once more: [3072, 1024] x K = 2048 in 8 slices took 32 us, in one 11 us.
-    // Same cost model as the tile-width choice below, in units of 0.72 us.
+    // Same cost model as the tile-width choice below.
     const long long ncl = sms / 2;
     const int most = asked ? 0 : few ? 1 : splitk;
     double best = 0;
@@ -1264,7 +1264,7 @@ static int gemm_impl(const void* a, const void* sa, long long lda, const void* b
       const long long t192 = (long long)((M + 255) / 256) * ((N + 191) / 192) * s;
       double cost = (double)((t192 + ncl - 1) / ncl) * (1.88 + 0.3255 * per_s);
       if (N % 256 == 0) cost = fmin(cost, (double)((pairs * s + ncl - 1) / ncl) * (2.98 + 0.346 * per_s));
-      if (s > 1) cost = fmax(cost, (double)s * (double)M * (double)N * 4.0 / (3.0e6 * 0.72));
+      if (s > 1) cost = fmax(cost, (double)s * (double)M * (double)N * 4.0 / (3.0e6 * 0.70));
       if (s == 1 || cost < best * 0.97) { best = cost; pick = s; }
     }
     splitk = pick;

@@ -51,7 +51,8 @@ __device__ __forceinline__ u32 amax_take(u32 m, const uint4& v) {
   return __vmaxu2(m, v.w & 0x7FFF7FFFu);
 }
 
-// HBM-bound: 6.9 TB/s on tensors of 300 MB and more.  A thread keeps four loads in flight all the time (the oldest is
+// HBM-bound: 5.0 to 5.2 TB/s on tensors of 134 to 403 MB, 7.1 at 2 GB, where the first loads and the uneven last round no
+// longer count.  A thread keeps four loads in flight all the time (the oldest is
 // consumed and replaced): batches of four with a wait in between left the memory idle once per batch, which on a tensor
 // of two or three batches is a fifth of the time (46 MB: 11.0 -> 8.7 us; 33 MB from L2: 4.6 -> 3.8 us).
 // Where the result goes:
